@@ -216,7 +216,7 @@ struct sgs_engine {
   unsigned long long *h_cnt = nullptr;     // pinned mirror
   DBuf<uint32_t> emark;                    // engine-level marks (touched sets)
   uint32_t estamp = 1;
-  DBuf<double> l1;                         // PR per-round L1
+  DBuf<double> prh;                        // PR per-round history (StepHist)
   DBuf<unsigned long long> rstat;          // per-round instance-edge counts
   DBuf<unsigned long long> hstat;          // per-round host-tier slots
   DBuf<unsigned long long> b_lane;         // [WLANES] per-lane edge counts
@@ -423,7 +423,7 @@ struct sgs_engine {
     b_reclaim.ensure(2);
     b_nkept.ensure(1);
     rl_count.ensure(1);
-    l1.ensure(cfg.max_rounds + 2);
+    prh.ensure(StepHist::FIELDS * (size_t)(cfg.max_rounds + 2));
     rstat.ensure(cfg.max_rounds + 2);
     hstat.ensure(cfg.max_rounds + 2);
     b_lane.ensure(WLANES);
@@ -1297,24 +1297,34 @@ struct sgs_engine {
     reset_counters(0);
     { ++n_launch; k_dense_frontier<<<grid_elem(nv), 256, 0, s>>>(gi, fview(0, cnt.p)); }
     const uint32_t maxr = cfg.max_rounds;
-    CK(cudaMemsetAsync(l1.p, 0, sizeof(double) * (maxr + 2), s));
+    CK(cudaMemsetAsync(prh.p, 0, sizeof(double) * StepHist::FIELDS * (maxr + 2), s));
     unsigned long long pr_in = 0;
     CK(cudaMemcpyAsync(&pr_in, cnt.p, sizeof(pr_in), cudaMemcpyDeviceToHost, s));
     sync();
-    return pr_steps(q, fview(0, cnt.p), fview(1, cnt.p + 1), pull, l1.p, 0, maxr, edge_stat, pr_in, conv,
-                    last_l1);
+    return pr_steps(q, fview(0, cnt.p), fview(1, cnt.p + 1), pull, StepHist{prh.p, maxr + 2}, 0, maxr, edge_stat,
+                    pr_in, conv, last_l1);
   }
 
   // Rounds r0, r0+1, ... (at most `limit`) over a prebuilt dense frontier
   // `fin` of the store the sweep reads (in-edge store when `pull`); per-round
-  // absorbed L1 in l1buf[r].  Returns the rounds run; conv when a round's L1
-  // falls below pr_tol.
-  uint32_t pr_steps(Query &q, FrontierView fin, FrontierView fout, bool pull, double *l1buf, uint32_t r0,
+  // history in h[r].  Returns the rounds run; conv when a round's L1 falls
+  // below the tolerance (pr_tol; less after a long round, sgs_steplen.cuh).
+  uint32_t pr_steps(Query &q, FrontierView fin, FrontierView fout, bool pull, StepHist h, uint32_t r0,
                     uint32_t limit, unsigned long long *edge_stat, unsigned long long pr_in, bool &conv,
                     double &last_l1) {
     const GraphView g = view();
     const GraphView gi = pull ? in_view() : g;
-    std::vector<double> hl(34);
+    // one strided copy reads the fields of a batch of rounds
+    std::vector<double> hl;
+    auto read_history = [&](uint32_t first, uint32_t n) {
+      hl.resize(StepHist::FIELDS * (size_t)n);
+      CK(cudaMemcpy2DAsync(hl.data(), n * sizeof(double), h.p + first, h.n * sizeof(double), n * sizeof(double),
+                           StepHist::FIELDS, cudaMemcpyDeviceToHost, s));
+    };
+    auto ends = [&](uint32_t k, uint32_t n) {
+      const StepHist f{hl.data(), n};
+      return StepRule::ends(f.step()[k], f.l1()[k], (int)f.state()[k], cfg.pr_tol);
+    };
     uint32_t r = 0, rb = 8;
     conv = false;
     last_l1 = 0;
@@ -1330,12 +1340,13 @@ struct sgs_engine {
       d_rounds.ensure(1);
       GraphView ga = g, gb = gi;
       FrontierView f = fin;
-      double *x = q.x.p, *rp = q.r.p, *pv = q.pv.p, *l1b = l1buf;
+      double *x = q.x.p, *rp = q.r.p, *pv = q.pv.p;
+      StepHist hh = h;
       double alpha = cfg.pr_alpha, tol = cfg.pr_tol;
       uint32_t r0a = r0, lim = limit;
       unsigned long long *es = edge_stat;
       uint32_t *ro = d_rounds.p;
-      void *args[] = {&ga, &f, &gb, &x, &rp, &pv, &alpha, &tol, &l1b, &r0a, &lim, &es, &ro};
+      void *args[] = {&ga, &f, &gb, &x, &rp, &pv, &alpha, &tol, &hh, &r0a, &lim, &es, &ro};
       // no more CTAs than units (idle CTAs only lengthen the grid barriers)
       const int grid = (int)std::max<uint64_t>(std::min<uint64_t>(units, (uint64_t)coop_grid(fn)), nsm);
       if (ktiming) {
@@ -1346,14 +1357,13 @@ struct sgs_engine {
       CK(cudaLaunchCooperativeKernel(fn, grid, RELAX_THREADS, args, 0, s));
       if (ktiming) CK(cudaEventRecord(kev[1], s));
       uint32_t ran = 0;
-      hl.resize(limit);
       CK(cudaMemcpyAsync(&ran, d_rounds.p, sizeof(ran), cudaMemcpyDeviceToHost, s));
-      CK(cudaMemcpyAsync(hl.data(), l1buf + r0, sizeof(double) * limit, cudaMemcpyDeviceToHost, s));
+      read_history(r0, limit);
       sync();
       if (ran > limit) fail(SGS_ERR_CUDA, "PageRank round kernel returned a bad round count");
       if (ran) {
         last_l1 = hl[ran - 1];
-        conv = last_l1 < cfg.pr_tol;
+        conv = ends(ran - 1, limit);
       }
       if (ktiming && ran) {
         float ms = 0;
@@ -1367,16 +1377,17 @@ struct sgs_engine {
       if (ktiming) ensure_kev(2 * nb);
       for (uint32_t k = 0; k < nb; ++k) {
         { ++n_launch; k_pr_absorb<<<grid_elem(nv), RELAX_THREADS, 0, s>>>(g, q.x.p, q.r.p, q.pv.p, cfg.pr_alpha,
-                                                           l1buf + r0 + r + k); }
+                                                           cfg.pr_tol, h, r0 + r + k); }
         if (ktiming) CK(cudaEventRecord(kev[2 * k], s));
         if (pull)
-          { ++n_launch; k_pull_pr<<<grid_map(), RELAX_THREADS, 0, s>>>(fin, gi, q.pv.p, q.r.p, edge_stat); }
+          { ++n_launch; k_pull_pr<<<grid_map(), RELAX_THREADS, 0, s>>>(fin, gi, q.pv.p, q.r.p, h.step() + r0 + r + k,
+                                                                   edge_stat); }
         else
           { ++n_launch; seg_map<<<grid_map(), RELAX_THREADS, 0, s>>>(fin, fout, op, edge_stat); }
         if (ktiming) CK(cudaEventRecord(kev[2 * k + 1], s));
       }
       CK(cudaGetLastError());
-      CK(cudaMemcpyAsync(hl.data(), l1buf + r0 + r, sizeof(double) * nb, cudaMemcpyDeviceToHost, s));
+      read_history(r0 + r, nb);
       sync();
       if (ktiming)
         for (uint32_t k = 0; k < nb; ++k)
@@ -1384,10 +1395,10 @@ struct sgs_engine {
                   kev[2 * k + 1]);
       for (uint32_t k = 0; k < nb; ++k) {
         last_l1 = hl[k];
-        if (hl[k] < cfg.pr_tol) { conv = true; return r + k + 1; }
+        if (ends(k, nb)) { conv = true; return r + k + 1; }
       }
       r += nb;
-      rb = std::min<uint32_t>(rb * 2, 32);
+      rb = 4;  // a round at this size takes far longer than a host read
     }
     return r;
   }
@@ -1403,7 +1414,7 @@ struct sgs_engine {
     Frontier f;
     uint32_t ucap = 0;
     DBuf<unsigned long long> c;  // [0] frontier counter, [1] output counter, [2] edge count
-    DBuf<double> l1;
+    DBuf<double> prh;
     unsigned long long pr_in = 0;
     float ms = 0;
     // a snapshot was applied while the job ran: its residual was amended
@@ -1443,7 +1454,7 @@ struct sgs_engine {
     job.f.ebase.ensure((size_t)nv + 1);
     job.f.ustart.ensure(job.ucap);
     job.c.ensure(3);
-    job.l1.ensure(cfg.max_rounds + 2);
+    job.prh.ensure(StepHist::FIELDS * (size_t)(cfg.max_rounds + 2));
     job.stale = false;
     job.pull = (cfg.pull & 1u) && ensure_in(job_view(0), job_view(1));
     auto q = std::make_unique<Query>();
@@ -1457,7 +1468,7 @@ struct sgs_engine {
     CK(cudaMemsetAsync(job.c.p, 0, sizeof(unsigned long long) * 3, s));
     const GraphView gi = job.pull ? in_view() : view();
     { ++n_launch; k_dense_frontier<<<grid_elem(nv), 256, 0, s>>>(gi, job_view(0)); }
-    CK(cudaMemsetAsync(job.l1.p, 0, sizeof(double) * (cfg.max_rounds + 2), s));
+    CK(cudaMemsetAsync(job.prh.p, 0, sizeof(double) * StepHist::FIELDS * (cfg.max_rounds + 2), s));
     CK(cudaMemcpyAsync(&job.pr_in, job.c.p, sizeof(job.pr_in), cudaMemcpyDeviceToHost, s));
     CK(cudaEventRecord(ev_q.b, s));
     sync();
@@ -1475,6 +1486,9 @@ struct sgs_engine {
     if (!job.q) fail(SGS_ERR_STATE, "no PageRank job");
     if (job.stale) {
       job_frontier();
+      // the residual was amended after round r - 1: no ratio across it
+      if (job.r)
+        CK(cudaMemsetAsync(StepHist{job.prh.p, cfg.max_rounds + 2}.step() + job.r - 1, 0, sizeof(double), s));
       job.stale = false;
     }
     Query &q = *job.q;
@@ -1482,7 +1496,8 @@ struct sgs_engine {
     bool conv = false;
     double l1v = 0;
     CK(cudaEventRecord(ev_q.a, s));
-    const uint32_t ran = pr_steps(q, job_view(0), job_view(1), job.pull, job.l1.p, job.r, lim, job.c.p + 2,
+    const uint32_t ran = pr_steps(q, job_view(0), job_view(1), job.pull,
+                                  StepHist{job.prh.p, cfg.max_rounds + 2}, job.r, lim, job.c.p + 2,
                                   job.pr_in, conv, l1v);
     CK(cudaEventRecord(ev_q.b, s));
     sync();
@@ -1521,7 +1536,7 @@ struct sgs_engine {
     CK(cudaMemsetAsync(f0.counter, 0, sizeof(unsigned long long), s));
     { ++n_launch; k_dense_frontier<<<grid_elem(nv), 256, 0, s>>>(gi, f0); }
     if (pull)
-      { ++n_launch; k_pull_pr<<<grid_map(), RELAX_THREADS, 0, s>>>(f0, gi, q.pv.p, q.r.p, nullptr); }
+      { ++n_launch; k_pull_pr<<<grid_map(), RELAX_THREADS, 0, s>>>(f0, gi, q.pv.p, q.r.p, nullptr, nullptr); }
     else
       { ++n_launch; seg_map<<<grid_map(), RELAX_THREADS, 0, s>>>(f0, f1, PrPushOp{g, q.pv.p, q.r.p}, nullptr); }
     CK(cudaGetLastError());

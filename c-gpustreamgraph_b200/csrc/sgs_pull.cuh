@@ -97,13 +97,14 @@ __global__ void k_transpose_keys(const uint64_t *in, uint32_t n, const uint32_t 
 // entry's lanes are contiguous), run heads add into a shared per-entry sum,
 // and each entry is written once per CTA: a plain store when the CTA holds
 // all of its positions, an atomicAdd (r is zero from the absorb step) when it
-// is split between CTAs.  edge_stat counts the live slots read.
+// is split between CTAs.  With `add` the sum goes on top of what the absorb
+// left in r (a long round).  edge_stat counts the live slots read.
 // Coherent: pv was written earlier in the same launch (the persistent round
 // kernel k_pr_rounds), so it is read through L2 instead of the non-coherent
 // read-only path.
 template <bool Coherent>
 __device__ __forceinline__ void pull_pr_body(const FrontierView &in, const GraphView &gi, const double *pv,
-                                             double *r, unsigned long long *edge_stat) {
+                                             double *r, bool add, unsigned long long *edge_stat) {
   constexpr int GC = CHUNK;
   __shared__ uint64_t s_eb[GC + 1];
   __shared__ uint32_t s_len[GC];
@@ -188,7 +189,7 @@ __device__ __forceinline__ void pull_pr_body(const FrontierView &in, const Graph
         if (idx < n && s_eb[t] < E1) {
           const uint64_t ee = s_eb[t] + ((s_len[t] + 3u) & ~3u);  // end of the entry's padded range
           const double x = s_acc[t];
-          if (s_eb[t] >= E0 && ee <= E1) r[s_vtx[t]] = x;
+          if (s_eb[t] >= E0 && ee <= E1) r[s_vtx[t]] = add ? (Coherent ? __ldcg(&r[s_vtx[t]]) : r[s_vtx[t]]) + x : x;
           else if (x != 0.0) atomicAdd(&r[s_vtx[t]], x);
         }
       }
@@ -203,9 +204,9 @@ __device__ __forceinline__ void pull_pr_body(const FrontierView &in, const Graph
 }
 
 __global__ void __launch_bounds__(RELAX_THREADS)
-    k_pull_pr(FrontierView in, GraphView gi, const double *pv, double *r,
+    k_pull_pr(FrontierView in, GraphView gi, const double *pv, double *r, const double *step,
               unsigned long long *edge_stat) {
-  pull_pr_body<false>(in, gi, pv, r, edge_stat);
+  pull_pr_body<false>(in, gi, pv, r, step && *step != 1.0, edge_stat);
 }
 
 // One bottom-up BFS round of a narrow group (S lanes, all running lanes

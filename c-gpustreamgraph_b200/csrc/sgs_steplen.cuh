@@ -1,0 +1,95 @@
+// sgs_steplen.cuh -- step lengths of the engine's fixed-point iterations
+// (PageRank rounds in sgs_kernels.cuh, personalized PageRank in ppr.cu).
+//
+// Both iterate x <- x + w d with d = c + M x - x, M = alpha P^T (or alpha P for
+// the adjoint): w = 1 is the reference's round.  Whatever the steps were, x is
+// that much nearer or further, never wrong: d is the residual of the
+// x at hand, and the iteration ends on a plain step whose d is below the
+// tolerance.
+//
+// With w = 1, d shrinks by M's largest eigenvalue mu per step -- 0.84 on R-MAT
+// graphs -- while everything in it beside the Perron vector shrinks by the
+// second one, 0.15 there.  So after a few steps d is all but a multiple of
+// that vector, and one long step, w = 1 / (1 - mu), whose factor
+// 1 - w (1 - lambda) is zero at lambda = mu, removes it.
+// mu is the ratio of the L1 norms of two successive d.  A long step leaves
+// w (d_k+1 - mu d_k), so the steps before it measure that: `fit` is the norm of
+// d_k - mu d_k-1 (one more read per vertex), and the long step is taken when it
+// would leave less than a fifth of d.  On graphs without such a gap
+// (bipartite ones, grids, cycles with a mixed-sign d) the fit stays bad and
+// every step stays plain.  Should a long step not halve d after all, no
+// other one follows.
+// Steps to the tolerance, long steps included, on R-MAT graphs of scale 10 to
+// 18: PageRank from scratch 116-151 -> 22-26, after an update 59-85 -> 18-21.
+//
+// Once a long step was taken, the end asks for a sixteenth of the tolerance
+// (one or two steps at the faster rate): the error at the end, 1e-9 to 1e-8 of
+// L1 norm instead of 7e-7 in those runs, is then no larger than that of the slow
+// approach and the steps that were queued past its end.
+#pragma once
+#include <cstdint>
+#include <cuda_runtime.h>
+
+namespace sgs {
+
+enum StepState : int { ST_PLAIN = 0, ST_LONG = 1, ST_FAILED = 2 };
+constexpr double LONG_TOL = 1.0 / 16.0;
+
+// One entry per step in device memory, zeroed before the first: |d|, the fit
+// and the mu it was taken with (0: none was), the step length (0 marks a d
+// that was changed between two steps, so no ratio across it counts), state.
+// Fields are `n` entries apart.  A step's rule reads entries that earlier
+// launches, or phases before a grid barrier, wrote.
+struct StepHist {
+  static constexpr int FIELDS = 5;
+  double *p;
+  uint32_t n;
+  __host__ __device__ double *l1() const { return p; }
+  __host__ __device__ double *fit() const { return p + n; }
+  __host__ __device__ double *mu() const { return p + 2 * (size_t)n; }
+  __host__ __device__ double *step() const { return p + 3 * (size_t)n; }
+  __host__ __device__ double *state() const { return p + 4 * (size_t)n; }
+};
+
+struct StepRule {
+  double w;   // step length
+  double mu;  // > 0: take the fit with it
+  int state;
+  // whether a step with norm l1 under this rule ends the iteration
+  __host__ __device__ static bool ends(double w, double l1, int state, double tol) {
+    return w == 1.0 && l1 < (state == ST_LONG ? tol * LONG_TOL : tol);
+  }
+};
+
+__device__ __forceinline__ StepRule step_rule(const StepHist &h, uint32_t k, double alpha, double tol) {
+  StepRule s{1.0, 0.0, k ? (int)__ldcg(h.state() + k - 1) : ST_PLAIN};
+  if (k < 2 || s.state == ST_FAILED) return s;
+  const double a = __ldcg(h.l1() + k - 1), b = __ldcg(h.l1() + k - 2);
+  const double w1 = __ldcg(h.step() + k - 1), w2 = __ldcg(h.step() + k - 2);
+  const double f = __ldcg(h.fit() + k - 1), mu0 = __ldcg(h.mu() + k - 1);
+  if (w2 > 1.0 && !(a < 0.5 * b)) {
+    s.state = ST_FAILED;
+    return s;
+  }
+  if (w1 != 1.0 || w2 != 1.0 || !(b > 0.0)) return s;
+  const double mu = a / b;
+  // (below 0.3 a plain step is as good; M's spectral radius is at most alpha)
+  if (!(mu > 0.3 && mu <= alpha * 1.0001)) return s;
+  // no long step near the end: a step queued past it must not raise d
+  if (a < (s.state == ST_LONG ? tol * LONG_TOL : tol)) return s;
+  s.mu = mu;
+  if (mu0 > 0.0 && f + fabs(mu - mu0) * b < 0.2 * (1.0 - mu) * a) {
+    s.w = 1.0 / (1.0 - mu);
+    s.state = ST_LONG;
+  }
+  return s;
+}
+
+// Records step k's rule (one thread of the step's grid).
+__device__ __forceinline__ void record_rule(const StepHist &h, uint32_t k, const StepRule &s) {
+  h.mu()[k] = s.mu;
+  h.step()[k] = s.w;
+  h.state()[k] = (double)s.state;
+}
+
+}  // namespace sgs
