@@ -692,15 +692,17 @@ __global__ void k_group_relax_inserted(GraphView g, unsigned long long *st, uint
   }
 }
 
+// One lane of every vertex: its values from the mirror (between snapshots
+// equal to the packed words' values, and half their bytes per row), or with
+// val == null its parents from the packed words.  Bound by the rows' sectors:
+// a lane's 4 or 8 bytes cost a 32-B sector each, which narrow values share
+// between two vertices.
 template <int S>
-__global__ void k_group_split(const unsigned long long *st, uint32_t nv, int lane, uint32_t *val,
-                              uint32_t *par) {
+__global__ void k_group_column(const unsigned long long *st, const uint32_t *val, uint32_t nv, int lane,
+                               uint32_t *out) {
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < nv; v += stride) {
-    const unsigned long long s = st[v * S + lane];
-    if (val) val[v] = (uint32_t)(s >> 32);
-    if (par) par[v] = (uint32_t)s;
-  }
+  for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < nv; v += stride)
+    out[v] = val ? val[v * S + lane] : (uint32_t)st[v * S + lane];
 }
 
 template <int S>
