@@ -370,6 +370,54 @@ __device__ __forceinline__ void frontier_append_block(const FrontierView &f, boo
   __syncthreads();  // s_warp / s_base are reused by the next call
 }
 
+// A warp's own queue (in shared memory) of vertices to append to a frontier.
+// A walk's step finds up to four per thread; appending them as they come took
+// one counter atomic per step and slot of the quad, all on one address, and
+// that address set the pace of rounds that improve many vertices.  The queue
+// hands them over 32 at a time: one scan, one atomic, coalesced length reads.
+// SSSP and BFS from scratch on a million vertices: the rounds 2163 -> 1085 us,
+// the query 2.6 -> 1.7 ms.
+struct WarpQueue {
+  static constexpr int CAP = 31 + 4 * 32;
+  uint32_t *v;     // [CAP] of this warp
+  uint32_t n = 0;  // warp-uniform
+  __device__ __forceinline__ explicit WarpQueue(uint32_t *mine) : v(mine) {}
+  // Bit k of `app`: append dst[k].  All 32 lanes, converged.
+  template <class Len>
+  __device__ __forceinline__ void push4(const FrontierView &f, uint32_t app, const uint32_t (&dst)[4],
+                                        const Len &len) {
+    if (!__ballot_sync(0xFFFFFFFFu, app != 0u)) return;
+    const uint32_t below = (1u << (threadIdx.x & 31)) - 1u;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const uint32_t m = __ballot_sync(0xFFFFFFFFu, app >> k & 1u);
+      if (app >> k & 1u) v[n + __popc(m & below)] = dst[k];
+      n += __popc(m);
+    }
+    __syncwarp();
+    while (n >= 32) flush(f, 32, len);
+  }
+  template <class Len>
+  __device__ __forceinline__ void push(const FrontierView &f, bool want, uint32_t dst, const Len &len) {
+    const uint32_t m = __ballot_sync(0xFFFFFFFFu, want);
+    if (!m) return;
+    if (want) v[n + __popc(m & ((1u << (threadIdx.x & 31)) - 1u))] = dst;
+    n += __popc(m);
+    __syncwarp();
+    while (n >= 32) flush(f, 32, len);
+  }
+  // Appends the last min(n, most) of the queue (most <= 32).
+  template <class Len>
+  __device__ __forceinline__ void flush(const FrontierView &f, uint32_t most, const Len &len) {
+    const uint32_t c = min(n, most), lane = threadIdx.x & 31;
+    const bool want = lane < c;
+    const uint32_t x = want ? v[n - c + lane] : 0u;
+    n -= c;
+    __syncwarp();  // read before the next push writes the places
+    frontier_append(f, want, x, want ? len(x) : 0u);
+  }
+};
+
 // Warp-aggregated atomicAdd: lanes with want add val to *p; returns each
 // lane's old value (exclusive prefix within the warp added).  All 32 lanes of
 // a converged warp must call it.

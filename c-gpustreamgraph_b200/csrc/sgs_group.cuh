@@ -289,6 +289,9 @@ __device__ __forceinline__ void group_map_body(FrontierView in, FrontierView out
   __shared__ uint32_t s_vtx[GC];
   __shared__ unsigned long long s_lane[GMAX];
   __shared__ unsigned long long s_host, s_all;  // host-tier slots read over the link / owned
+  __shared__ uint32_t s_queue[RELAX_THREADS / 32][WarpQueue::CAP];
+  WarpQueue queue(s_queue[threadIdx.x >> 5]);
+  auto len_of = [&](uint32_t v) { return op.append_len(v); };
   clear_prev_masks(prev_vtx, prev_cnt, prev_mask);
   if (threadIdx.x < GMAX) s_lane[threadIdx.x] = 0;
   if (threadIdx.x == 0) s_host = s_all = 0;
@@ -426,18 +429,13 @@ __device__ __forceinline__ void group_map_body(FrontierView in, FrontierView out
           jc = jn;
           qc = qn;
           hc = hn;
-          if (__ballot_sync(0xFFFFFFFFu, app != 0u)) {
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              const bool w = app >> k & 1u;
-              frontier_append(out, w, dst[k], w ? op.append_len(dst[k]) : 0u);
-            }
-          }
+          queue.push4(out, app, dst, len_of);
         }
       }
       if (s_eb[GC] >= E1 || s + GC >= n) break;
       s += GC;
     }
+    queue.flush(out, 32, len_of);
   }
   const unsigned long long hs = warp_sum((unsigned long long)host_acc);
   if ((threadIdx.x & 31) == 0 && hs) atomicAdd(&s_host, hs);
