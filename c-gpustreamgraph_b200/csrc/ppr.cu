@@ -23,11 +23,13 @@
 // Work split: a warp owns a work item.  Vertices of degree <= PIECE are one
 // item each; a heavier vertex (R-MAT hubs reach 10^5 in-edges) is cut into
 // pieces of PIECE edges whose partial sums go to a scratch row each and are
-// added up, in piece order, by a finalize kernel -- so no warp walks more
-// than PIECE edges and the sums are deterministic.  Inside a warp, LPE lanes
+// added up, in piece order, by the warp that finishes the vertex's last piece
+// -- so no warp walks more than PIECE edges and the sums are deterministic.  Inside a warp, LPE lanes
 // cover the columns of one neighbour row (CPL columns per lane) and 32/LPE
 // neighbours are gathered at once, four deep, so one neighbour row is one
 // coalesced read for any K.
+#include <cooperative_groups.h>
+
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
 
@@ -39,6 +41,7 @@
 #include <vector>
 
 #include "../../include/sgs.h"
+#include "sgs_steplen.cuh"
 
 namespace sgs {
 void set_last_error(const std::string &msg);
@@ -170,14 +173,20 @@ __global__ void k_csc_probs(const double *pr, const uint32_t *ceid, uint64_t ne,
     pc[i] = pr[ceid[i]];
 }
 
+// Row values: read-only cached loads, or, in the launch that runs many steps
+// (it wrote the rows itself, from other SMs too), loads through L2.
+template <bool Coh>
+__device__ __forceinline__ double ld_row(const double *p) {
+  return Coh ? __ldcg(p) : __ldg(p);
+}
+
 // Narrow rows (K < 32): each lane group loads its own neighbours' ids,
 // probabilities and rows, four neighbours deep (neighbours b+eg, b+eg+NEG, ...).
-template <int LPE, int CPL>
+template <int LPE, int CPL, bool Coh>
 __device__ __forceinline__ void gather_rows_direct(const uint32_t *__restrict__ nbr,
                                                    const double *__restrict__ p, uint64_t b,
                                                    uint64_t e, int eg, uint32_t kb, uint32_t K,
-                                                   const double *__restrict__ x,
-                                                   double (&acc)[CPL]) {
+                                                   const double *x, double (&acc)[CPL]) {
   constexpr int NEG = 32 / LPE;
   uint64_t i = b + eg;
   for (; i + 3 * NEG < e; i += 4 * NEG) {
@@ -194,7 +203,7 @@ __device__ __forceinline__ void gather_rows_direct(const uint32_t *__restrict__ 
 #pragma unroll
       for (int j = 0; j < CPL; ++j) {
         const uint32_t k = kb + j * LPE;
-        xv[q][j] = k < K ? x[(uint64_t)u[q] * K + k] : 0.0;
+        xv[q][j] = k < K ? ld_row<Coh>(x + (uint64_t)u[q] * K + k) : 0.0;
       }
 #pragma unroll
     for (int q = 0; q < 4; ++q)
@@ -207,7 +216,7 @@ __device__ __forceinline__ void gather_rows_direct(const uint32_t *__restrict__ 
 #pragma unroll
     for (int j = 0; j < CPL; ++j) {
       const uint32_t k = kb + j * LPE;
-      if (k < K) acc[j] = fma(pp, x[(uint64_t)u * K + k], acc[j]);
+      if (k < K) acc[j] = fma(pp, ld_row<Coh>(x + (uint64_t)u * K + k), acc[j]);
     }
   }
 }
@@ -217,11 +226,11 @@ __device__ __forceinline__ void gather_rows_direct(const uint32_t *__restrict__ 
 // one coalesced load per warp and are handed to the lane groups by shuffles
 // (group eg takes neighbours eg, eg + NEG, ...), so the only dependent load
 // per neighbour is its row; DEPTH neighbours per group are in flight at once.
-template <int LPE, int CPL>
+template <int LPE, int CPL, bool Coh>
 __device__ __forceinline__ void gather_rows(const uint32_t *__restrict__ nbr,
                                             const double *__restrict__ p, uint64_t b, uint64_t e,
                                             int lane, int eg, uint32_t kb, uint32_t K,
-                                            const double *__restrict__ x, double (&acc)[CPL]) {
+                                            const double *x, double (&acc)[CPL]) {
   constexpr int NEG = 32 / LPE;
   constexpr int DEPTH = LPE < 4 ? LPE : 4;
   for (uint64_t c = b; c < e; c += 32) {
@@ -246,7 +255,7 @@ __device__ __forceinline__ void gather_rows(const uint32_t *__restrict__ nbr,
 #pragma unroll
         for (int jj = 0; jj < CPL; ++jj) {
           const uint32_t k = kb + jj * LPE;
-          xv[q][jj] = ok[q] && k < K ? __ldg(x + (uint64_t)u[q] * K + k) : 0.0;
+          xv[q][jj] = ok[q] && k < K ? ld_row<Coh>(x + (uint64_t)u[q] * K + k) : 0.0;
         }
 #pragma unroll
       for (int q = 0; q < DEPTH; ++q)
@@ -256,45 +265,78 @@ __device__ __forceinline__ void gather_rows(const uint32_t *__restrict__ nbr,
   }
 }
 
-// One Jacobi step over the work items [0, npieces) (pieces of heavy vertices:
-// partial sums to part[piece][K]) and [npieces, npieces + nv) (light vertices:
-// out[v,k] = c B[v,k] + alpha sum p x, |out - x| added to *diff).
-template <int LPE, int CPL>
-__global__ void __launch_bounds__(THREADS, LPE == 32 ? 1 : 8)
-    k_ppr_step(const uint64_t *__restrict__ ptr, const uint32_t *__restrict__ nbr,
-               const double *__restrict__ p, uint32_t nv, const uint32_t *__restrict__ pv,
-               const uint32_t *__restrict__ poff, uint32_t npieces, uint32_t K, double alpha,
-               double c, const double *__restrict__ B, const double *__restrict__ x,
-               double *__restrict__ out, double *__restrict__ part, double *diff) {
+// One step's arguments: the edge lists with their pieces, out = x + w d with
+// d = c B + alpha sum p x - x, and the history of the step lengths.
+struct StepArgs {
+  const uint64_t *ptr;
+  const uint32_t *nbr;
+  const double *p;
+  uint32_t nv;
+  const uint32_t *pv, *poff;
+  uint32_t npieces;
+  uint32_t K;
+  double alpha, c;
+  const double *B;
+  double *part;    // a row of K per piece
+  uint32_t *done;  // finished pieces, at the vertex's first piece (zero between steps)
+  sgs::StepHist h;
+  double tol;
+};
+
+// The new state of one entry; |d| and the fit (sgs_steplen.cuh) into dsum,
+// fsum.  out still holds the state before x, so x - out is the previous d.
+template <bool Coh>
+__device__ __forceinline__ void finish_entry(const StepArgs &a, const sgs::StepRule &rule, uint64_t o, double sum,
+                                             const double *x, double *out, double &dsum, double &fsum) {
+  const double nx = a.c * __ldg(a.B + o) + a.alpha * sum;
+  const double xo = ld_row<Coh>(x + o);
+  const double d = nx - xo;
+  dsum += fabs(d);
+  if (rule.mu > 0.0) fsum += fabs(d - rule.mu * (xo - __ldcg(out + o)));
+  out[o] = rule.w == 1.0 ? nx : fma(rule.w, d, xo);
+}
+
+// One step over the work items [0, npieces) (pieces of heavy vertices: partial
+// sums to part[piece][K]; the warp that finishes a vertex's last piece adds
+// them up in piece order and writes the vertex) and [npieces, npieces + nv)
+// (light vertices).  The pieces come first, so their sums are added while the
+// other warps walk the light vertices; a kernel of its own for them cost 5 us
+// per step on a small graph and 85 us at a million vertices and K = 64.
+template <int LPE, int CPL, bool Coh>
+__device__ __forceinline__ void ppr_step_body(const StepArgs &a, const sgs::StepRule &rule, const double *x,
+                                              double *out, uint32_t k_hist) {
   const int lane = threadIdx.x & 31;
   const int sub = lane % LPE, eg = lane / LPE;
-  double dsum = 0.0;
-  const uint32_t items = npieces + nv;
+  const uint32_t K = a.K;
+  double dsum = 0.0, fsum = 0.0;
+  const uint32_t items = a.npieces + a.nv;
   const uint32_t W = num_warps();
   uint64_t pb = 0, pe = 0;  // bounds of this warp's next light vertex, loaded ahead
   bool have = false;
   for (uint32_t wi = warp_id(); wi < items; wi += W) {
-    uint32_t v;
+    uint32_t v, first = 0, last = 0;
     uint64_t b, e;
-    const bool piece = wi < npieces;
+    const bool piece = wi < a.npieces;
     if (piece) {
-      v = pv[wi];
-      b = ptr[v] + (uint64_t)(wi - poff[v]) * PIECE;
-      e = min(b + PIECE, ptr[v + 1]);
+      v = a.pv[wi];
+      first = a.poff[v];
+      last = a.poff[v + 1];
+      b = a.ptr[v] + (uint64_t)(wi - first) * PIECE;
+      e = min(b + PIECE, a.ptr[v + 1]);
     } else {
-      v = wi - npieces;
+      v = wi - a.npieces;
       if (have) {
         b = pb;
         e = pe;
       } else {
-        b = ptr[v];
-        e = ptr[v + 1];
+        b = a.ptr[v];
+        e = a.ptr[v + 1];
       }
       if constexpr (LPE == 32) {  // the narrow forms have no registers to spare
         have = wi + W < items;
         if (have) {
-          pb = ptr[v + W];
-          pe = ptr[v + W + 1];
+          pb = a.ptr[v + W];
+          pe = a.ptr[v + W + 1];
         }
       }
       if (e - b > PIECE) continue;  // summed by its pieces
@@ -304,9 +346,9 @@ __global__ void __launch_bounds__(THREADS, LPE == 32 ? 1 : 8)
 #pragma unroll
       for (int j = 0; j < CPL; ++j) acc[j] = 0.0;
       if constexpr (LPE == 32)
-        gather_rows<LPE, CPL>(nbr, p, b, e, lane, eg, k0 + sub, K, x, acc);
+        gather_rows<LPE, CPL, Coh>(a.nbr, a.p, b, e, lane, eg, k0 + sub, K, x, acc);
       else
-        gather_rows_direct<LPE, CPL>(nbr, p, b, e, eg, k0 + sub, K, x, acc);
+        gather_rows_direct<LPE, CPL, Coh>(a.nbr, a.p, b, e, eg, k0 + sub, K, x, acc);
 #pragma unroll
       for (int j = 0; j < CPL; ++j)
 #pragma unroll
@@ -316,48 +358,77 @@ __global__ void __launch_bounds__(THREADS, LPE == 32 ? 1 : 8)
         for (int j = 0; j < CPL; ++j) {
           const uint32_t k = k0 + sub + j * LPE;
           if (k >= K) continue;
-          if (piece) {
-            part[(uint64_t)wi * K + k] = acc[j];
-          } else {
-            const uint64_t o = (uint64_t)v * K + k;
-            const double nx = c * B[o] + alpha * acc[j];
-            dsum += fabs(nx - x[o]);
-            out[o] = nx;
-          }
+          if (piece) a.part[(uint64_t)wi * K + k] = acc[j];
+          else finish_entry<Coh>(a, rule, (uint64_t)v * K + k, acc[j], x, out, dsum, fsum);
+        }
+      }
+    }
+    if (piece) {
+      __threadfence();  // this warp's row before its count
+      __syncwarp();
+      uint32_t n = 0;
+      if (lane == 0) n = atomicAdd(a.done + first, 1u);
+      n = __shfl_sync(0xFFFFFFFFu, n, 0);
+      if (n + 1 == last - first) {
+        __threadfence();
+        if (lane == 0) a.done[first] = 0;
+        for (uint32_t k = lane; k < K; k += 32) {
+          double sum = 0.0;
+#pragma unroll 8
+          for (uint32_t q = first; q < last; ++q) sum += __ldcg(a.part + (uint64_t)q * K + k);
+          finish_entry<Coh>(a, rule, (uint64_t)v * K + k, sum, x, out, dsum, fsum);
         }
       }
     }
   }
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) dsum += __shfl_xor_sync(0xFFFFFFFFu, dsum, o);
-  if (lane == 0 && dsum != 0.0) atomicAdd(diff, dsum);
+  for (int o = 16; o > 0; o >>= 1) {
+    dsum += __shfl_xor_sync(0xFFFFFFFFu, dsum, o);
+    fsum += __shfl_xor_sync(0xFFFFFFFFu, fsum, o);
+  }
+  if (lane == 0) {
+    if (dsum != 0.0) atomicAdd(a.h.l1() + k_hist, dsum);
+    if (fsum != 0.0) atomicAdd(a.h.fit() + k_hist, fsum);
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) sgs::record_rule(a.h, k_hist, rule);
 }
 
-// Heavy vertices: out[v,k] = c B[v,k] + alpha (sum of v's piece rows, in
-// piece order); one warp per first piece.
-__global__ void __launch_bounds__(THREADS)
-    k_ppr_finalize(const uint32_t *__restrict__ pv, const uint32_t *__restrict__ poff,
-                   uint32_t npieces, uint32_t K, double alpha, double c,
-                   const double *__restrict__ B, const double *__restrict__ x,
-                   double *__restrict__ out, const double *__restrict__ part, double *diff) {
-  const int lane = threadIdx.x & 31;
-  double dsum = 0.0;
-  for (uint32_t pi = warp_id(); pi < npieces; pi += num_warps()) {
-    const uint32_t v = pv[pi];
-    if (poff[v] != pi) continue;
-    const uint32_t pe = poff[v + 1];
-    for (uint32_t k = lane; k < K; k += 32) {
-      double s = 0.0;
-      for (uint32_t q = pi; q < pe; ++q) s += part[(uint64_t)q * K + k];
-      const uint64_t o = (uint64_t)v * K + k;
-      const double nx = c * B[o] + alpha * s;
-      dsum += fabs(nx - x[o]);
-      out[o] = nx;
-    }
+template <int LPE, int CPL>
+__global__ void __launch_bounds__(THREADS, LPE == 32 ? 4 : LPE == 1 ? 6 : 8)
+    k_ppr_step(StepArgs a, const double *__restrict__ x, double *out, uint32_t k) {
+  ppr_step_body<LPE, CPL, false>(a, sgs::step_rule(a.h, k, a.alpha, a.tol * sgs::LONG_TOL), x, out, k);
+}
+
+// The end of the iteration, the same on both sides: a plain step below the
+// tolerance that is also a sixteenth of it (LONG_TOL; a second one after a long
+// step, sgs_steplen.cuh), or the EXTRA-th one below it, should rounding keep
+// the rest away.
+constexpr uint32_t EXTRA = 20;
+__host__ __device__ inline bool ppr_ends(double w, double l1, int state, double tol, uint32_t &under) {
+  if (w == 1.0 && l1 < tol) ++under;
+  return w == 1.0 && l1 < tol && (sgs::StepRule::ends(w, l1, state, tol * sgs::LONG_TOL) || under > EXTRA);
+}
+
+// Steps k0 .. k1 - 1 in one cooperative launch, a grid barrier after each, until
+// the end; step k reads buffer k % 2 and writes the other.  For graphs whose
+// step takes about as long as a launch: forward and backward on 4,096 vertices
+// with K = 8 took 8.0 ms with two launches per step and 0.84 per step, 2.3 with
+// this loop and the long steps.
+template <int LPE, int CPL>
+__global__ void __launch_bounds__(THREADS, 4)
+    k_ppr_steps(StepArgs a, double *x0, double *x1, uint32_t k0, uint32_t k1, uint32_t under, uint32_t *ran) {
+  cooperative_groups::grid_group grid = cooperative_groups::this_grid();
+  uint32_t k = k0;
+  while (k < k1) {
+    const sgs::StepRule rule = sgs::step_rule(a.h, k, a.alpha, a.tol * sgs::LONG_TOL);
+    ppr_step_body<LPE, CPL, true>(a, rule, k % 2 ? x1 : x0, k % 2 ? x0 : x1, k);
+    __threadfence();
+    grid.sync();
+    const double l1 = __ldcg(a.h.l1() + k);
+    ++k;
+    if (ppr_ends(rule.w, l1, rule.state, a.tol, under)) break;
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) dsum += __shfl_xor_sync(0xFFFFFFFFu, dsum, o);
-  if (lane == 0 && dsum != 0.0) atomicAdd(diff, dsum);
+  if (blockIdx.x == 0 && threadIdx.x == 0) *ran = k - k0;
 }
 
 // gw[e] = inv_s[u] (alpha sum_k X[u,k] Y[v,k] + c_u) for e = (u,v), where
@@ -440,12 +511,18 @@ struct sgs_ppr {
   uint64_t ne = 0;
   Buf<uint64_t> row, crow;
   Buf<uint32_t> col, csrc, ceid;
-  Buf<double> w, inv_s, pr, pc, t, x, xn, g, y, yn, part, diff;
+  Buf<double> w, inv_s, pr, pc, t, x, xn, g, y, yn, part;
+  // one allocation: the step history, then (u32) the steps a looping launch ran
+  // and the finished pieces per heavy vertex
+  Buf<double> work;
+  uint32_t *ran() { return (uint32_t *)(work.p + sgs::StepHist::FIELDS * (size_t)HIST); }
+  uint32_t *done() { return ran() + 1; }
+  static constexpr uint32_t HIST = 512;  // steps the history holds
   Buf<unsigned int> err;
   Adj in, out;  // CSC (forward) and CSR (adjoint, edge gradient)
   // timing and counters
   bool timing = false;
-  std::vector<cudaEvent_t> ev;  // 2 per step of a batch (timing on)
+  std::vector<cudaEvent_t> ev;  // around a batch of steps (timing on)
   cudaEvent_t call_ev[2] = {nullptr, nullptr};
   sgs_ppr_stats st{};
   uint64_t n_launch = 0;
@@ -460,7 +537,7 @@ struct sgs_ppr {
       PCK(cudaEventCreate(&call_ev[0]));
       PCK(cudaEventCreate(&call_ev[1]));
     }
-    while (ev.size() < 64) {
+    while (ev.size() < 2) {
       cudaEvent_t e;
       PCK(cudaEventCreate(&e));
       ev.push_back(e);
@@ -574,7 +651,9 @@ struct sgs_ppr {
     inv_s.ensure(nv);
     pr.ensure(ne);
     pc.ensure(ne);
-    diff.ensure(64);
+    const size_t words = 1 + (size_t)std::max(in.npieces, out.npieces);
+    work.ensure(sgs::StepHist::FIELDS * (size_t)HIST + (words + 1) / 2);
+    PCK(cudaMemsetAsync(ran(), 0, sizeof(uint32_t) * words, s));
     sync();
   }
 
@@ -592,68 +671,111 @@ struct sgs_ppr {
     if (h) throw PprFail{SGS_ERR_INVALID, "edge weights must be positive and finite"};
   }
 
-  template <int LPE, int CPL>
-  void launch_step(const Adj &a, const double *p, uint32_t K, double alpha, double c,
-                   const double *B, const double *xin, double *xout, double *d) {
-    { ++n_launch; k_ppr_step<LPE, CPL><<<rgrid((const void *)k_ppr_step<LPE, CPL>), THREADS, 0, s>>>(a.ptr, a.nbr, p, nv, a.pv.p, a.poff.p,
-                                                    a.npieces, K, alpha, c, B, xin, xout, part.p, d); }
-  }
-
   template <int L>
   void launch_grad(uint32_t K, double alpha, const double *Y, double *dst) {
     { ++n_launch; k_ppr_edge_grad<L><<<rgrid((const void *)k_ppr_edge_grad<L>), THREADS, 0, s>>>(row.p, col.p, inv_s.p, nv, out.pv.p, out.poff.p,
                                                   out.npieces, K, alpha, x.p, Y, g.p, dst); }
   }
 
-  // One Jacobi step xin -> xout along `a` with probabilities p.
-  void step(const Adj &a, const double *p, uint32_t K, double alpha, double c, const double *B,
-            const double *xin, double *xout, double *d) {
-    switch (K <= 32 ? lanes_per_edge(K) : 64) {
-      case 1: launch_step<1, 1>(a, p, K, alpha, c, B, xin, xout, d); break;
-      case 2: launch_step<2, 1>(a, p, K, alpha, c, B, xin, xout, d); break;
-      case 4: launch_step<4, 1>(a, p, K, alpha, c, B, xin, xout, d); break;
-      case 8: launch_step<8, 1>(a, p, K, alpha, c, B, xin, xout, d); break;
-      case 16: launch_step<16, 1>(a, p, K, alpha, c, B, xin, xout, d); break;
-      case 32: launch_step<32, 1>(a, p, K, alpha, c, B, xin, xout, d); break;
-      default: launch_step<32, 2>(a, p, K, alpha, c, B, xin, xout, d); break;
+  // A step of fewer bytes than this (step_bytes) takes less than about 20 us
+  // and runs in the launch that loops on the device; a longer one hides its
+  // launch and gathers through the read-only cache.
+  static constexpr double LOOP_BYTES = 64e6;
+
+  template <int LPE, int CPL>
+  void launch(const StepArgs &a, bool loop, double *b0, double *b1, uint32_t k, uint32_t k1, uint32_t under) {
+    if (loop) {
+      const void *f = (const void *)k_ppr_steps<LPE, CPL>;
+      StepArgs aa = a;
+      uint32_t *r = ran();
+      void *args[] = {&aa, &b0, &b1, &k, &k1, &under, &r};
+      // no more CTAs than items (idle ones only lengthen the barriers)
+      const uint64_t need = ((uint64_t)a.npieces + a.nv + THREADS / 32 - 1) / (THREADS / 32);
+      const uint32_t gr = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(rgrid(f), need));
+      ++n_launch;
+      PCK(cudaLaunchCooperativeKernel(f, gr, THREADS, args, 0, s));
+      return;
     }
-    if (a.npieces)
-      { ++n_launch; k_ppr_finalize<<<rgrid((const void *)k_ppr_finalize), THREADS, 0, s>>>(a.pv.p, a.poff.p, a.npieces, K, alpha, c, B, xin,
-                                                xout, part.p, d); }
+    for (; k < k1; ++k) {
+      ++n_launch;
+      k_ppr_step<LPE, CPL><<<rgrid((const void *)k_ppr_step<LPE, CPL>), THREADS, 0, s>>>(a, k % 2 ? b1 : b0,
+                                                                                       k % 2 ? b0 : b1, k);
+    }
+  }
+  // Steps k .. k1 - 1 (or, looping, up to the end of the iteration).
+  void steps(const StepArgs &a, bool loop, double *b0, double *b1, uint32_t k, uint32_t k1, uint32_t under) {
+    switch (a.K <= 32 ? lanes_per_edge(a.K) : 64) {
+      case 1: launch<1, 1>(a, loop, b0, b1, k, k1, under); break;
+      case 2: launch<2, 1>(a, loop, b0, b1, k, k1, under); break;
+      case 4: launch<4, 1>(a, loop, b0, b1, k, k1, under); break;
+      case 8: launch<8, 1>(a, loop, b0, b1, k, k1, under); break;
+      case 16: launch<16, 1>(a, loop, b0, b1, k, k1, under); break;
+      case 32: launch<32, 1>(a, loop, b0, b1, k, k1, under); break;
+      default: launch<32, 2>(a, loop, b0, b1, k, k1, under); break;
+    }
+    PCK(cudaGetLastError());
   }
 
-  // Jacobi steps (cur -> nxt, swap) until one step changes the state by
-  // less than tol in L1; batches of 4, 8, ..., 32 steps between host reads
-  // (the steps after the first converged one only move the state closer).
-  template <class Step>
-  int iterate(Step stepf, double *&cur, double *&nxt, double tol, uint32_t max_iter) {
-    uint32_t it = 0, batch = 4;
-    double hd[32];
+  // The fixed point of x = c B + alpha A x from the state in b0, b1 as the
+  // second buffer: steps until one changes the state by less than tol in L1
+  // (ppr_ends).  `cur` = the buffer with the result.  Returns the steps run, -1
+  // when max_iter did not suffice.
+  int iterate(const Adj &adj, const double *p, uint32_t K, double alpha, double c, const double *B, double *b0,
+              double *b1, double tol, uint32_t max_iter, double *&cur) {
+    const double bytes = step_bytes(K);
+    const bool loop = bytes < LOOP_BYTES;
+    StepArgs a{adj.ptr, adj.nbr, p, nv, adj.pv.p, adj.poff.p, adj.npieces, K, alpha, c, B, part.p, done(),
+               sgs::StepHist{work.p, HIST}, tol};
+    const size_t row = sizeof(double);
+    PCK(cudaMemsetAsync(work.p, 0, row * sgs::StepHist::FIELDS * HIST, s));
+    uint32_t it = 0, k = 0, under = 0;
+    bool below = false;  // the last plain step was below tol
+    std::vector<double> hd;
     while (it < max_iter) {
-      const uint32_t nb = std::min<uint32_t>(batch, max_iter - it);
-      PCK(cudaMemsetAsync(diff.p, 0, sizeof(double) * nb, s));
-      for (uint32_t b = 0; b < nb; ++b) {
-        if (timing) PCK(cudaEventRecord(ev[2 * b], s));
-        stepf(cur, nxt, diff.p + b);
-        if (timing) PCK(cudaEventRecord(ev[2 * b + 1], s));
-        std::swap(cur, nxt);
-      }
-      PCK(cudaGetLastError());
-      PCK(cudaMemcpyAsync(hd, diff.p, sizeof(double) * nb, cudaMemcpyDeviceToHost, s));
-      sync();
-      if (timing)
-        for (uint32_t b = 0; b < nb; ++b) {
-          float ms = 0.f;
-          PCK(cudaEventElapsedTime(&ms, ev[2 * b], ev[2 * b + 1]));
-          st.steps_ms += ms;
+      if (k == HIST) {
+        // the rule looks back four entries: move them to the front.  (An even
+        // number, so that k % 2 still names the buffer to read.)
+        constexpr uint32_t keep = 4;
+        for (int f = 0; f < sgs::StepHist::FIELDS; ++f) {
+          double *q = work.p + (size_t)f * HIST;
+          PCK(cudaMemcpyAsync(q, q + HIST - keep, row * keep, cudaMemcpyDeviceToDevice, s));
+          PCK(cudaMemsetAsync(q + keep, 0, row * (HIST - keep), s));
         }
-      it += nb;
+        k = keep;
+      }
+      // A launch per step: 8 steps before the first host read (never fewer are
+      // needed), then 2 to 4 -- a read costs about 10 us, steps past the end
+      // their own time.
+      uint32_t nb = std::min<uint32_t>(HIST - k, max_iter - it);
+      if (!loop) nb = std::min<uint32_t>(nb, it == 0 ? 8 : bytes > 256e6 ? 2 : 4);
+      if (timing) PCK(cudaEventRecord(ev[0], s));
+      steps(a, loop, b0, b1, k, k + nb, under);
+      if (timing) PCK(cudaEventRecord(ev[1], s));
+      hd.resize(sgs::StepHist::FIELDS * (size_t)nb);
+      uint32_t n = nb;
+      PCK(cudaMemcpy2DAsync(hd.data(), row * nb, work.p + k, row * HIST, row * nb, sgs::StepHist::FIELDS,
+                            cudaMemcpyDeviceToHost, s));
+      if (loop) PCK(cudaMemcpyAsync(&n, ran(), sizeof(n), cudaMemcpyDeviceToHost, s));
+      sync();
+      if (n > nb) throw PprFail{SGS_ERR_CUDA, "PPR step kernel returned a bad step count"};
+      if (timing) {
+        float ms = 0.f;
+        PCK(cudaEventElapsedTime(&ms, ev[0], ev[1]));
+        st.steps_ms += ms;
+      }
+      const sgs::StepHist h{hd.data(), nb};
+      bool end = false;
+      for (uint32_t b = 0; b < n; ++b) {
+        end = end || ppr_ends(h.step()[b], h.l1()[b], (int)h.state()[b], tol, under);
+        below = h.step()[b] == 1.0 && h.l1()[b] < tol;
+      }
+      it += n;
+      k += n;
       st.iters = (int32_t)it;
-      for (uint32_t b = 0; b < nb; ++b)
-        if (hd[b] < tol) return (int)it;
-      batch = std::min<uint32_t>(batch * 2, 32);
+      cur = k % 2 ? b1 : b0;
+      if (end) return (int)it;
     }
-    return -1;
+    return below ? (int)it : -1;
   }
 
   int forward(const double *T, uint32_t K, double alpha, double tol, uint32_t max_iter, double *X,
@@ -665,10 +787,8 @@ struct sgs_ppr {
     part.ensure((uint64_t)std::max(in.npieces, out.npieces) * K);
     PCK(cudaMemcpyAsync(t.p, T, sizeof(double) * n, kin(mem), s));
     { ++n_launch; k_scale<<<grid(), THREADS, 0, s>>>(t.p, 1.0 - alpha, n, x.p); }
-    double *cur = x.p, *nxt = xn.p;
-    const int it = iterate(
-        [&](double *a, double *b, double *d) { step(in, pc.p, K, alpha, 1.0 - alpha, t.p, a, b, d); },
-        cur, nxt, tol, max_iter);
+    double *cur = x.p;
+    const int it = iterate(in, pc.p, K, alpha, 1.0 - alpha, t.p, x.p, xn.p, tol, max_iter, cur);
     PCK(cudaMemcpyAsync(X, cur, sizeof(double) * n, kout(mem), s));
     sync();
     return it;
@@ -685,10 +805,8 @@ struct sgs_ppr {
     PCK(cudaMemcpyAsync(x.p, X, sizeof(double) * n, kin(mem), s));
     PCK(cudaMemcpyAsync(g.p, G, sizeof(double) * n, kin(mem), s));
     PCK(cudaMemcpyAsync(y.p, g.p, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
-    double *cur = y.p, *nxt = yn.p;
-    const int it = iterate(
-        [&](double *a, double *b, double *d) { step(out, pr.p, K, alpha, 1.0, g.p, a, b, d); },
-        cur, nxt, tol, max_iter);
+    double *cur = y.p;
+    const int it = iterate(out, pr.p, K, alpha, 1.0, g.p, y.p, yn.p, tol, max_iter, cur);
     if (it < 0) return it;
     if (gw && ne) {
       Buf<double> tmp;
