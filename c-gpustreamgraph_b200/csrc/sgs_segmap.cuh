@@ -50,9 +50,61 @@ __device__ __forceinline__ uint32_t visit_quad(const Op &op, uint32_t u,
   }
 }
 
+// A warp's walk over its share of a staged chunk, one window of 32 quads (128
+// positions) per step, lane i on quad i.  Owners need no search per quad: lane
+// j holds the start of entry s0 + j (s0 = owner of the window's first quad),
+// every start inside the window sets bit (start - window) / 4 of a warp-wide
+// OR, and a lane's owner is s0 plus the set bits at or below its quad.  Every
+// frontier entry has at least one slot (each append site checks it), so a
+// window meets at most 32 entries and no two starts share a bit.  The same
+// bits give the next window's first owner.  (With a binary search per
+// quad, eight dependent shared-memory reads, tombstoning 500,000 deletes at
+// scale 24 took 420 us instead of 402.)
+template <int GC>
+struct WindowWalk {
+  const uint64_t *eb;   // [GC + 1] starts of the chunk's entries
+  const uint32_t *len;  // [GC] their slots
+  uint64_t q, end;      // this warp's share in quads: next window, end
+  int s0;
+  // Warp `wid` of `nw`, over positions [lo, hi) of the chunk.
+  __device__ __forceinline__ WindowWalk(const uint64_t *eb_, const uint32_t *len_, uint64_t lo, uint64_t hi,
+                                        uint32_t wid, uint32_t nw)
+      : eb(eb_), len(len_) {
+    const uint64_t nq = hi > lo ? (hi - lo) >> 2 : 0;
+    q = (lo >> 2) + nq * wid / nw;
+    end = (lo >> 2) + nq * (wid + 1) / nw;
+    int a = 0, b = GC - 1;
+    if (q < end)
+      while (a < b) {  // owner of the share's first quad, once per chunk
+        const int m = (a + b + 1) >> 1;
+        if (eb[m] <= q << 2) a = m;
+        else b = m - 1;
+      }
+    s0 = a;
+  }
+  // The window at q: this lane's owner and its first slot there; true when
+  // the quad holds slots.  All 32 lanes, while q < end; moves on by a window.
+  __device__ __forceinline__ bool next(int &own, uint32_t &j0) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint64_t p0 = q << 2, pe = p0 + 4 * 32;
+    const int j = s0 + (int)lane;
+    const uint64_t bj = j <= GC ? eb[j] : ~0ull;
+    const uint32_t bit = (lane >= 1 && bj < pe) ? 1u << (uint32_t)((bj - p0) >> 2) : 0u;
+    const uint32_t m = __reduce_or_sync(0xFFFFFFFFu, bit);
+    own = s0 + __popc(m & (0xFFFFFFFFu >> (31 - lane)));
+    int ns = s0 + __popc(m);
+    if (ns < GC && eb[ns + 1] <= pe) ++ns;  // an entry starting exactly at pe
+    s0 = ns;
+    const bool in = q + lane < end && own < GC;
+    j0 = in ? (uint32_t)(p0 + 4 * lane - eb[own]) : 0u;
+    q += 32;
+    return in && j0 < len[own];
+  }
+};
+
 // Each CTA walks one contiguous run of units [u_begin, u_end), staging up to
-// CHUNK entries at a time in shared memory; each thread takes four
-// consecutive positions per iteration.
+// CHUNK entries at a time in shared memory; its warps share the chunk's
+// positions, each thread on four consecutive ones per step.
 template <class Op>
 __global__ void __launch_bounds__(RELAX_THREADS)
     seg_map(FrontierView in, FrontierView out, Op op, unsigned long long *edge_stat) {
@@ -95,22 +147,15 @@ __global__ void __launch_bounds__(RELAX_THREADS)
       __syncthreads();
       const uint64_t lo = max(E0, s_eb[0]);
       const uint64_t hi = min(E1, s_eb[CHUNK]);
-      for (uint64_t base = lo; base < hi; base += 4 * RELAX_THREADS) {
-        const uint64_t e = base + 4 * threadIdx.x;
+      WindowWalk<CHUNK> walk(s_eb, s_len, lo, hi, threadIdx.x >> 5, RELAX_THREADS / 32);
+      while (walk.q < walk.end) {
         bool app[4] = {false, false, false, false};
         uint32_t av[4] = {0, 0, 0, 0}, ad[4] = {0, 0, 0, 0};
-        if (e < hi) {
-          // largest i with s_eb[i] <= e
-          int l = 0, r = CHUNK - 1;
-          while (l < r) {
-            const int m = (l + r + 1) >> 1;
-            if (s_eb[m] <= e) l = m;
-            else r = m - 1;
-          }
-          const uint32_t j0 = (uint32_t)(e - s_eb[l]);
-          if (j0 < s_len[l]) counted += visit_quad(op, s_vtx[l], s_pay[l], j0, s_len[l], app, av, ad);
-        }
+        int l;
+        uint32_t j0;
+        if (walk.next(l, j0)) counted += visit_quad(op, s_vtx[l], s_pay[l], j0, s_len[l], app, av, ad);
         if (Op::kAppends) {
+          __syncwarp();
 #pragma unroll
           for (int k = 0; k < 4; ++k) frontier_append(out, app[k], av[k], ad[k]);
         }
