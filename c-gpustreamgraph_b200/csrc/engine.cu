@@ -988,13 +988,42 @@ struct sgs_engine {
   }
 
   template <class Op>
-  void launch_group(uint32_t rr, const Op &op) {
+  void launch_group(uint32_t rr, const Op &op, uint32_t lanes = 0, const unsigned long long *resets = nullptr,
+                    unsigned long long restrict_max = 0) {
     const bool hp = rr >= 1;
     auto k = host_tier() ? group_map<Op, true> : group_map<Op, false>;
     { ++n_launch; k<<<grid_map(), RELAX_THREADS, 0, s>>>(
         fview(rr, cnt.p + rr), fview(rr + 1, cnt.p + rr + 1), op,
         hp ? fb[(rr - 1) % 3].vtx.p : nullptr, hp ? cnt.p + rr - 1 : nullptr,
-        hp ? gm[(rr - 1) % 3].p : nullptr, b_lane.p, rstat.p + rr, hstat.p + rr); }
+        hp ? gm[(rr - 1) % 3].p : nullptr, b_lane.p, rstat.p + rr, hstat.p + rr, lanes, resets,
+        restrict_max); }
+  }
+
+  // Whether a narrow group's relaxation runs its round 0 as a launch of its own
+  // (cfg.persistent bit 2), which a repair may then restrict to the edges into
+  // reset vertices.
+  bool own_round0() const { return (cfg.persistent & 4u) && !(cfg.persistent & 1u); }
+  // Up to this many (lane, vertex) resets the restricted sweep is used: an
+  // eighth of the vertices, where about that share of the edges passes the
+  // filter.  (The update streams measured here reset 0.5 to 10 % of it.)
+  unsigned long long restrict_max() const { return std::max<uint32_t>(nv / 8, 1); }
+  DBuf<uint32_t> b_coarse;  // folded reset bitmap
+  void launch_sweep(Group &G, const GroupRelaxOp<GMAX> &op, unsigned long long rmax) {
+    uint32_t shift = 0;
+    while (((nv - 1) >> shift) >= SWEEP_FILTER_BITS) ++shift;
+    const uint32_t words = ((nv - 1) >> shift) / 32 + 1;
+    if (shift) {
+      b_coarse.ensure(words);
+      { ++n_launch; k_fold_bits<<<grid_elem(words), 256, 0, s>>>(G.ibits.p, (nv - 1) / 32 + 1, shift, b_coarse.p,
+                                                                 words); }
+    }
+    auto k = host_tier() ? k_group_sweep<true> : k_group_sweep<false>;
+    const size_t smem = sweep_smem(words);
+    CK(cudaFuncSetAttribute((const void *)k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    { ++n_launch; k<<<(uint32_t)nsm, SWEEP_THREADS, smem, s>>>(
+        fview(0, cnt.p), fview(1, cnt.p + 1), op, G.ibits.p, b_coarse.p, words, shift, (uint32_t)G.used, G.dstat.p,
+        rmax, rstat.p, hstat.p); }
+    CK(cudaGetLastError());
   }
 
   // BFS rounds of the lanes `lanes` (all BFS) of a narrow group, each round
@@ -1218,9 +1247,11 @@ struct sgs_engine {
   // `only0` (wide groups: per vertex the lanes reset there), round 0 relaxes
   // an edge only in the lanes its destination had reset, i.e. only edges into
   // bitmap; `after0` runs right after round 0 (it may append to frontier 1).
+  // rmax > 0 (narrow groups, own_round0): the repair after an invalidation;
+  // round 0 by the device's choice (RepairMode).
   uint32_t group_relax(Group &G, bool &conv, const char *round0 = nullptr,
                        const unsigned long long *only0 = nullptr,
-                       const std::function<void()> *after0 = nullptr) {
+                       const std::function<void()> *after0 = nullptr, unsigned long long rmax = 0) {
     GraphView g = view();
     if (G.wide()) {
       const bool anyw = G.sssp && cfg.weight_mode == SGS_W_EXPLICIT;
@@ -1245,7 +1276,7 @@ struct sgs_engine {
       return run_wide_rounds(op, op, conv, SGS_K_WIDE, anyw ? 8.0 : 4.0, nullptr, round0, after0);
     }
     const uint32_t anyw = G.any_sssp(G.used | 0xF) && cfg.weight_mode == SGS_W_EXPLICIT;
-    if ((cfg.persistent & 4u) && !(cfg.persistent & 1u) && !after0) {
+    if (own_round0() && !after0) {
       // round 0 (a snapshot's sweep, or a start's first round) as a plain
       // launch on the large grid, the rest of the phase as one cooperative
       // launch: the sweep wants the grid, the small later rounds want no
@@ -1254,15 +1285,21 @@ struct sgs_engine {
       CK(cudaMemsetAsync(hstat.p, 0, sizeof(unsigned long long) * (cfg.max_rounds + 2), s));
       if (round0) nvtxRangePushA(round0);
       if (ktiming) { ensure_kev(2); CK(cudaEventRecord(kev[0], s)); }
-      launch_group(0, GroupRelaxOp<GMAX>{g, G.st.p, G.val.p, gm[0].p, gm[1].p, G.algo(), anyw});
+      const GroupRelaxOp<GMAX> op0{g, G.st.p, G.val.p, gm[0].p, gm[1].p, G.algo(), anyw};
+      if (rmax) launch_sweep(G, op0, rmax);
+      launch_group(0, op0, (uint32_t)G.used, rmax ? G.dstat.p : nullptr, rmax);
       if (ktiming) {
         CK(cudaEventRecord(kev[1], s));
-        unsigned long long c0 = 0, r0s = 0, h0 = 0;
+        unsigned long long c0 = 0, r0s = 0, h0 = 0, rs[GMAX] = {}, nr = 0;
+        if (rmax) CK(cudaMemcpyAsync(rs, G.dstat.p, sizeof(rs), cudaMemcpyDeviceToHost, s));
         CK(cudaMemcpyAsync(&c0, cnt.p, sizeof(c0), cudaMemcpyDeviceToHost, s));
         CK(cudaMemcpyAsync(&r0s, rstat.p, sizeof(r0s), cudaMemcpyDeviceToHost, s));
         CK(cudaMemcpyAsync(&h0, hstat.p, sizeof(h0), cudaMemcpyDeviceToHost, s));
         sync();
-        account(SGS_K_GROUP_SWEEP, c0, r0s, anyw ? 8.0 : 4.0, 8.0, kev[0], kev[1], h0);
+        for (int q = 0; q < GMAX; ++q) nr += (G.used >> q & 1u) ? rs[q] : 0;
+        // the restricted sweep reads weights only for the pairs it relaxes
+        const bool restricted = rmax && nr && nr <= rmax;
+        account(SGS_K_GROUP_SWEEP, c0, r0s, anyw && !restricted ? 8.0 : 4.0, 8.0, kev[0], kev[1], h0);
       }
       if (round0) nvtxRangePop();
       return run_group_persistent(GroupRelaxOp<GMAX>{g, G.st.p, G.val.p, nullptr, nullptr, G.algo(), anyw}, 1,
@@ -2340,12 +2377,12 @@ struct sgs_engine {
       if (G.wide()) {  // the lanes this invalidation resets, per vertex
         G.wreset.ensure(nv);
         CK(cudaMemsetAsync(G.wreset.p, 0, sizeof(unsigned long long) * nv, s));
-      } else if (prep) {  // bitmap of the vertices this invalidation resets
+      } else if (prep || own_round0()) {  // bitmap of the vertices this invalidation resets
         const size_t nw = (size_t)nv / 32 + 1;
         G.ibits.ensure(nw);
         CK(cudaMemsetAsync(G.ibits.p, 0, sizeof(uint32_t) * nw, s));
       }
-      uint32_t *nmark = prep ? G.ibits.p : nullptr;  // narrow groups mark only for the pull repair
+      uint32_t *nmark = prep || own_round0() ? G.ibits.p : nullptr;
       bool conv = false;
       if (G.wide()) {
         { ++n_launch; k_wide_seed_deleted<<<grid_elem(nd), 256, 0, s>>>(
@@ -2434,17 +2471,15 @@ struct sgs_engine {
       }
     }
     // ---- add phase per group.  After an invalidation the reference re-pushes
-    // from every reached vertex (SyncPushDDBAll), and so do narrow groups.
-    // In a wide group that first round visits the same edges but relaxes
-    // only those into vertices reset in this snapshot (bitmap G.ibits), and
-    // the kept inserted edges are relaxed right after it: before the repair,
-    // every other edge (u,v) already satisfies value(u) + w >= value(v) -- u
-    // kept a value that was valid on the old graph, v kept its own, and the
-    // edge existed -- so these two sets hold every violated edge.  Later
-    // rounds are unrestricted, so the fixed point is the same.  (For a narrow
-    // group the 16-B state row costs no more than the bitmap probe, so the
-    // restriction does not pay.)  Without invalidation only the inserted
-    // edges are relaxed.  Then rounds to convergence.
+    // from every reached vertex (SyncPushDDBAll).  Here that first round visits
+    // the same edges but relaxes only those into vertices reset in this
+    // snapshot, and the kept inserted edges are relaxed beside it: before the
+    // repair, every other edge (u,v) already satisfies value(u) + w >= value(v)
+    // -- u kept a value that was valid on the old graph, v kept its own, and
+    // the edge existed -- so these two sets hold every violated edge.  Later
+    // rounds are unrestricted, so the fixed point is the same.  (A narrow group
+    // does so unless much was reset, see RepairMode.)  Without invalidation
+    // only the inserted edges are relaxed.  Then rounds to convergence.
     for (size_t i = 0; i < ng; ++i) {
       Group &G = *groups[i];
       if (!G.used) continue;
@@ -2459,6 +2494,7 @@ struct sgs_engine {
       // the path is chosen on the device from the group's reset counts
       // (G.dstat[0, 64)): the dense frontier only if a lane was reset
       const unsigned long long *resets = G.dstat.p;
+      const unsigned long long rmax = !G.wide() && gdel[i] && own_round0() ? restrict_max() : 0;
       if (!G.wide() && prep) {  // work-efficient repair: pull into the reset vertices
         bool conv = false;
         grounds[i] = pull_repair(G, gdel[i] != 0, ni, explicit_w);
@@ -2473,11 +2509,11 @@ struct sgs_engine {
                                                                fview(0, cnt.p), resets); }
       else
         { ++n_launch; k_group_dense<GMAX><<<grid_elem(nv), 256, 0, s>>>(g, G.val.p, (uint32_t)G.used, G.algo(),
-                                                            gm[0].p, fview(0, cnt.p), resets); }
-      if (ni && !G.wide())  // narrow, nothing reset: only the inserted edges
+                                                            gm[0].p, fview(0, cnt.p), resets, rmax, b_lane.p); }
+      if (ni && !G.wide())  // narrow, the sweep does not cover them
         { ++n_launch; k_group_relax_inserted<GMAX><<<grid_elem(ni), 256, 0, s>>>(
             g, G.st.p, G.val.p, (uint32_t)G.used, G.algo(), b_ikept.p, explicit_w ? b_iw_kept.p : nullptr,
-            b_nkept.p, gm[0].p, fview(0, cnt.p), b_lane.p, resets); }
+            b_nkept.p, gm[0].p, fview(0, cnt.p), b_lane.p, resets, rmax, gm[1].p, fview(1, cnt.p + 1)); }
       CK(cudaGetLastError());
       if (stage_wanted()) stage_host();  // explicit host policy: repair reads an HBM copy
       // wide: the inserted edges after the restricted round 0, into its
@@ -2489,7 +2525,7 @@ struct sgs_engine {
       };
       bool conv = false;
       grounds[i] = G.wide() ? group_relax(G, conv, "sgs:sweep", G.wreset.p, ni ? &ins_after0 : nullptr)
-                            : group_relax(G, conv, "sgs:sweep");
+                            : group_relax(G, conv, "sgs:sweep", nullptr, nullptr, rmax);
       if (!conv) fail(SGS_ERR_NOCONV, "round limit reached before convergence");
       CK(cudaEventRecord(gev[4 * i + 3], s));
       CK(cudaMemcpyAsync(G.dstat.p + 2 * WLANES, b_lane.p, sizeof(unsigned long long) * WLANES,

@@ -65,6 +65,26 @@ __device__ __forceinline__ void load_vals(const uint32_t *val, uint32_t v, uint3
   }
 }
 
+// How a narrow group's repair starts, decided on the device from the reset
+// counts of the invalidation (per lane), the same in every kernel involved:
+//  NONE        nothing was reset: only the inserted edges are relaxed;
+//  RESTRICTED  round 0 walks every reached vertex's edges but relaxes only
+//              those into reset vertices (k_group_sweep), and the inserted
+//              edges are relaxed beside it: all other edges already satisfy
+//              value(u) + w >= value(v), so these hold every violated one;
+//  FULL        round 0 relaxes every edge (group_map), when more than
+//              `restrict_max` (lane, vertex) pairs were reset -- the filter
+//              then passes so many edges that testing them costs more.
+enum RepairMode : int { REPAIR_NONE = 0, REPAIR_RESTRICTED = 1, REPAIR_FULL = 2 };
+__device__ __forceinline__ int repair_mode(const unsigned long long *resets, uint32_t lanes,
+                                           unsigned long long restrict_max) {
+  unsigned long long n = 0;
+#pragma unroll
+  for (int q = 0; q < GMAX; ++q)
+    if (lanes >> q & 1u) n += __ldg(resets + q);
+  return n == 0 ? REPAIR_NONE : n <= restrict_max ? REPAIR_RESTRICTED : REPAIR_FULL;
+}
+
 // Clears the masks of the previous frontier (grid-stride, all threads).
 __device__ __forceinline__ void clear_prev_masks(const uint32_t *vtx, const unsigned long long *cnt,
                                                  uint32_t *mask) {
@@ -457,7 +477,10 @@ __global__ void __launch_bounds__(RELAX_THREADS, SGS_GROUP_MIN_BLOCKS)
     group_map(FrontierView in, FrontierView out, Op op, const uint32_t *prev_vtx,
               const unsigned long long *prev_cnt, uint32_t *prev_mask,
               unsigned long long *lane_edges, unsigned long long *edge_stat,
-              unsigned long long *host_stat) {
+              unsigned long long *host_stat, uint32_t lanes = 0,
+              const unsigned long long *resets = nullptr, unsigned long long restrict_max = 0) {
+  // round 0 of a repair that k_group_sweep has done
+  if (resets && repair_mode(resets, lanes, restrict_max) == REPAIR_RESTRICTED) return;
   group_map_body<Op, H>(in, out, op, prev_vtx, prev_cnt, prev_mask, lane_edges, edge_stat, host_stat);
 }
 
@@ -538,43 +561,350 @@ __global__ void k_group_init_lane(unsigned long long *st, uint32_t *val, uint32_
 }
 
 // Every vertex with a non-empty block; mask = selected lanes whose value is
-// finite there (CC lanes always).  One writer per vertex: plain stores.
-// With `only_if_reset`, the launch does nothing unless a selected lane was
-// reset by the last invalidation (its per-lane counts).
+// finite there (CC lanes always).  One writer per vertex: plain stores.  With
+// `resets`: nothing in mode NONE; in mode RESTRICTED no masks (k_group_sweep
+// reads none) but the (lane, edge) pairs of the sweep added to lane_edges.
+// Bound by memory: 20 B read and 16-20 B written per vertex.  A warp takes 32
+// consecutive vertices per step (one 512-B read of their values) and scans
+// the eight steps of its 256 one after the other; the block appends its 2048
+// vertices, in order, with one atomic.
 template <int S>
-__global__ void k_group_dense(GraphView g, const uint32_t *val, uint32_t lanes,
-                              LaneAlgo algo, uint32_t *m_out, FrontierView out,
-                              const unsigned long long *only_if_reset = nullptr) {
-  if (only_if_reset && !block_any_lane(only_if_reset, lanes)) return;
-  // eight consecutive vertices per thread, one block append per 2048
-  constexpr int N = 8;
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x * N;
-  for (uint64_t b = (uint64_t)blockIdx.x * blockDim.x * N; b < g.nv; b += stride) {
-    const uint64_t v0 = b + (uint64_t)threadIdx.x * N;
-    bool want[N];
-    uint32_t d[N];
+__global__ void __launch_bounds__(RELAX_THREADS)
+    k_group_dense(GraphView g, const uint32_t *val, uint32_t lanes, LaneAlgo algo, uint32_t *m_out,
+                  FrontierView out, const unsigned long long *resets = nullptr,
+                  unsigned long long restrict_max = 0, unsigned long long *lane_edges = nullptr) {
+  constexpr int N = 8, NW = RELAX_THREADS / 32;
+  __shared__ unsigned long long s_warp[NW], s_base;
+  const int mode = resets ? repair_mode(resets, lanes, restrict_max) : REPAIR_FULL;
+  if (mode == REPAIR_NONE) return;
+  const unsigned full = 0xFFFFFFFFu;
+  const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  unsigned long long edges[S] = {};
+  const uint64_t stride = (uint64_t)gridDim.x * RELAX_THREADS * N;
+  for (uint64_t b = (uint64_t)blockIdx.x * RELAX_THREADS * N; b < g.nv; b += stride) {
+    const uint64_t v0 = b + (uint64_t)wid * 32 * N + lane;
+    uint32_t d[N], m[N];
+    uint32_t blk[N][S];
+#pragma unroll
+    for (int i = 0; i < N; ++i) d[i] = v0 + 32 * i < g.nv ? g.slots[v0 + 32 * i] : 0u;
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+      if (d[i]) load_vals<S>(val, (uint32_t)(v0 + 32 * i), blk[i]);
 #pragma unroll
     for (int i = 0; i < N; ++i) {
-      const uint64_t v = v0 + i;
-      want[i] = false;
-      d[i] = 0;
-      if (v < g.nv) {
-        d[i] = g.slots[v];
-        if (d[i]) {
-          uint32_t blk[S];
-          load_vals<S>(val, (uint32_t)v, blk);
-          uint32_t m = 0;
+      m[i] = 0;
+      if (d[i]) {
 #pragma unroll
-          for (int q = 0; q < S; ++q)
-            if ((lanes >> q & 1u) && (algo.at(q) == A_CC || blk[q] != INF32)) m |= 1u << q;
-          if (m) {
-            m_out[v] = m;
-            want[i] = true;
-          }
+        for (int q = 0; q < S; ++q)
+          if ((lanes >> q & 1u) && (algo.at(q) == A_CC || blk[i][q] != INF32)) m[i] |= 1u << q;
+        if (mode == REPAIR_RESTRICTED && m[i]) {
+          const uint32_t l = g.live[v0 + 32 * i];
+#pragma unroll
+          for (int q = 0; q < S; ++q) edges[q] += (m[i] >> q & 1u) ? l : 0u;
         }
       }
     }
-    frontier_append_block_n<N>(out, want, (uint32_t)v0, d);
+    // inclusive scans of the (count, padded slots) words, step after step
+    unsigned long long x[N], run = 0;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      x[i] = m[i] ? (1ull << CNT_SHIFT) | (unsigned long long)((d[i] + 3u) & ~3u) : 0ull;
+#pragma unroll
+      for (int s = 1; s < 32; s <<= 1) {
+        const unsigned long long y = __shfl_up_sync(full, x[i], s);
+        if (lane >= (uint32_t)s) x[i] += y;
+      }
+      x[i] += run;
+      run = __shfl_sync(full, x[i], 31);
+    }
+    if (lane == 0) s_warp[wid] = run;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      unsigned long long t = 0;
+      for (int w = 0; w < NW; ++w) {
+        const unsigned long long y = s_warp[w];
+        s_warp[w] = t;
+        t += y;
+      }
+      s_base = t ? atomicAdd((unsigned long long *)out.counter, t) : 0ull;
+    }
+    __syncthreads();
+    const unsigned long long base = s_base + s_warp[wid];
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      if (!m[i]) continue;
+      const uint32_t v = (uint32_t)(v0 + 32 * i), dp = (d[i] + 3u) & ~3u;
+      const unsigned long long pos = base + x[i] - ((1ull << CNT_SHIFT) | (unsigned long long)dp);
+      const uint32_t slot = (uint32_t)(pos >> CNT_SHIFT);
+      const uint64_t eb = pos & EDGE_MASK;
+      out.vtx[slot] = v;
+      out.len[slot] = d[i];
+      out.ebase[slot] = eb;
+      const uint64_t u0 = (eb + UNIT - 1) / UNIT, u1 = (eb + dp - 1) / UNIT;
+      for (uint64_t u = u0; u <= u1 && u < out.ucap; ++u) out.ustart[u] = slot;
+      if (mode == REPAIR_FULL) m_out[v] = m[i];
+    }
+    __syncthreads();  // s_warp / s_base are rewritten by the next step
+  }
+  if (lane_edges && mode == REPAIR_RESTRICTED) {
+#pragma unroll
+    for (int q = 0; q < S; ++q) {
+      const unsigned long long e = warp_sum(edges[q]);
+      if (lane == 0 && e) atomicAdd(&lane_edges[q], e);
+    }
+  }
+}
+
+// Coarse form of the reset bitmap for k_group_sweep's shared-memory filter: bit
+// b = some vertex of [b << shift, (b + 1) << shift) was reset.
+__global__ void k_fold_bits(const uint32_t *bits, uint32_t nwords, uint32_t shift, uint32_t *coarse,
+                            uint32_t cwords) {
+  for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < cwords; c += gridDim.x * blockDim.x) {
+    uint32_t o = 0;
+    for (uint32_t b = 0; b < 32; ++b) {
+      const uint64_t v0 = ((uint64_t)c * 32 + b) << shift;
+      uint32_t any = 0;
+      if (shift >= 5) {
+        for (uint64_t w = v0 >> 5; w < (v0 >> 5) + (1u << (shift - 5)) && w < nwords; ++w) any |= bits[w];
+      } else if ((v0 >> 5) < nwords) {
+        any = bits[v0 >> 5] >> (v0 & 31) & ((1u << (1u << shift)) - 1u);
+      }
+      if (any) o |= 1u << b;
+    }
+    coarse[c] = o;
+  }
+}
+
+// Round 0 of a narrow group's repair in mode RESTRICTED: a walk of the ids of
+// every reached vertex's block (the dense frontier), in which only the edges
+// into reset vertices are relaxed.
+//
+// The full sweep reads a random 16-B mirror row per slot, and that gather
+// (one L1 tag per slot, and DRAM for the rows that miss L2), not the id
+// stream, sets its time.  Here a slot costs one bit of a filter in shared
+// memory: the reset bitmap, for up to 2^20 vertices exactly, above that one bit
+// per 2^shift consecutive vertices, with the exact bitmap probed for the slots
+// that pass.  What passes goes through per-warp queues and is handled 32
+// edges at a time, so the few edges per window that need the rows of both
+// ends do not stall the walk with mostly idle warps.
+// One CTA of 32 warps per SM (the filter takes 128 KB); every warp walks its
+// own run of units with 32 staged entries, two windows of ids in flight, and
+// no barrier.  With 65 % of a million-vertex graph in host memory a snapshot
+// goes from 4.9 to 3.6 ms, since weights are read for the few relaxed edges only;
+// with all of it in HBM the sweep takes as long as the full one (1.56 and 1.67 ms
+// at scale 24).
+constexpr int SWEEP_THREADS = 1024;
+constexpr uint32_t SWEEP_FILTER_BITS = 1u << 20;
+struct SweepWarp {
+  uint64_t eb[33], off[32];
+  uint32_t len[32], vtx[32];
+  // queues: up to 31 waiting and 32 new
+  uint32_t q1_dst[63], q1_src[63], q1_j[63];
+  uint32_t q2_dst[63], q2_src[63], q2_j[63];
+  uint32_t app[WarpQueue::CAP];
+};
+inline size_t sweep_smem(uint32_t filter_words) {
+  return sizeof(SweepWarp) * (SWEEP_THREADS / 32) + ((size_t)filter_words + 3) / 4 * 16;
+}
+
+template <bool H>
+__global__ void __launch_bounds__(SWEEP_THREADS, 1)
+    k_group_sweep(FrontierView in, FrontierView out, GroupRelaxOp<GMAX> op, const uint32_t *bits,
+                  const uint32_t *coarse, uint32_t filter_words, uint32_t shift, uint32_t lanes,
+                  const unsigned long long *resets, unsigned long long restrict_max,
+                  unsigned long long *edge_stat, unsigned long long *host_stat) {
+  if (repair_mode(resets, lanes, restrict_max) != REPAIR_RESTRICTED) return;
+  extern __shared__ __align__(16) unsigned char s_raw[];
+  SweepWarp &sw = reinterpret_cast<SweepWarp *>(s_raw)[threadIdx.x >> 5];
+  uint32_t *filter = reinterpret_cast<uint32_t *>(s_raw + sizeof(SweepWarp) * (SWEEP_THREADS / 32));
+  const uint32_t *f_src = shift ? coarse : bits;
+  for (uint32_t i = threadIdx.x; i < filter_words; i += SWEEP_THREADS) filter[i] = f_src[i];
+  __syncthreads();
+  const GraphView &g = op.g;
+  const uint32_t lane = threadIdx.x & 31;
+  const uint64_t packed = __ldcg((const unsigned long long *)in.counter);
+  const uint32_t n = (uint32_t)(packed >> CNT_SHIFT);
+  const uint64_t T = packed & EDGE_MASK;
+  const uint64_t nunits = (T + UNIT - 1) / UNIT;
+  // a small frontier's units go to warps of different SMs
+  const uint64_t w = (uint64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+  const uint64_t W = (uint64_t)gridDim.x * (SWEEP_THREADS / 32);
+  const uint64_t ub = w * nunits / W, ue = (w + 1) * nunits / W;
+  WarpQueue queue(sw.app);
+  auto len_of = [&](uint32_t v) { return g.slots[v]; };
+  uint32_t evald = 0, host_acc = 0;
+  unsigned long long host_all = 0;
+  uint32_t n1 = 0, n2 = 0;  // queued edges (warp-uniform)
+  // relaxes the last min(n2, 32) of queue 2
+  auto relax = [&]() {
+    const uint32_t c = min(n2, 32u);
+    const bool on = lane < c;
+    uint32_t d = 0, u = 0, j = 0;
+    if (on) {
+      d = sw.q2_dst[n2 - c + lane];
+      u = sw.q2_src[n2 - c + lane];
+      j = sw.q2_j[n2 - c + lane];
+    }
+    n2 -= c;
+    __syncwarp();
+    bool want = false;
+    if (on) {
+      uint32_t su[GMAX], cur[GMAX];
+      load_vals<GMAX>(op.val, u, su);
+      load_vals<GMAX>(op.val, d, cur);
+      uint32_t wt = 1;
+      if (op.any_w) {
+        if (g.wmode == W_EXPLICIT) wt = H ? *wgt_at(g, g.off[u], j) : g.wgt_d[g.off[u] + j];
+        else if (g.wmode == W_SYNTH) wt = (u + d) % 128u + 1u;
+      } else if (g.wmode == W_SYNTH) {
+        wt = (u + d) % 128u + 1u;
+      }
+      uint32_t got = 0;
+#pragma unroll
+      for (int q = 0; q < GMAX; ++q) {
+        if (!(lanes >> q & 1u)) continue;
+        if (su[q] == INF32 && !(op.algo.cc >> q & 1u)) continue;
+        ++evald;
+        const uint32_t cand = op.cand_of(su[q] + (op.algo.inc >> q & 1u), wt, q);
+        if (cand >= cur[q]) continue;
+        const uint64_t idx = (uint64_t)d * GMAX + q;
+        if (relax_mirror_packed(&op.val[idx], &op.st[idx], cand, u)) got |= 1u << q;
+      }
+      want = got && g.slots[d] && atomicOr(&op.m_out[d], got) == 0u;
+    }
+    queue.push(out, want, d, len_of);
+  };
+  // probes the exact bitmap for the last min(n1, 32) of queue 1
+  auto probe = [&]() {
+    const uint32_t c = min(n1, 32u);
+    bool on = lane < c;
+    uint32_t d = 0, u = 0, j = 0;
+    if (on) {
+      d = sw.q1_dst[n1 - c + lane];
+      u = sw.q1_src[n1 - c + lane];
+      j = sw.q1_j[n1 - c + lane];
+      on = __ldg(bits + (d >> 5)) >> (d & 31) & 1u;
+    }
+    n1 -= c;
+    const uint32_t m = __ballot_sync(0xFFFFFFFFu, on);
+    if (on) {
+      const uint32_t at = n2 + __popc(m & ((1u << lane) - 1u));
+      sw.q2_dst[at] = d;
+      sw.q2_src[at] = u;
+      sw.q2_j[at] = j;
+    }
+    n2 += __popc(m);
+    __syncwarp();
+    if (n2 >= 32) relax();
+  };
+  if (n != 0 && ub < ue) {
+    const uint64_t E0 = ub * UNIT, E1 = min(ue * (uint64_t)UNIT, T);
+    uint32_t s = __ldcg(&in.ustart[ub]);
+    for (;;) {
+      const uint32_t idx = s + lane;
+      const uint64_t eb = idx < n ? __ldcg((const unsigned long long *)&in.ebase[idx]) : T;
+      if (lane == 0) sw.eb[32] = s + 32 < n ? __ldcg((const unsigned long long *)&in.ebase[s + 32]) : T;
+      sw.eb[lane] = eb;
+      if (idx < n && eb < E1) {
+        const uint32_t v = __ldcg(&in.vtx[idx]), l = __ldcg(&in.len[idx]);
+        uint64_t o = g.off[v];
+        if constexpr (H) {
+          if (o & HOST_BIT) {
+            if (eb >= E0) {
+              hot_bump(g, v, o);
+              host_all += l;
+            }
+            o = resolve_block(g, o, l);
+          }
+        }
+        sw.vtx[lane] = v;
+        sw.len[lane] = l;
+        sw.off[lane] = o;
+      }
+      __syncwarp();
+      WindowWalk<32> walk(sw.eb, sw.len, max(E0, sw.eb[0]), min(E1, sw.eb[32]), 0, 1);
+      struct Win {
+        int own;
+        uint32_t j;
+        bool has;
+        uint4 ids;
+      };
+      auto fetch = [&](Win &x) -> bool {
+        if (walk.q >= walk.end) return false;
+        x.has = walk.next(x.own, x.j);
+        if (x.has) x.ids = ld_quad_stream(H ? adj_at(g, sw.off[x.own], x.j) : g.adj_d + sw.off[x.own] + x.j);
+        return true;
+      };
+      Win a{}, b{};
+      bool more = fetch(a), more_b = more && fetch(b);
+      while (more) {
+        Win c{};
+        const bool more_c = more_b && fetch(c);
+        const uint32_t left = a.has ? sw.len[a.own] - a.j : 0u;
+        const uint32_t u = a.has ? sw.vtx[a.own] : 0u;
+        if constexpr (H) {
+          if (a.has) {
+            const uint64_t o = sw.off[a.own];
+            if ((o & HOST_BIT) && cache_line(g, (o & OFF_MASK) + a.j) == NO_LINE) host_acc += min(4u, left);
+          }
+        }
+        uint32_t hit = 0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const uint32_t d = quad_at(a.ids, k), f = d >> shift;
+          if ((uint32_t)k < left && d != SGS_TOMB && (filter[f >> 5] >> (f & 31) & 1u)) hit |= 1u << k;
+        }
+        if (__ballot_sync(0xFFFFFFFFu, hit != 0u)) {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const bool h = hit >> k & 1u;
+            const uint32_t m = __ballot_sync(0xFFFFFFFFu, h);
+            if (!m) continue;
+            const uint32_t at = __popc(m & ((1u << lane) - 1u));
+            if (shift) {
+              if (h) {
+                sw.q1_dst[n1 + at] = quad_at(a.ids, k);
+                sw.q1_src[n1 + at] = u;
+                sw.q1_j[n1 + at] = a.j + k;
+              }
+              n1 += __popc(m);
+              __syncwarp();
+              if (n1 >= 32) probe();
+            } else {
+              if (h) {
+                sw.q2_dst[n2 + at] = quad_at(a.ids, k);
+                sw.q2_src[n2 + at] = u;
+                sw.q2_j[n2 + at] = a.j + k;
+              }
+              n2 += __popc(m);
+              __syncwarp();
+              if (n2 >= 32) relax();
+            }
+          }
+        }
+        a = b;
+        b = c;
+        more = more_b;
+        more_b = more_c;
+      }
+      __syncwarp();  // the staged entries are rewritten below
+      if (sw.eb[32] >= E1 || s + 32 >= n) break;
+      s += 32;
+      __syncwarp();
+    }
+    if (n1) probe();
+    if (n2) relax();
+    queue.flush(out, 32, len_of);
+  }
+  const unsigned long long ev = warp_sum((unsigned long long)evald);
+  if (lane == 0 && ev && edge_stat) atomicAdd(edge_stat, ev);
+  if constexpr (H) {
+    const unsigned long long hs = warp_sum((unsigned long long)host_acc), ha = warp_sum(host_all);
+    if (lane == 0 && hs && host_stat) atomicAdd(host_stat, hs);
+    if (lane == 0 && g.cstat) {
+      if (ha) atomicAdd(&g.cstat[0], ha);
+      if (hs) atomicAdd(&g.cstat[1], hs);
+    }
   }
 }
 
@@ -631,15 +961,27 @@ __global__ void k_group_seed_deleted(GraphView g, unsigned long long *st, uint32
 // Relaxes just the kept inserted edges in the selected lanes: the whole
 // repair of an insert-only batch, and the inserted-edge half of the repair
 // after an invalidation (the other half is the restricted first round).
-// With `skip_if_reset`, the launch does nothing when a selected lane was
-// reset by the last invalidation (the full sweep covers the inserted edges).
+// With `resets` the repair's mode decides: FULL, nothing (the full sweep
+// covers the inserted edges); RESTRICTED, improved vertices go to frontier 1
+// (out1, m_out1) and the edges are not counted (the sweep's count has them);
+// NONE, to frontier 0 (out, m_out).
 template <int S>
 __global__ void k_group_relax_inserted(GraphView g, unsigned long long *st, uint32_t *val, uint32_t lanes,
                                        LaneAlgo algo, const uint64_t *keys, const uint32_t *w,
                                        const uint32_t *n_ptr, uint32_t *m_out, FrontierView out,
                                        unsigned long long *lane_edges,
-                                       const unsigned long long *skip_if_reset = nullptr) {
-  if (skip_if_reset && block_any_lane(skip_if_reset, lanes)) return;
+                                       const unsigned long long *resets = nullptr,
+                                       unsigned long long restrict_max = 0, uint32_t *m_out1 = nullptr,
+                                       FrontierView out1 = FrontierView{}) {
+  if (resets) {
+    const int mode = repair_mode(resets, lanes, restrict_max);
+    if (mode == REPAIR_FULL) return;
+    if (mode == REPAIR_RESTRICTED) {
+      out = out1;
+      m_out = m_out1;
+      lane_edges = nullptr;
+    }
+  }
   const uint32_t n = *n_ptr;
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   uint32_t counted = 0;
@@ -683,7 +1025,7 @@ __global__ void k_group_relax_inserted(GraphView g, unsigned long long *st, uint
     }
     frontier_append(out, want, v, d);
   }
-  if (counted) {
+  if (counted && lane_edges) {
 #pragma unroll
     for (int q = 0; q < S; ++q)
       if (lanes >> q & 1u) atomicAdd(&lane_edges[q], (unsigned long long)counted);
