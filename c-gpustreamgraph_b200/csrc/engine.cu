@@ -226,8 +226,9 @@ struct sgs_engine {
 
   // batch scratch
   DBuf<uint32_t> b_isrc, b_idst, b_iw, b_dsrc, b_ddst;
-  DBuf<uint64_t> b_ikeys, b_ikeys_s, b_ikept, b_dkeys, b_dkeys_s;
-  DBuf<uint32_t> b_iw_s, b_iw_kept, b_gstart;
+  DBuf<uint64_t> b_keys, b_keys_s, b_ikept, b_dkeys_s;  // sort keys; kept inserts and deletes, sorted
+  DBuf<uint32_t> b_vals, b_vals_s, b_iw_kept, b_gstart;
+  DBuf<uint32_t> b_counts;  // k_filter_inserts' kept counts
   DBuf<unsigned char> b_flag;
   DBuf<uint32_t> b_nkept;
   DBuf<unsigned int> b_err;
@@ -297,8 +298,7 @@ struct sgs_engine {
   DBuf<unsigned long long> in_top;     // [2]; tier 1 unused
   uint64_t in_capslots = 0;
   uint64_t in_builds = 0;
-  DBuf<uint64_t> t_dkeys, t_ikeys, t_tmp;  // the batch's keys transposed
-  DBuf<uint32_t> t_iw;                     // and the kept inserts' weights
+  DBuf<uint64_t> t_dkeys, t_ikeys;     // the batch's keys transposed
 
   // explicit-copy host policy (cfg.host_policy): the used host arena copied
   // to HBM by the copy engine for a snapshot's repair, readers pointed at it
@@ -638,15 +638,16 @@ struct sgs_engine {
   void in_apply(uint64_t ni, uint64_t nd, uint32_t nkept) {
     if (!in_built) return;
     const GraphView gi = in_view();
-    const int eb = sort_bits();
-    size_t tb = 0;
+    const uint64_t nk = ni ? nkept : 0, nt = nk + nd;
+    if (!nt) return;
+    ensure_keys(nt, in_w());
+    t_dkeys.ensure(batch_cap(nd));
+    t_ikeys.ensure(batch_cap(nk));
+    { ++n_launch; k_transpose_keys<<<grid_elem(nt), 256, 0, s>>>(b_ikept.p, b_iw_kept.p, nk, b_dkeys_s.p, nd,
+                                                                 id_bits(), b_keys.p, in_w() ? b_vals.p : nullptr); }
+    sort_keys(nt, in_w());
+    { ++n_launch; k_expand_keys<<<grid_elem(nt), 256, 0, s>>>(b_keys_s.p, nk, nd, id_bits(), t_ikeys.p, t_dkeys.p); }
     if (nd) {
-      t_dkeys.ensure(batch_cap(nd));
-      t_tmp.ensure(batch_cap(std::max<uint64_t>(nd, nkept)));
-      { ++n_launch; k_transpose_keys<<<grid_elem(nd), 256, 0, s>>>(b_dkeys_s.p, (uint32_t)nd, nullptr, t_tmp.p); }
-      CK(cub::DeviceRadixSort::SortKeys(nullptr, tb, t_tmp.p, t_dkeys.p, (int)nd, 0, eb, s));
-      cub_ensure(tb);
-      CK(cub::DeviceRadixSort::SortKeys(cub_tmp.p, tb, t_tmp.p, t_dkeys.p, (int)nd, 0, eb, s));
       CK(cudaMemsetAsync(special(4), 0, sizeof(unsigned long long) * 2, s));
       b_gstart.ensure((size_t)nv + 1);
       { ++n_launch; k_group_heads<<<grid_elem(nd), 256, 0, s>>>(gi, t_dkeys.p, nullptr, (uint32_t)nd, b_gstart.p,
@@ -657,23 +658,7 @@ struct sgs_engine {
       compact_blocks(gi, nd, b_reclaim.p + 1);
       CK(cudaGetLastError());
     }
-    if (!ni || !nkept) return;
-    t_ikeys.ensure(batch_cap(nkept));
-    t_tmp.ensure(batch_cap(nkept));
-    { ++n_launch; k_transpose_keys<<<grid_elem(nkept), 256, 0, s>>>(b_ikept.p, nkept, nullptr, t_tmp.p); }
-    tb = 0;
-    if (in_w()) {  // the kept inserts' weights travel with their transposed keys
-      t_iw.ensure(batch_cap(nkept));
-      CK(cub::DeviceRadixSort::SortPairs(nullptr, tb, t_tmp.p, t_ikeys.p, b_iw_kept.p, t_iw.p, (int)nkept, 0, eb,
-                                         s));
-      cub_ensure(tb);
-      CK(cub::DeviceRadixSort::SortPairs(cub_tmp.p, tb, t_tmp.p, t_ikeys.p, b_iw_kept.p, t_iw.p, (int)nkept, 0,
-                                         eb, s));
-    } else {
-      CK(cub::DeviceRadixSort::SortKeys(nullptr, tb, t_tmp.p, t_ikeys.p, (int)nkept, 0, eb, s));
-      cub_ensure(tb);
-      CK(cub::DeviceRadixSort::SortKeys(cub_tmp.p, tb, t_tmp.p, t_ikeys.p, (int)nkept, 0, eb, s));
-    }
+    if (!nk) return;
     InsertCtx c{};
     c.arena_top = in_top.p;
     c.arena_cap[0] = in_capslots;
@@ -702,7 +687,7 @@ struct sgs_engine {
     CK(cudaMemsetAsync(rl_count.p, 0, sizeof(unsigned long long), s));
     CK(cudaMemsetAsync(b_err.p, 0, sizeof(unsigned int), s));
     { ++n_launch; k_insert_plan<<<grid_elem(nkept), 256, 0, s>>>(gi, t_ikeys.p, b_nkept.p, c, 0, nullptr); }
-    { ++n_launch; k_insert_write<<<grid_elem(nkept), 256, 0, s>>>(gi, t_ikeys.p, in_w() ? t_iw.p : nullptr,
+    { ++n_launch; k_insert_write<<<grid_elem(nkept), 256, 0, s>>>(gi, t_ikeys.p, in_w() ? b_vals_s.p : nullptr,
                                                       b_nkept.p, wbase.p); }
     CK(cudaMemsetAsync(special(6), 0, sizeof(unsigned long long) * 2, s));
     { ++n_launch; k_reloc_frontier<<<grid_elem(nkept), 256, 0, s>>>(rl_count.p, rl_len.p, fview(0, special(6))); }
@@ -2139,12 +2124,11 @@ struct sgs_engine {
   // to, so that a later batch of at most that size allocates nothing (a
   // growth frees and allocates, and a free waits for the whole device).
   void reserve_batch(uint64_t ni, uint64_t nd) {
-    const size_t ci = batch_cap(ni), cd = batch_cap(nd), cm = batch_cap(std::max(ni, nd));
-    for (DBuf<uint32_t> *b : {&b_isrc, &b_idst, &b_iw, &b_iw_s, &b_iw_kept, &t_iw}) b->ensure(ci);
+    const size_t ci = batch_cap(ni), cd = batch_cap(nd);
+    for (DBuf<uint32_t> *b : {&b_isrc, &b_idst, &b_iw, &b_iw_kept}) b->ensure(ci);
     for (DBuf<uint32_t> *b : {&b_dsrc, &b_ddst}) b->ensure(cd);
-    for (DBuf<uint64_t> *b : {&b_ikeys, &b_ikeys_s, &b_ikept, &t_ikeys}) b->ensure(ci);
-    for (DBuf<uint64_t> *b : {&b_dkeys, &b_dkeys_s, &t_dkeys}) b->ensure(cd);
-    t_tmp.ensure(cm);
+    for (DBuf<uint64_t> *b : {&b_ikept, &t_ikeys}) b->ensure(ci);
+    for (DBuf<uint64_t> *b : {&b_dkeys_s, &t_dkeys}) b->ensure(cd);
     b_flag.ensure(ci);
     big_list.ensure(batch_cap(nd + 1));
     const size_t cr = batch_cap(ni + 1);
@@ -2152,20 +2136,47 @@ struct sgs_engine {
     rl_len.ensure(cr);
     rl_from.ensure(cr);
     rl_to.ensure(cr);
-    // the sorts and the selection of apply_batch and of the in-edge store's
-    // update, at the largest sizes
-    const int eb = sort_bits();
-    size_t tb = 0, t2 = 0, t3 = 0, t4 = 0;
-    if (nd || ni)
-      CK(cub::DeviceRadixSort::SortKeys(nullptr, tb, b_dkeys.p, b_dkeys_s.p, (int)std::max(ni, nd), 0, eb, s));
-    if (ni) {
-      CK(cub::DeviceRadixSort::SortPairs(nullptr, t2, b_ikeys.p, b_ikeys_s.p, b_iw.p, b_iw_s.p, (int)ni, 0,
-                                         eb, s));
-      CK(cub::DeviceSelect::Flagged(nullptr, t3, b_ikeys_s.p, b_flag.p, b_ikept.p, b_nkept.p, (int)ni, s));
-      CK(cub::DeviceRadixSort::SortPairs(nullptr, t4, t_tmp.p, t_ikeys.p, b_iw_kept.p, t_iw.p, (int)ni, 0,
-                                         eb, s));
+    // the sorts of apply_batch and of the in-edge store's update, at the
+    // largest size
+    ensure_keys(std::max<uint64_t>(ni + nd, 1), true);
+    size_t t1 = 0, t2 = 0;
+    CK(sort_call(nullptr, t1, ni + nd, false));
+    CK(sort_call(nullptr, t2, ni + nd, true));
+    cub_ensure(std::max(t1, t2));
+  }
+
+  // The radix sort of a batch's keys (k_batch_keys): b_keys -> b_keys_s, with
+  // values b_vals -> b_vals_s.
+  int id_bits() const {
+    int b = 1;
+    while (b < 32 && (1ull << b) < nv) ++b;
+    return b;
+  }
+  void ensure_keys(uint64_t n, bool vals) {
+    const size_t c = batch_cap(n);
+    b_keys.ensure(c);
+    b_keys_s.ensure(c);
+    if (vals) {
+      b_vals.ensure(c);
+      b_vals_s.ensure(c);
     }
-    cub_ensure(std::max(std::max(tb, t2), std::max(t3, t4)));
+  }
+  cudaError_t sort_call(void *tmp, size_t &bytes, uint64_t n, bool vals) {
+    const int eb = 2 * id_bits() + 1;
+    // (a list of 2^31 or more takes 64-bit counts)
+    if (n >= (1ull << 31))
+      return vals ? cub::DeviceRadixSort::SortPairs(tmp, bytes, b_keys.p, b_keys_s.p, b_vals.p, b_vals_s.p, n, 0,
+                                                    eb, s)
+                  : cub::DeviceRadixSort::SortKeys(tmp, bytes, b_keys.p, b_keys_s.p, n, 0, eb, s);
+    return vals ? cub::DeviceRadixSort::SortPairs(tmp, bytes, b_keys.p, b_keys_s.p, b_vals.p, b_vals_s.p, (int)n, 0,
+                                                  eb, s)
+                : cub::DeviceRadixSort::SortKeys(tmp, bytes, b_keys.p, b_keys_s.p, (int)n, 0, eb, s);
+  }
+  void sort_keys(uint64_t n, bool vals) {
+    size_t tb = 0;
+    CK(sort_call(nullptr, tb, n, vals));
+    cub_ensure(tb);
+    CK(sort_call(cub_tmp.p, tb, n, vals));
   }
 
   // Tombstone reclamation of the blocks touched by this snapshot's nd
@@ -2218,12 +2229,6 @@ struct sgs_engine {
                                             1, conv, SGS_K_GROUP, anyw ? 8.0 : 4.0);
     if (!conv) fail(SGS_ERR_NOCONV, "round limit reached before convergence");
     return r;
-  }
-
-  int sort_bits() const {
-    int b = 1;
-    while (b < 32 && (1ull << b) < nv) ++b;
-    return 32 + b;
   }
 
   // The current layout as user algorithms see it (sgs_graph_view).
@@ -2291,38 +2296,28 @@ struct sgs_engine {
     upload(b_ddst, dd, nd, mem);
     if (staged_in) CK(cudaEventRecord(staged_in->consumed, s));  // its slot may be refilled
     const size_t ci = batch_cap(ni), cd = batch_cap(nd);
-    b_ikeys.ensure(ci); b_ikeys_s.ensure(ci); b_ikept.ensure(ci);
-    b_iw_s.ensure(ci); b_iw_kept.ensure(ci); b_flag.ensure(ci);
-    b_dkeys.ensure(cd); b_dkeys_s.ensure(cd);
+    b_ikept.ensure(ci);
+    b_iw_kept.ensure(ci);
+    b_flag.ensure(ci);
+    b_dkeys_s.ensure(cd);
     CK(cudaMemsetAsync(b_err.p, 0, sizeof(unsigned int), s));
     CK(cudaMemsetAsync(b_stat.p, 0, sizeof(unsigned long long) * 8, s));
-    if (ni)
-      { ++n_launch; k_make_keys<<<grid_elem(ni), 256, 0, s>>>(b_isrc.p, b_idst.p, ni, nv, b_ikeys.p,
-                                                explicit_w ? b_iw.p : nullptr, explicit_w, b_err.p); }
-    if (nd)
-      { ++n_launch; k_make_keys<<<grid_elem(nd), 256, 0, s>>>(b_dsrc.p, b_ddst.p, nd, nv, b_dkeys.p, nullptr, 0,
-                                                b_err.p); }
-    const int eb = sort_bits();
-    size_t tb = 0, t2 = 0, t3 = 0;
-    if (nd) CK(cub::DeviceRadixSort::SortKeys(nullptr, tb, b_dkeys.p, b_dkeys_s.p, (int)nd, 0, eb, s));
-    if (ni) {
-      CK(cub::DeviceRadixSort::SortPairs(nullptr, t2, b_ikeys.p, b_ikeys_s.p,
-                                         explicit_w ? b_iw.p : b_isrc.p, b_iw_s.p, (int)ni, 0, eb, s));
-      CK(cub::DeviceSelect::Flagged(nullptr, t3, b_ikeys_s.p, b_flag.p, b_ikept.p, b_nkept.p, (int)ni, s));
-    }
-    cub_ensure(std::max(tb, std::max(t2, t3)));
-    if (nd) CK(cub::DeviceRadixSort::SortKeys(cub_tmp.p, tb, b_dkeys.p, b_dkeys_s.p, (int)nd, 0, eb, s));
     CK(cudaMemsetAsync(b_nkept.p, 0, sizeof(uint32_t), s));
-    if (ni) {
-      CK(cub::DeviceRadixSort::SortPairs(cub_tmp.p, t2, b_ikeys.p, b_ikeys_s.p,
-                                         explicit_w ? b_iw.p : b_isrc.p, b_iw_s.p, (int)ni, 0, eb, s));
-      { ++n_launch; k_filter_inserts<<<grid_elem(ni), 256, 0, s>>>(b_ikeys_s.p, (uint32_t)ni, b_dkeys_s.p,
-                                                     (uint32_t)nd, b_flag.p); }
-      CK(cub::DeviceSelect::Flagged(cub_tmp.p, t3, b_ikeys_s.p, b_flag.p, b_ikept.p, b_nkept.p,
-                                    (int)ni, s));
-      if (explicit_w)
-        CK(cub::DeviceSelect::Flagged(cub_tmp.p, t3, b_iw_s.p, b_flag.p, b_iw_kept.p, b_nkept.p,
-                                      (int)ni, s));
+    if (ni + nd) {
+      const bool vals = explicit_w && ni;
+      ensure_keys(ni + nd, vals);
+      { ++n_launch; k_batch_keys<<<grid_elem(ni + nd), 256, 0, s>>>(
+          b_isrc.p, b_idst.p, b_iw.p, ni, b_dsrc.p, b_ddst.p, nd, nv, id_bits(), b_keys.p,
+          vals ? b_vals.p : nullptr, b_err.p); }
+      sort_keys(ni + nd, vals);
+      const uint32_t gf = grid_elem(std::max(ni, nd));
+      b_counts.ensure((size_t)nsm * 8);
+      { ++n_launch; k_filter_inserts<<<gf, 256, 0, s>>>(b_keys_s.p, (uint32_t)ni, (uint32_t)nd, id_bits(), b_flag.p,
+                                                        b_counts.p, b_dkeys_s.p); }
+      if (ni)
+        { ++n_launch; k_keep_inserts<<<gf, 256, 0, s>>>(b_keys_s.p, vals ? b_vals_s.p : nullptr, (uint32_t)ni,
+                                                        id_bits(), b_flag.p, b_counts.p, b_ikept.p,
+                                                        vals ? b_iw_kept.p : nullptr, b_nkept.p); }
     }
     CK(cudaGetLastError());
     unsigned int herr = 0;
@@ -2694,10 +2689,9 @@ struct sgs_engine {
       fail(SGS_ERR_INVALID, "unknown field");
     // one lane's column of the group's rows into a buffer that the engine
     // keeps, then one copy to the caller.  (A buffer allocated and freed per
-    // call cost 0.6 ms in the two calls, each of which waits for the device; a
-    // snapshot with 64 results on 262,144 vertices went from 52 to 3.8 ms, one
-    // with 3 on a million from 4.0 to 1.2 ms.)  The lock is for callers that
-    // read several queries from several threads.
+    // call cost 0.6 ms in the two calls, each of which waits for the device:
+    // GATHER_TIMES.)  The lock is for callers that read several
+    // queries from several threads.
     std::lock_guard<std::mutex> lock(gather_mu);
     b_gather.ensure(nv);
     const bool parent = field == SGS_FIELD_PARENT;

@@ -81,12 +81,15 @@ struct InFillOp {
   }
 };
 
-// (src << 32 | dst) -> (dst << 32 | src) for the first *n_dev (or n) keys.
-__global__ void k_transpose_keys(const uint64_t *in, uint32_t n, const uint32_t *n_dev, uint64_t *out) {
-  const uint32_t cnt = n_dev ? *n_dev : n;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < cnt; i += gridDim.x * blockDim.x) {
-    const uint64_t k = in[i];
-    out[i] = (k << 32) | (k >> 32);
+// The batch's kept inserts and its deletes transposed, as one list of sort
+// keys (k_batch_keys) with the inserts' weights.
+__global__ void k_transpose_keys(const uint64_t *ins, const uint32_t *iw, uint64_t ni, const uint64_t *del,
+                                 uint64_t nd, int bits, uint64_t *keys, uint32_t *vals) {
+  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < ni + nd; i += stride) {
+    const uint64_t k = i < ni ? ins[i] : del[i - ni];
+    keys[i] = ((uint64_t)(i >= ni) << (2 * bits)) | ((k & 0xFFFFFFFFull) << bits) | (k >> 32);
+    if (vals) vals[i] = i < ni ? iw[i] : 0u;
   }
 }
 
