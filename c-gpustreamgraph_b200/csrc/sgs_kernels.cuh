@@ -584,6 +584,7 @@ struct InsertCtx {
   uint64_t *rl_to;
   uint32_t *rl_len;
   unsigned long long *rl_count64;
+  unsigned long long *fit;         // 0: no room, nothing is changed
 };
 
 __device__ __forceinline__ uint32_t grow_cap(uint32_t need) {
@@ -592,8 +593,15 @@ __device__ __forceinline__ uint32_t grow_cap(uint32_t need) {
   return (uint32_t)min(c, (uint64_t)0xFFFFFFF0u);
 }
 
+// Between the dry run and the plan: whether the relocations fit the arenas.
+// `again`: they were made to.
+__global__ void k_insert_fits(InsertCtx c, const unsigned long long *demand, bool again) {
+  *c.fit = again || (c.arena_top[0] + demand[0] <= c.arena_cap[0] && c.arena_top[1] + demand[1] <= c.arena_cap[1]);
+}
+
 __global__ void k_insert_plan(GraphView g, const uint64_t *keys, const uint32_t *n_ptr,
                               InsertCtx c, int dry, unsigned long long *demand) {
+  if (!dry && !*c.fit) return;
   const uint32_t n = *n_ptr;
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t b = (uint64_t)blockIdx.x * blockDim.x; b < n; b += stride) {
@@ -673,7 +681,9 @@ __global__ void k_insert_plan(GraphView g, const uint64_t *keys, const uint32_t 
 // Insert phase 2: one thread per kept insert writes (dst, w) at its rank
 // within its source's group.
 __global__ void k_insert_write(GraphView g, const uint64_t *keys, const uint32_t *w,
-                               const uint32_t *n_ptr, const uint64_t *wbase) {
+                               const uint32_t *n_ptr, InsertCtx c) {
+  if (!*c.fit) return;
+  const uint64_t *wbase = c.wbase;
   const uint32_t n = *n_ptr;
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
@@ -732,38 +742,78 @@ __global__ void k_compact_blocks(GraphView g, FrontierView f, unsigned long long
                                  uint32_t *big, uint32_t *big_n) {
   const uint32_t n = (uint32_t)(__ldcg((const unsigned long long *)f.counter) >> CNT_SHIFT);
   const uint32_t lane = threadIdx.x & 31;
-  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+  const uint64_t nwarps = (gridDim.x * blockDim.x) >> 5;
   const bool ew = g.wmode == W_EXPLICIT;
   unsigned long long got = 0;
-  for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += nwarps) {
-    const uint32_t v = __ldcg(&f.vtx[i]);
-    const uint32_t sl = g.slots[v], lv = g.live[v];
-    const uint32_t dead = sl - lv;
-    if (dead == 0 || (uint64_t)dead * 16 < lv) continue;  // warp-uniform
-    if (sl >= COMPACT_LARGE) {
-      if (lane == 0) big[atomicAdd(big_n, 1u)] = v;
-      continue;
+  // A warp looks at up to 32 touched blocks at a time, a lane each (fewer when
+  // the list is short, so that all warps get some), then compacts the due ones
+  // one after the other, the first slots of the next loaded while it works on
+  // one.  A warp per block spent a chain of reads on every block, also on
+  // those that stay as they are.
+  const uint32_t per = (uint32_t)min((n + nwarps - 1) / nwarps, (uint64_t)32);
+  for (uint64_t i0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * (uint64_t)per; i0 < n; i0 += nwarps * per) {
+    uint32_t mv = 0, msl = 0;
+    uint64_t mo = 0;
+    bool due = false;
+    if (lane < per && i0 + lane < n) {
+      mv = __ldcg(&f.vtx[i0 + lane]);
+      msl = g.slots[mv];
+      const uint32_t lv = g.live[mv], dead = msl - lv;
+      due = dead != 0 && (uint64_t)dead * 16 >= lv;
+      if (due && msl >= COMPACT_LARGE) {
+        big[atomicAdd(big_n, 1u)] = mv;
+        due = false;
+      }
+      if (due) mo = g.off[mv];
     }
-    const uint64_t o = g.off[v];
-    const uint32_t *a = adj_wptr(g, o);
-    const uint32_t *wt = ew ? wgt_wptr(g, o) : nullptr;
-    uint32_t out = 0;
-    for (uint32_t j = 0; j < sl; j += 32) {
+    struct Step {
+      uint32_t id, w;
+    };
+    auto load = [&](uint64_t o, uint32_t j, uint32_t sl) {
       const uint32_t k = j + lane;
-      const uint32_t id = k < sl ? __ldcg(a + k) : SGS_TOMB;
-      const uint32_t w = (ew && k < sl) ? __ldcg(wt + k) : 0u;
-      const bool keep = id != SGS_TOMB;
-      const uint32_t b = __ballot_sync(0xFFFFFFFFu, keep);
-      // every lane's reads of this step are done before any write; writes
-      // land at or below the positions just read, never on unread slots
-      __syncwarp();
-      if (keep) store_slot(g, o, out + __popc(b & ((1u << lane) - 1u)), id, ew, w);
-      out += __popc(b);
-      __syncwarp();
+      return Step{k < sl ? __ldcg(adj_wptr(g, o) + k) : SGS_TOMB,
+                  (ew && k < sl) ? __ldcg(wgt_wptr(g, o) + k) : 0u};
+    };
+    uint32_t todo = __ballot_sync(0xFFFFFFFFu, due);
+    uint64_t o = 0;
+    uint32_t sl = 0;
+    Step st{SGS_TOMB, 0};
+    if (todo) {
+      const int from = __ffs(todo) - 1;
+      o = __shfl_sync(0xFFFFFFFFu, mo, from);
+      sl = __shfl_sync(0xFFFFFFFFu, msl, from);
+      st = load(o, 0, sl);
     }
-    if (lane == 0) {
-      g.slots[v] = out;
-      got += sl - out;
+    while (todo) {
+      const int from = __ffs(todo) - 1;
+      todo &= todo - 1;
+      uint64_t no = 0;
+      uint32_t nsl = 0;
+      Step nst{SGS_TOMB, 0};
+      if (todo) {
+        const int nf = __ffs(todo) - 1;
+        no = __shfl_sync(0xFFFFFFFFu, mo, nf);
+        nsl = __shfl_sync(0xFFFFFFFFu, msl, nf);
+        nst = load(no, 0, nsl);
+      }
+      uint32_t out = 0;
+      for (uint32_t j = 0; j < sl; j += 32) {
+        // every lane's reads of this step and the next are done before any
+        // write; writes land at or below the positions of this step
+        const Step nx = load(o, j + 32, sl);
+        const bool keep = st.id != SGS_TOMB;
+        const uint32_t b = __ballot_sync(0xFFFFFFFFu, keep);
+        __syncwarp();
+        if (keep) store_slot(g, o, out + __popc(b & ((1u << lane) - 1u)), st.id, ew, st.w);
+        out += __popc(b);
+        st = nx;
+        __syncwarp();
+      }
+      if ((int)lane == from) g.slots[mv] = out;
+      if (lane == 0) got += sl - out;
+      o = no;
+      sl = nsl;
+      st = nst;
     }
   }
   if (lane == 0 && got) atomicAdd(reclaimed, got);
