@@ -20,14 +20,15 @@
 // over the CSC (forward: in-edges) or the CSR (adjoint: out-edges), with the
 // edge probabilities p = P[u,v] precomputed once per weight vector.
 //
-// Work split: a warp owns a work item.  Vertices of degree <= PIECE are one
-// item each; a heavier vertex (R-MAT hubs reach 10^5 in-edges) is cut into
-// pieces of PIECE edges whose partial sums go to a scratch row each and are
-// added up, in piece order, by the warp that finishes the vertex's last piece
-// -- so no warp walks more than PIECE edges and the sums are deterministic.  Inside a warp, LPE lanes
-// cover the columns of one neighbour row (CPL columns per lane) and 32/LPE
-// neighbours are gathered at once, four deep, so one neighbour row is one
-// coalesced read for any K.
+// Work split: a warp owns a work item.  Vertices of at most `piece` edges come
+// a few consecutive ones to an item (Impl::items_per_warp); a heavier vertex
+// (R-MAT hubs reach 10^5 in-edges) is cut into pieces of that many edges whose
+// partial sums go to a scratch row each and are added up, in piece order, by
+// the warp that finishes the vertex's last piece -- so no warp walks more than
+// `piece` edges of a vertex and the sums are deterministic.  Inside a warp, LPE
+// lanes cover the columns of one neighbour row (CPL columns per lane) and
+// 32/LPE neighbours are gathered at once, four deep, so one neighbour row is
+// one coalesced read for any K.
 #include <cooperative_groups.h>
 
 #include <cub/device/device_radix_sort.cuh>
@@ -81,7 +82,13 @@ struct Buf {
 };
 
 constexpr int THREADS = 256;
-constexpr uint32_t PIECE = 256;  // most edges one warp walks per item
+// Most edges of one vertex a warp walks per item, chosen per graph: 128, and 64
+// on graphs small enough that the longest walk, not the sum of all, is a step's
+// time (4096 vertices, 65536 edges, K = 8, forward and backward: 2.6 ms with
+// 256, 1.6 with 64; 2^20 vertices, K = 64: 144 ms with 256 and 32 light
+// vertices per item, 102 with 128 and 8).
+constexpr uint32_t PIECE_MAX = 128, PIECE_SMALL = 64;
+constexpr uint64_t SMALL_EDGES = 2u << 20;
 
 __device__ __forceinline__ uint32_t warp_id() { return (blockIdx.x * blockDim.x + threadIdx.x) >> 5; }
 __device__ __forceinline__ uint32_t num_warps() { return (gridDim.x * blockDim.x) >> 5; }
@@ -130,11 +137,11 @@ __global__ void k_gather_u32(const uint32_t *a, const uint32_t *idx, uint64_t n,
 }
 
 // cnt[v] = number of pieces of v (0 for a vertex of degree <= PIECE); cnt[nv] = 0.
-__global__ void k_piece_count(const uint64_t *ptr, uint32_t nv, uint32_t *cnt) {
+__global__ void k_piece_count(const uint64_t *ptr, uint32_t nv, uint32_t piece, uint32_t *cnt) {
   for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v <= nv;
        v += (uint64_t)gridDim.x * blockDim.x) {
     const uint64_t d = v < nv ? ptr[v + 1] - ptr[v] : 0;
-    cnt[v] = d > PIECE ? (uint32_t)((d + PIECE - 1) / PIECE) : 0u;
+    cnt[v] = d > piece ? (uint32_t)((d + piece - 1) / piece) : 0u;
   }
 }
 
@@ -145,32 +152,94 @@ __global__ void k_piece_fill(const uint32_t *poff, uint32_t nv, uint32_t *pv) {
     for (uint32_t p = poff[v]; p < poff[v + 1]; ++p) pv[p] = (uint32_t)v;
 }
 
-// inv_s[u] = 1 / sum of u's out-edge weights (0 without out-edges), and the
-// CSR edge probabilities pr[e] = w[e] inv_s[u].  err bit 0: a weight that is
-// not positive and finite.
-__global__ void k_row_probs(const uint64_t *row, uint32_t nv, const double *w, double *inv_s,
-                            double *pr, unsigned int *err) {
+// inv_s[u] = 1 / sum of u's out-edge weights (0 without out-edges) and, with
+// pr, the CSR edge probabilities pr[e] = w[e] inv_s[u] of the light vertices;
+// err bit 0: a weight that is not positive and finite.  Heavy rows go by their
+// pieces (one warp walked a whole hub's row before: 1.6 ms at 2^20 vertices and
+// 16.8 M edges, 0.15 now), whose sums the last one to finish adds up in
+// piece order; a light row takes 8 lanes, four rows per warp.
+__global__ void __launch_bounds__(THREADS)
+    k_row_sums(const uint64_t *row, uint32_t nv, const double *w, const uint32_t *pv, const uint32_t *poff,
+               uint32_t npieces, uint32_t piece, double *part, uint32_t *done, double *inv_s, double *pr,
+               unsigned int *err) {
+  constexpr unsigned full = 0xFFFFFFFFu;
   const int lane = threadIdx.x & 31;
-  for (uint32_t u = warp_id(); u < nv; u += num_warps()) {
+  bool bad = false;
+  for (uint32_t i = warp_id(); i < npieces; i += num_warps()) {
+    const uint32_t u = pv[i], first = poff[u], n = poff[u + 1] - first;
+    const uint64_t b = row[u] + (uint64_t)(i - first) * piece, e = min(b + piece, row[u + 1]);
     double s = 0.0;
-    for (uint64_t e = row[u] + lane; e < row[u + 1]; e += 32) {
-      const double x = w[e];
-      if (!(x > 0.0) || !isfinite(x)) atomicOr(err, 1u);
+#pragma unroll
+    for (uint32_t k = 0; k < PIECE_MAX; k += 32)
+      if (b + k + lane < e) {
+        const double x = w[b + k + lane];
+        bad |= !(x > 0.0) || !isfinite(x);
+        s += x;
+      }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(full, s, o);
+    uint32_t c = 0;
+    if (lane == 0) {
+      part[i] = s;
+      __threadfence();
+      c = atomicAdd(done + first, 1u);
+    }
+    if (__shfl_sync(full, c, 0) + 1 != n) continue;
+    __threadfence();
+    double t = 0.0;
+    for (uint32_t q = lane; q < n; q += 32) t += __ldcg(part + first + q);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(full, t, o);
+    if (lane == 0) {
+      done[first] = 0;
+      inv_s[u] = t > 0.0 ? 1.0 / t : 0.0;
+    }
+  }
+  const int sub = lane & 7;
+  for (uint64_t v0 = (uint64_t)warp_id() * 4; v0 < nv; v0 += (uint64_t)num_warps() * 4) {
+    const uint64_t u = v0 + (lane >> 3);
+    uint64_t b = 0, e = 0;
+    if (u < nv) {
+      b = row[u];
+      e = row[u + 1];
+    }
+    const bool light = e - b <= piece;
+    if (!light) e = b;
+    double s = 0.0;
+    for (uint64_t i = b + sub; i < e; i += 8) {
+      const double x = w[i];
+      bad |= !(x > 0.0) || !isfinite(x);
       s += x;
     }
+    __syncwarp();
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
+    for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(full, s, o);
     const double is = s > 0.0 ? 1.0 / s : 0.0;
-    if (lane == 0) inv_s[u] = is;
-    for (uint64_t e = row[u] + lane; e < row[u + 1]; e += 32) pr[e] = w[e] * is;
+    if (u < nv && light && sub == 0) inv_s[u] = is;
+    if (pr)
+      for (uint64_t i = b + sub; i < e; i += 8) pr[i] = w[i] * is;
+  }
+  if (bad) atomicOr(err, 1u);
+}
+
+// CSR probabilities of the heavy vertices, a warp per piece.
+__global__ void k_piece_probs(const uint64_t *row, const double *w, const uint32_t *pv, const uint32_t *poff,
+                              uint32_t npieces, uint32_t piece, const double *inv_s, double *pr) {
+  const int lane = threadIdx.x & 31;
+  for (uint32_t i = warp_id(); i < npieces; i += num_warps()) {
+    const uint32_t u = pv[i];
+    const uint64_t b = row[u] + (uint64_t)(i - poff[u]) * piece, e = min(b + piece, row[u + 1]);
+    const double is = inv_s[u];
+    for (uint64_t k = b + lane; k < e; k += 32) pr[k] = w[k] * is;
   }
 }
 
-// CSC probabilities: pc[i] = pr[ceid[i]].
-__global__ void k_csc_probs(const double *pr, const uint32_t *ceid, uint64_t ne, double *pc) {
+// CSC probabilities: pc[i] = w inv_s of the edge at CSC position i.
+__global__ void k_csc_probs(const double *w, const double *inv_s, const uint32_t *ceid, const uint32_t *csrc,
+                            uint64_t ne, double *pc) {
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < ne;
        i += (uint64_t)gridDim.x * blockDim.x)
-    pc[i] = pr[ceid[i]];
+    pc[i] = w[ceid[i]] * inv_s[csrc[i]];
 }
 
 // Row values: read-only cached loads, or, in the launch that runs many steps
@@ -180,88 +249,74 @@ __device__ __forceinline__ double ld_row(const double *p) {
   return Coh ? __ldcg(p) : __ldg(p);
 }
 
-// Narrow rows (K < 32): each lane group loads its own neighbours' ids,
-// probabilities and rows, four neighbours deep (neighbours b+eg, b+eg+NEG, ...).
-template <int LPE, int CPL, bool Coh>
-__device__ __forceinline__ void gather_rows_direct(const uint32_t *__restrict__ nbr,
-                                                   const double *__restrict__ p, uint64_t b,
-                                                   uint64_t e, int eg, uint32_t kb, uint32_t K,
-                                                   const double *x, double (&acc)[CPL]) {
-  constexpr int NEG = 32 / LPE;
-  uint64_t i = b + eg;
-  for (; i + 3 * NEG < e; i += 4 * NEG) {
-    uint32_t u[4];
-    double pp[4];
+// Narrow rows (K <= 16): a group of LPE lanes sums the rows of [b, e), LPE lanes
+// covering a row's columns and taking every `stride`-th edge, DEPTH at a time.
+template <int LPE, int DEPTH, bool Coh>
+__device__ __forceinline__ double gather_narrow(const uint32_t *__restrict__ nbr, const double *__restrict__ p,
+                                                uint64_t b, uint64_t e, uint32_t stride, uint32_t k, uint32_t K,
+                                                const double *x) {
+  double acc = 0.0;
+  uint64_t i = b;
+  for (; i < e; i += DEPTH * stride) {
+    uint32_t u[DEPTH];
+    double pp[DEPTH], xv[DEPTH];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      u[q] = nbr[i + q * NEG];
-      pp[q] = p[i + q * NEG];
+    for (int q = 0; q < DEPTH; ++q) {
+      const bool ok = i + q * stride < e;
+      u[q] = ok ? __ldg(nbr + i + q * stride) : 0u;
+      pp[q] = ok ? __ldg(p + i + q * stride) : 0.0;
     }
-    double xv[4][CPL];
 #pragma unroll
-    for (int q = 0; q < 4; ++q)
+    for (int q = 0; q < DEPTH; ++q)
+      xv[q] = k < K && i + q * stride < e ? ld_row<Coh>(x + (uint64_t)u[q] * K + k) : 0.0;
 #pragma unroll
-      for (int j = 0; j < CPL; ++j) {
-        const uint32_t k = kb + j * LPE;
-        xv[q][j] = k < K ? ld_row<Coh>(x + (uint64_t)u[q] * K + k) : 0.0;
-      }
-#pragma unroll
-    for (int q = 0; q < 4; ++q)
-#pragma unroll
-      for (int j = 0; j < CPL; ++j) acc[j] = fma(pp[q], xv[q][j], acc[j]);
+    for (int q = 0; q < DEPTH; ++q) acc = fma(pp[q], xv[q], acc);
   }
-  for (; i < e; i += NEG) {
-    const uint32_t u = nbr[i];
-    const double pp = p[i];
-#pragma unroll
-    for (int j = 0; j < CPL; ++j) {
-      const uint32_t k = kb + j * LPE;
-      if (k < K) acc[j] = fma(pp, ld_row<Coh>(x + (uint64_t)u * K + k), acc[j]);
-    }
-  }
+  return acc;
 }
 
-// acc[j] += sum_{i in [b,e)} p[i] x[nbr[i], kb + j LPE] for this lane's
-// neighbour group eg.  Neighbour ids and probabilities come 32 at a time in
-// one coalesced load per warp and are handed to the lane groups by shuffles
-// (group eg takes neighbours eg, eg + NEG, ...), so the only dependent load
-// per neighbour is its row; DEPTH neighbours per group are in flight at once.
-template <int LPE, int CPL, bool Coh>
-__device__ __forceinline__ void gather_rows(const uint32_t *__restrict__ nbr,
-                                            const double *__restrict__ p, uint64_t b, uint64_t e,
-                                            int lane, int eg, uint32_t kb, uint32_t K,
+// Wide rows (K > 16): the warp covers the row's columns kb, kb + 32, ... (CPL
+// per lane); acc[j] += sum over [b, e) of p x.  Neighbour ids and
+// probabilities come 32 at a time in one coalesced load (the first 32 are
+// given: they were loaded ahead) and are handed out by shuffles, so the only
+// dependent load per neighbour is its row; DEPTH rows are in flight.
+struct Head {
+  uint32_t u;
+  double p;
+};
+__device__ __forceinline__ Head load_head(const uint32_t *__restrict__ nbr, const double *__restrict__ p,
+                                          uint64_t b, uint64_t e, int lane) {
+  return b + lane < e ? Head{__ldg(nbr + b + lane), __ldg(p + b + lane)} : Head{0u, 0.0};
+}
+template <int CPL, bool Coh>
+__device__ __forceinline__ void gather_wide(const uint32_t *__restrict__ nbr, const double *__restrict__ p,
+                                            uint64_t b, uint64_t e, Head h, int lane, uint32_t kb, uint32_t K,
                                             const double *x, double (&acc)[CPL]) {
-  constexpr int NEG = 32 / LPE;
-  constexpr int DEPTH = LPE < 4 ? LPE : 4;
+  constexpr int DEPTH = 4;
   for (uint64_t c = b; c < e; c += 32) {
     const uint32_t cnt = e - c < 32 ? (uint32_t)(e - c) : 32u;
-    const uint32_t mu = (uint32_t)lane < cnt ? __ldg(nbr + c + lane) : 0u;
-    const double mp = (uint32_t)lane < cnt ? __ldg(p + c + lane) : 0.0;
-#pragma unroll 1
-    for (int r0 = 0; r0 < LPE && (uint32_t)(NEG * r0) < cnt; r0 += DEPTH) {
+    const Head nx = load_head(nbr, p, c + 32, e, lane);
+    for (uint32_t r = 0; r < cnt; r += DEPTH) {
       uint32_t u[DEPTH];
-      double pp[DEPTH];
-      bool ok[DEPTH];
+      double pp[DEPTH], xv[DEPTH][CPL];
 #pragma unroll
       for (int q = 0; q < DEPTH; ++q) {
-        const int jn = eg + NEG * (r0 + q);  // < 32
-        u[q] = __shfl_sync(0xFFFFFFFFu, mu, jn);
-        pp[q] = __shfl_sync(0xFFFFFFFFu, mp, jn);
-        ok[q] = (uint32_t)jn < cnt;
+        u[q] = __shfl_sync(0xFFFFFFFFu, h.u, (r + q) & 31);
+        pp[q] = __shfl_sync(0xFFFFFFFFu, h.p, (r + q) & 31);
       }
-      double xv[DEPTH][CPL];
 #pragma unroll
       for (int q = 0; q < DEPTH; ++q)
 #pragma unroll
-        for (int jj = 0; jj < CPL; ++jj) {
-          const uint32_t k = kb + jj * LPE;
-          xv[q][jj] = ok[q] && k < K ? ld_row<Coh>(x + (uint64_t)u[q] * K + k) : 0.0;
+        for (int j = 0; j < CPL; ++j) {
+          const uint32_t k = kb + 32 * j;
+          xv[q][j] = r + q < cnt && k < K ? ld_row<Coh>(x + (uint64_t)u[q] * K + k) : 0.0;
         }
 #pragma unroll
       for (int q = 0; q < DEPTH; ++q)
 #pragma unroll
-        for (int jj = 0; jj < CPL; ++jj) acc[jj] = fma(pp[q], xv[q][jj], acc[jj]);
+        for (int j = 0; j < CPL; ++j) acc[j] = fma(pp[q], xv[q][j], acc[j]);
     }
+    h = nx;
   }
 }
 
@@ -273,12 +328,14 @@ struct StepArgs {
   const double *p;
   uint32_t nv;
   const uint32_t *pv, *poff;
-  uint32_t npieces;
+  uint32_t npieces, piece;
   uint32_t K;
   double alpha, c;
   const double *B;
   double *part;    // a row of K per piece
   uint32_t *done;  // finished pieces, at the vertex's first piece (zero between steps)
+  uint32_t *next;  // next item, one counter per step of the history (zero before it)
+  uint32_t per;    // light vertices per item
   sgs::StepHist h;
   double tol;
 };
@@ -298,77 +355,74 @@ __device__ __forceinline__ void finish_entry(const StepArgs &a, const sgs::StepR
 
 // One step over the work items [0, npieces) (pieces of heavy vertices: partial
 // sums to part[piece][K]; the warp that finishes a vertex's last piece adds
-// them up in piece order and writes the vertex) and [npieces, npieces + nv)
-// (light vertices).  The pieces come first, so their sums are added while the
-// other warps walk the light vertices; a kernel of its own for them cost 5 us
-// per step on a small graph and 85 us at a million vertices and K = 64.
+// them up in piece order and writes the vertex) and then `per` consecutive
+// vertices each, of which it handles the light ones.  The pieces come first, so
+// their sums are added while the other warps walk the light vertices; a kernel
+// of its own for them cost 5 us per step on a small graph and 85 us at a
+// million vertices and K = 64.
+// Dyn: warps take items from a counter, the next one requested while one is
+// handled.  (Degrees follow the ids' bits on R-MAT graphs, and with a fixed
+// stride the resident warps averaged 30 % where 50 % were launched.)  The
+// looping launch, whose steps are too short for a round trip per item, strides.
+// Vertices without edges keep their first value, c B, for good: only step 0
+// writes them.  (2^20 vertices, 16.8 M edges, K = 64: 2.46 ms a step with a
+// fixed stride, 32 vertices an item and pieces of 256; 1.01 ms now, 10.3 TB/s
+// by the bytes of step_bytes, most rows coming from L2.)
 template <int LPE, int CPL, bool Coh>
 __device__ __forceinline__ void ppr_step_body(const StepArgs &a, const sgs::StepRule &rule, const double *x,
-                                              double *out, uint32_t k_hist) {
+                                              double *out, uint32_t k_hist, bool first_step) {
+  constexpr bool Dyn = !Coh;
+  constexpr unsigned full = 0xFFFFFFFFu;
+  constexpr int NEG = 32 / LPE;
   const int lane = threadIdx.x & 31;
   const int sub = lane % LPE, eg = lane / LPE;
   const uint32_t K = a.K;
   double dsum = 0.0, fsum = 0.0;
-  const uint32_t items = a.npieces + a.nv;
+  const uint32_t items = a.npieces + (a.nv + a.per - 1) / a.per;
   const uint32_t W = num_warps();
-  uint64_t pb = 0, pe = 0;  // bounds of this warp's next light vertex, loaded ahead
-  bool have = false;
-  for (uint32_t wi = warp_id(); wi < items; wi += W) {
-    uint32_t v, first = 0, last = 0;
-    uint64_t b, e;
-    const bool piece = wi < a.npieces;
-    if (piece) {
-      v = a.pv[wi];
-      first = a.poff[v];
-      last = a.poff[v + 1];
-      b = a.ptr[v] + (uint64_t)(wi - first) * PIECE;
-      e = min(b + PIECE, a.ptr[v + 1]);
+  // the row sums of [b, e) for the whole warp, columns k0 on: every lane ends up
+  // with those of its columns (narrow forms: each lane group with all)
+  auto row_sums = [&](uint64_t b, uint64_t e, const Head &h, uint32_t k0, double (&acc)[CPL]) {
+#pragma unroll
+    for (int j = 0; j < CPL; ++j) acc[j] = 0.0;
+    if constexpr (LPE == 32) {
+      gather_wide<CPL, Coh>(a.nbr, a.p, b, e, h, lane, k0 + lane, K, x, acc);
     } else {
-      v = wi - a.npieces;
-      if (have) {
-        b = pb;
-        e = pe;
-      } else {
-        b = a.ptr[v];
-        e = a.ptr[v + 1];
-      }
-      if constexpr (LPE == 32) {  // the narrow forms have no registers to spare
-        have = wi + W < items;
-        if (have) {
-          pb = a.ptr[v + W];
-          pe = a.ptr[v + W + 1];
+      acc[0] = gather_narrow<LPE, Coh ? 8 : 4, Coh>(a.nbr, a.p, b + eg, e, NEG, k0 + sub, K, x);
+#pragma unroll
+      for (int o = 16; o >= LPE; o >>= 1) acc[0] += __shfl_xor_sync(full, acc[0], o);
+    }
+  };
+  uint32_t it = warp_id();
+  if constexpr (Dyn) {
+    if (lane == 0) it = atomicAdd(a.next + k_hist, 1u);
+    it = __shfl_sync(full, it, 0);
+  }
+  while (it < items) {
+    uint32_t nxt = it + W;
+    if constexpr (Dyn) {
+      if (lane == 0) nxt = atomicAdd(a.next + k_hist, 1u);
+    }
+    if (it < a.npieces) {
+      const uint32_t v = a.pv[it], first = a.poff[v], last = a.poff[v + 1];
+      const uint64_t b = a.ptr[v] + (uint64_t)(it - first) * a.piece, e = min(b + a.piece, a.ptr[v + 1]);
+      const Head h = LPE == 32 ? load_head(a.nbr, a.p, b, e, lane) : Head{0u, 0.0};
+      for (uint32_t k0 = 0; k0 < K; k0 += LPE * CPL) {
+        double acc[CPL];
+        row_sums(b, e, h, k0, acc);
+        if (eg == 0) {
+#pragma unroll
+          for (int j = 0; j < CPL; ++j) {
+            const uint32_t k = k0 + sub + j * LPE;
+            if (k < K) a.part[(uint64_t)it * K + k] = acc[j];
+          }
         }
       }
-      if (e - b > PIECE) continue;  // summed by its pieces
-    }
-    for (uint32_t k0 = 0; k0 < K; k0 += LPE * CPL) {
-      double acc[CPL];
-#pragma unroll
-      for (int j = 0; j < CPL; ++j) acc[j] = 0.0;
-      if constexpr (LPE == 32)
-        gather_rows<LPE, CPL, Coh>(a.nbr, a.p, b, e, lane, eg, k0 + sub, K, x, acc);
-      else
-        gather_rows_direct<LPE, CPL, Coh>(a.nbr, a.p, b, e, eg, k0 + sub, K, x, acc);
-#pragma unroll
-      for (int j = 0; j < CPL; ++j)
-#pragma unroll
-        for (int o = 16; o >= LPE; o >>= 1) acc[j] += __shfl_xor_sync(0xFFFFFFFFu, acc[j], o);
-      if (eg == 0) {
-#pragma unroll
-        for (int j = 0; j < CPL; ++j) {
-          const uint32_t k = k0 + sub + j * LPE;
-          if (k >= K) continue;
-          if (piece) a.part[(uint64_t)wi * K + k] = acc[j];
-          else finish_entry<Coh>(a, rule, (uint64_t)v * K + k, acc[j], x, out, dsum, fsum);
-        }
-      }
-    }
-    if (piece) {
       __threadfence();  // this warp's row before its count
       __syncwarp();
       uint32_t n = 0;
       if (lane == 0) n = atomicAdd(a.done + first, 1u);
-      n = __shfl_sync(0xFFFFFFFFu, n, 0);
+      n = __shfl_sync(full, n, 0);
       if (n + 1 == last - first) {
         __threadfence();
         if (lane == 0) a.done[first] = 0;
@@ -379,34 +433,118 @@ __device__ __forceinline__ void ppr_step_body(const StepArgs &a, const sgs::Step
           finish_entry<Coh>(a, rule, (uint64_t)v * K + k, sum, x, out, dsum, fsum);
         }
       }
+    } else {
+      const uint32_t v0 = (it - a.npieces) * a.per;
+      const uint32_t n = min(a.per, a.nv - v0);
+      const uint64_t rb = (uint32_t)lane < n ? a.ptr[v0 + lane] : 0;
+      const uint64_t re = (uint32_t)lane < n ? a.ptr[v0 + lane + 1] : 0;
+      const uint64_t deg = re - rb;
+      if (first_step) {
+        for (uint32_t em = __ballot_sync(full, (uint32_t)lane < n && deg == 0); em; em &= em - 1) {
+          const uint64_t o = (uint64_t)(v0 + __ffs(em) - 1) * K;
+          for (uint32_t k = lane; k < K; k += 32) finish_entry<Coh>(a, rule, o + k, 0.0, x, out, dsum, fsum);
+        }
+      }
+      uint32_t todo = __ballot_sync(full, deg > 0 && deg <= a.piece);
+      if constexpr (LPE < 32) {
+        // up to 32 edges: a lane group per vertex, NEG vertices at a time
+        uint32_t lo = __ballot_sync(full, deg > 0 && deg <= 32);
+        todo &= ~lo;
+        while (lo) {
+          const int my = eg < __popc(lo) ? (int)__fns(lo, 0, eg + 1) : -1;
+          const uint64_t b = __shfl_sync(full, rb, my & 31), e = __shfl_sync(full, re, my & 31);
+          if (my >= 0) {
+            const double s = gather_narrow<LPE, Coh ? 8 : 4, Coh>(a.nbr, a.p, b, e, 1, sub, K, x);
+            if ((uint32_t)sub < K) finish_entry<Coh>(a, rule, (uint64_t)(v0 + my) * K + sub, s, x, out, dsum, fsum);
+          }
+          __syncwarp();
+#pragma unroll
+          for (int q = 0; q < NEG; ++q) lo &= lo - 1;
+        }
+      }
+      // one vertex at a time, the next one's first ids and probabilities ahead
+      Head h{0u, 0.0};
+      uint64_t b = 0, e = 0;
+      if (todo) {
+        const int f = __ffs(todo) - 1;
+        b = __shfl_sync(full, rb, f);
+        e = __shfl_sync(full, re, f);
+        if constexpr (LPE == 32) h = load_head(a.nbr, a.p, b, e, lane);
+      }
+      while (todo) {
+        const uint32_t v = v0 + __ffs(todo) - 1;
+        todo &= todo - 1;
+        uint64_t nb = 0, ne = 0;
+        Head nh{0u, 0.0};
+        if (todo) {
+          const int f = __ffs(todo) - 1;
+          nb = __shfl_sync(full, rb, f);
+          ne = __shfl_sync(full, re, f);
+          if constexpr (LPE == 32) nh = load_head(a.nbr, a.p, nb, ne, lane);
+        }
+        for (uint32_t k0 = 0; k0 < K; k0 += LPE * CPL) {
+          double acc[CPL];
+          row_sums(b, e, h, k0, acc);
+          if (eg == 0) {
+#pragma unroll
+            for (int j = 0; j < CPL; ++j) {
+              const uint32_t k = k0 + sub + j * LPE;
+              if (k < K) finish_entry<Coh>(a, rule, (uint64_t)v * K + k, acc[j], x, out, dsum, fsum);
+            }
+          }
+        }
+        b = nb;
+        e = ne;
+        h = nh;
+      }
     }
+    it = Dyn ? __shfl_sync(full, nxt, 0) : nxt;
   }
+  // one atomic per CTA (one per warp, all on one address, cost a small graph's
+  // step more than its sums)
+  __shared__ double s_d[THREADS / 32], s_f[THREADS / 32];
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
-    dsum += __shfl_xor_sync(0xFFFFFFFFu, dsum, o);
-    fsum += __shfl_xor_sync(0xFFFFFFFFu, fsum, o);
+    dsum += __shfl_xor_sync(full, dsum, o);
+    fsum += __shfl_xor_sync(full, fsum, o);
   }
   if (lane == 0) {
-    if (dsum != 0.0) atomicAdd(a.h.l1() + k_hist, dsum);
-    if (fsum != 0.0) atomicAdd(a.h.fit() + k_hist, fsum);
+    s_d[threadIdx.x >> 5] = dsum;
+    s_f[threadIdx.x >> 5] = fsum;
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) sgs::record_rule(a.h, k_hist, rule);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double d = 0.0, f = 0.0;
+#pragma unroll
+    for (int w = 0; w < THREADS / 32; ++w) {
+      d += s_d[w];
+      f += s_f[w];
+    }
+    if (d != 0.0) atomicAdd(a.h.l1() + k_hist, d);
+    if (f != 0.0) atomicAdd(a.h.fit() + k_hist, f);
+    if (blockIdx.x == 0) sgs::record_rule(a.h, k_hist, rule);
+  }
 }
 
 template <int LPE, int CPL>
-__global__ void __launch_bounds__(THREADS, LPE == 32 ? 4 : LPE == 1 ? 6 : 8)
-    k_ppr_step(StepArgs a, const double *__restrict__ x, double *out, uint32_t k) {
-  ppr_step_body<LPE, CPL, false>(a, sgs::step_rule(a.h, k, a.alpha, a.tol * sgs::LONG_TOL), x, out, k);
+__global__ void __launch_bounds__(THREADS, LPE == 32 ? 4 : 5)
+    k_ppr_step(StepArgs a, const double *__restrict__ x, double *out, uint32_t k, bool first) {
+  ppr_step_body<LPE, CPL, false>(a, sgs::step_rule(a.h, k, a.alpha, a.tol * sgs::LONG_TOL), x, out, k, first);
 }
 
 // The end of the iteration, the same on both sides: a plain step below the
 // tolerance that is also a sixteenth of it (LONG_TOL; a second one after a long
 // step, sgs_steplen.cuh), or the EXTRA-th one below it, should rounding keep
 // the rest away.
+// Rounding: the steps' changes no longer fall (`prev`: the change of the step
+// before, 0 if that was a long one).
 constexpr uint32_t EXTRA = 20;
-__host__ __device__ inline bool ppr_ends(double w, double l1, int state, double tol, uint32_t &under) {
-  if (w == 1.0 && l1 < tol) ++under;
-  return w == 1.0 && l1 < tol && (sgs::StepRule::ends(w, l1, state, tol * sgs::LONG_TOL) || under > EXTRA);
+__host__ __device__ inline bool ppr_ends(double w, double l1, double prev, int state, double tol, double alpha,
+                                         uint32_t &under) {
+  if (w != 1.0 || !(l1 < tol)) return false;
+  ++under;
+  return sgs::StepRule::ends(w, l1, state, tol * sgs::LONG_TOL) || under > EXTRA ||
+         (prev > 0.0 && l1 > (alpha > 0.9 ? alpha : 0.9) * prev);
 }
 
 // Steps k0 .. k1 - 1 in one cooperative launch, a grid barrier after each, until
@@ -416,64 +554,113 @@ __host__ __device__ inline bool ppr_ends(double w, double l1, int state, double 
 // this loop and the long steps.
 template <int LPE, int CPL>
 __global__ void __launch_bounds__(THREADS, 4)
-    k_ppr_steps(StepArgs a, double *x0, double *x1, uint32_t k0, uint32_t k1, uint32_t under, uint32_t *ran) {
+    k_ppr_steps(StepArgs a, double *x0, double *x1, uint32_t k0, uint32_t k1, uint32_t under, bool first,
+                uint32_t *ran) {
   cooperative_groups::grid_group grid = cooperative_groups::this_grid();
   uint32_t k = k0;
   while (k < k1) {
     const sgs::StepRule rule = sgs::step_rule(a.h, k, a.alpha, a.tol * sgs::LONG_TOL);
-    ppr_step_body<LPE, CPL, true>(a, rule, k % 2 ? x1 : x0, k % 2 ? x0 : x1, k);
-    __threadfence();
+    ppr_step_body<LPE, CPL, true>(a, rule, k % 2 ? x1 : x0, k % 2 ? x0 : x1, k, first && k == k0);
     grid.sync();
     const double l1 = __ldcg(a.h.l1() + k);
+    const double prev = k && __ldcg(a.h.step() + k - 1) == 1.0 ? __ldcg(a.h.l1() + k - 1) : 0.0;
     ++k;
-    if (ppr_ends(rule.w, l1, rule.state, a.tol, under)) break;
+    if (ppr_ends(rule.w, l1, prev, rule.state, a.tol, a.alpha, under)) break;
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) *ran = k - k0;
 }
 
 // gw[e] = inv_s[u] (alpha sum_k X[u,k] Y[v,k] + c_u) for e = (u,v), where
 // c_u = sum_k X[u,k] (G[u,k] - Y[u,k]); work items as in k_ppr_step over the
-// CSR (each item recomputes c_u for its source).
-template <int LPE>
+// CSR, taken from a counter.  Bound by the gather of Y's rows: four are in
+// flight per lane group, and their dot products are reduced together, halving
+// the values held with the lanes they cover (6 exchanges for four sums instead of
+// 20).  (2^20 vertices, K = 64: 7.2 ms with fixed strides and a reduction per
+// edge, 1.96 now.)
+// CPL columns per lane (its X entries stay in registers), LPE lanes per row.
+template <int LPE, int CPL>
 __global__ void __launch_bounds__(THREADS)
     k_ppr_edge_grad(const uint64_t *__restrict__ row, const uint32_t *__restrict__ col,
                     const double *__restrict__ inv_s, uint32_t nv, const uint32_t *__restrict__ pv,
-                    const uint32_t *__restrict__ poff, uint32_t npieces, uint32_t K, double alpha,
-                    const double *__restrict__ X, const double *__restrict__ Y,
-                    const double *__restrict__ G, double *__restrict__ gw) {
+                    const uint32_t *__restrict__ poff, uint32_t npieces, uint32_t piece, uint32_t K,
+                    double alpha, const double *__restrict__ X, const double *__restrict__ Y,
+                    const double *__restrict__ G, double *__restrict__ gw, uint32_t *next) {
   constexpr int NEG = 32 / LPE;
+  constexpr unsigned full = 0xFFFFFFFFu;
+  constexpr uint32_t PER = 8;  // vertices per item
   const int lane = threadIdx.x & 31;
   const int sub = lane % LPE, eg = lane / LPE;
-  const uint32_t items = npieces + nv;
-  for (uint32_t wi = warp_id(); wi < items; wi += num_warps()) {
-    uint32_t u;
-    uint64_t b, e;
-    if (wi < npieces) {
-      u = pv[wi];
-      b = row[u] + (uint64_t)(wi - poff[u]) * PIECE;
-      e = min(b + PIECE, row[u + 1]);
-    } else {
-      u = wi - npieces;
-      b = row[u];
-      e = row[u + 1];
-      if (e == b || e - b > PIECE) continue;
-    }
+  const uint32_t items = npieces + (nv + PER - 1) / PER;
+  auto edges = [&](uint32_t u, uint64_t b, uint64_t e) {
     const uint64_t ou = (uint64_t)u * K;
-    double cu = 0.0;
+    const double is = inv_s[u];
+    double xu[CPL], cu = 0.0;
     for (uint32_t k = lane; k < K; k += 32) cu += X[ou + k] * (G[ou + k] - Y[ou + k]);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) cu += __shfl_xor_sync(0xFFFFFFFFu, cu, o);
-    const double is = inv_s[u];
-    for (uint64_t e0 = b; e0 < e; e0 += NEG) {
-      const uint64_t i = e0 + eg;
-      const bool ok = i < e;
-      const uint32_t v = ok ? col[i] : 0u;
-      double t = 0.0;
-      if (ok)
-        for (uint32_t k = sub; k < K; k += LPE) t = fma(X[ou + k], Y[(uint64_t)v * K + k], t);
+    for (int o = 16; o > 0; o >>= 1) cu += __shfl_xor_sync(full, cu, o);
 #pragma unroll
-      for (int o = LPE / 2; o > 0; o >>= 1) t += __shfl_xor_sync(0xFFFFFFFFu, t, o);
-      if (ok && sub == 0) gw[i] = is * fma(alpha, t, cu);
+    for (int j = 0; j < CPL; ++j) xu[j] = sub + j * LPE < K ? X[ou + sub + j * LPE] : 0.0;
+    for (uint64_t e0 = b; e0 < e; e0 += 4 * NEG) {
+      double t[4];
+      uint32_t v[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const uint64_t i = e0 + q * NEG + eg;
+        v[q] = i < e ? __ldg(col + i) : 0u;
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        t[q] = 0.0;
+        const bool ok = e0 + q * NEG + eg < e;
+#pragma unroll
+        for (int j = 0; j < CPL; ++j)
+          if (ok && sub + j * LPE < K) t[q] = fma(xu[j], __ldg(Y + (uint64_t)v[q] * K + sub + j * LPE), t[q]);
+        if constexpr (CPL == 2)  // more than 64 columns: the rest of the row
+          if (ok)
+            for (uint32_t k = sub + CPL * LPE; k < K; k += LPE)
+              t[q] = fma(X[ou + k], __ldg(Y + (uint64_t)v[q] * K + k), t[q]);
+      }
+      if constexpr (LPE >= 4) {
+        // four sums over LPE lanes: after two halving steps lane group s / (LPE/4)
+        // holds edge q = s / (LPE/4)'s
+        const bool up = sub & (LPE / 2);
+        double a0 = up ? t[2] : t[0], a1 = up ? t[3] : t[1];
+        a0 += __shfl_xor_sync(full, up ? t[0] : t[2], LPE / 2);
+        a1 += __shfl_xor_sync(full, up ? t[1] : t[3], LPE / 2);
+        const bool up2 = sub & (LPE / 4);
+        double z = up2 ? a1 : a0;
+        z += __shfl_xor_sync(full, up2 ? a0 : a1, LPE / 4);
+#pragma unroll
+        for (int o = LPE / 8; o > 0; o >>= 1) z += __shfl_xor_sync(full, z, o);
+        const int q = (up ? 2 : 0) + (up2 ? 1 : 0);
+        const uint64_t i = e0 + q * NEG + eg;
+        if (i < e && sub % (LPE / 4) == 0) gw[i] = is * fma(alpha, z, cu);
+      } else {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+#pragma unroll
+          for (int o = LPE / 2; o > 0; o >>= 1) t[q] += __shfl_xor_sync(full, t[q], o);
+          const uint64_t i = e0 + q * NEG + eg;
+          if (i < e && sub == 0) gw[i] = is * fma(alpha, t[q], cu);
+        }
+      }
+    }
+  };
+  for (;;) {
+    uint32_t it = 0;
+    if (lane == 0) it = atomicAdd(next, 1u);
+    it = __shfl_sync(full, it, 0);
+    if (it >= items) break;
+    if (it < npieces) {
+      const uint32_t u = pv[it];
+      const uint64_t b = row[u] + (uint64_t)(it - poff[u]) * piece;
+      edges(u, b, min(b + piece, row[u + 1]));
+    } else {
+      const uint32_t v0 = (it - npieces) * PER;
+      for (uint32_t u = v0; u < min(v0 + PER, nv); ++u) {
+        const uint64_t b = row[u], e = row[u + 1];
+        if (e != b && e - b <= piece) edges(u, b, e);
+      }
     }
   }
 }
@@ -512,13 +699,15 @@ struct sgs_ppr {
   Buf<uint64_t> row, crow;
   Buf<uint32_t> col, csrc, ceid;
   Buf<double> w, inv_s, pr, pc, t, x, xn, g, y, yn, part;
-  // one allocation: the step history, then (u32) the steps a looping launch ran
-  // and the finished pieces per heavy vertex
+  // one allocation: the step history, then (u32) the steps' item counters, the
+  // steps a looping launch ran and the finished pieces per heavy vertex
   Buf<double> work;
-  uint32_t *ran() { return (uint32_t *)(work.p + sgs::StepHist::FIELDS * (size_t)HIST); }
+  uint32_t *next() { return (uint32_t *)(work.p + sgs::StepHist::FIELDS * (size_t)HIST); }
+  uint32_t *ran() { return next() + HIST; }
   uint32_t *done() { return ran() + 1; }
   static constexpr uint32_t HIST = 512;  // steps the history holds
   Buf<unsigned int> err;
+  uint32_t piece = PIECE_MAX;
   Adj in, out;  // CSC (forward) and CSR (adjoint, edge gradient)
   // timing and counters
   bool timing = false;
@@ -590,7 +779,7 @@ struct sgs_ppr {
     a.ptr = ptr;
     a.nbr = nbr;
     a.poff.ensure((size_t)nv + 1);
-    { ++n_launch; k_piece_count<<<grid(), THREADS, 0, s>>>(ptr, nv, a.poff.p); }
+    { ++n_launch; k_piece_count<<<grid(), THREADS, 0, s>>>(ptr, nv, piece, a.poff.p); }
     size_t tb = 0;
     PCK(cub::DeviceScan::ExclusiveSum(nullptr, tb, a.poff.p, a.poff.p, (int)(nv + 1), s));
     Buf<unsigned char> tmp;
@@ -623,47 +812,53 @@ struct sgs_ppr {
     // CSC: sort (destination, CSR edge index) by destination (stable, so the
     // in-edges of a vertex keep CSR order), sources through the edge index.
     {
-      Buf<uint32_t> src, dst_s, eid;
-      src.ensure(ne);
-      dst_s.ensure(ne);
-      eid.ensure(ne);
       csrc.ensure(ne);
       ceid.ensure(ne);
       crow.ensure((size_t)nv + 1);
-      { ++n_launch; k_edge_src<<<grid(), THREADS, 0, s>>>(row.p, nv, src.p); }
-      { ++n_launch; k_iota<<<grid(), THREADS, 0, s>>>(eid.p, ne); }
       int bits = 1;
       while (bits < 32 && (1ull << bits) < nv) ++bits;
       size_t tb = 0;
-      PCK(cub::DeviceRadixSort::SortPairs(nullptr, tb, col.p, dst_s.p, eid.p, ceid.p, (int)ne, 0,
-                                          bits, s));
+      PCK(cub::DeviceRadixSort::SortPairs(nullptr, tb, col.p, col.p, col.p, ceid.p, (int)ne, 0, bits, s));
+      // source, sorted destination and index of every edge, and the sort's
+      // storage: one allocation (each costs about as much as a small sort)
+      const size_t part3 = (ne * sizeof(uint32_t) + 255) / 256 * 256;
       Buf<unsigned char> tmp;
-      tmp.ensure(tb);
-      PCK(cub::DeviceRadixSort::SortPairs(tmp.p, tb, col.p, dst_s.p, eid.p, ceid.p, (int)ne, 0,
-                                          bits, s));
-      { ++n_launch; k_csc_rows<<<grid(), THREADS, 0, s>>>(dst_s.p, ne, nv, crow.p); }
-      { ++n_launch; k_gather_u32<<<grid(), THREADS, 0, s>>>(src.p, ceid.p, ne, csrc.p); }
+      tmp.ensure(3 * part3 + tb);
+      uint32_t *src = (uint32_t *)tmp.p, *dst_s = (uint32_t *)(tmp.p + part3), *eid = (uint32_t *)(tmp.p + 2 * part3);
+      { ++n_launch; k_edge_src<<<grid(), THREADS, 0, s>>>(row.p, nv, src); }
+      { ++n_launch; k_iota<<<grid(), THREADS, 0, s>>>(eid, ne); }
+      PCK(cub::DeviceRadixSort::SortPairs(tmp.p + 3 * part3, tb, col.p, dst_s, eid, ceid.p, (int)ne, 0, bits, s));
+      { ++n_launch; k_csc_rows<<<grid(), THREADS, 0, s>>>(dst_s, ne, nv, crow.p); }
+      { ++n_launch; k_gather_u32<<<grid(), THREADS, 0, s>>>(src, ceid.p, ne, csrc.p); }
       PCK(cudaGetLastError());
       sync();
     }
+    piece = ne <= SMALL_EDGES ? PIECE_SMALL : PIECE_MAX;
     pieces(in, crow.p, csrc.p);
     pieces(out, row.p, col.p);
     inv_s.ensure(nv);
     pr.ensure(ne);
     pc.ensure(ne);
     const size_t words = 1 + (size_t)std::max(in.npieces, out.npieces);
-    work.ensure(sgs::StepHist::FIELDS * (size_t)HIST + (words + 1) / 2);
+    work.ensure(sgs::StepHist::FIELDS * (size_t)HIST + (HIST + words + 1) / 2);
     PCK(cudaMemsetAsync(ran(), 0, sizeof(uint32_t) * words, s));
     sync();
   }
 
-  // Loads a weight vector and forms inv_s, pr (CSR order) and pc (CSC order).
-  void set_weights(const double *wt, int mem) {
+  // Loads a weight vector and forms inv_s and the probabilities of the direction
+  // asked for: pc (CSC order, forward) or pr (CSR order, adjoint).
+  void set_weights(const double *wt, bool adjoint, int mem) {
     w.ensure(ne);
+    part.ensure(out.npieces);
     if (ne) PCK(cudaMemcpyAsync(w.p, wt, sizeof(double) * ne, kin(mem), s));
     PCK(cudaMemsetAsync(err.p, 0, sizeof(unsigned int), s));
-    { ++n_launch; k_row_probs<<<grid(), THREADS, 0, s>>>(row.p, nv, w.p, inv_s.p, pr.p, err.p); }
-    { ++n_launch; k_csc_probs<<<grid(), THREADS, 0, s>>>(pr.p, ceid.p, ne, pc.p); }
+    { ++n_launch; k_row_sums<<<grid(), THREADS, 0, s>>>(row.p, nv, w.p, out.pv.p, out.poff.p, out.npieces, piece, part.p,
+                                                        done(), inv_s.p, adjoint ? pr.p : nullptr, err.p); }
+    if (!adjoint)
+      { ++n_launch; k_csc_probs<<<grid(), THREADS, 0, s>>>(w.p, inv_s.p, ceid.p, csrc.p, ne, pc.p); }
+    else if (out.npieces)
+      { ++n_launch; k_piece_probs<<<grid(), THREADS, 0, s>>>(row.p, w.p, out.pv.p, out.poff.p, out.npieces, piece,
+                                                             inv_s.p, pr.p); }
     PCK(cudaGetLastError());
     unsigned int h = 0;
     PCK(cudaMemcpyAsync(&h, err.p, sizeof(h), cudaMemcpyDeviceToHost, s));
@@ -671,26 +866,32 @@ struct sgs_ppr {
     if (h) throw PprFail{SGS_ERR_INVALID, "edge weights must be positive and finite"};
   }
 
-  template <int L>
+  template <int L, int C>
   void launch_grad(uint32_t K, double alpha, const double *Y, double *dst) {
-    { ++n_launch; k_ppr_edge_grad<L><<<rgrid((const void *)k_ppr_edge_grad<L>), THREADS, 0, s>>>(row.p, col.p, inv_s.p, nv, out.pv.p, out.poff.p,
-                                                  out.npieces, K, alpha, x.p, Y, g.p, dst); }
+    PCK(cudaMemsetAsync(next(), 0, sizeof(uint32_t), s));
+    { ++n_launch; k_ppr_edge_grad<L, C><<<rgrid((const void *)k_ppr_edge_grad<L, C>), THREADS, 0, s>>>(
+        row.p, col.p, inv_s.p, nv, out.pv.p, out.poff.p, out.npieces, piece, K, alpha, x.p, Y, g.p, dst, next()); }
   }
 
   // A step of fewer bytes than this (step_bytes) takes less than about 20 us
   // and runs in the launch that loops on the device; a longer one hides its
-  // launch and gathers through the read-only cache.
+  // launch, takes its items from a counter and gathers through the read-only
+  // cache.  Forward and backward, a launch per step against the loop: 2.8
+  // against 1.6 ms at 6 MB a step, 3.9 against 2.7 at 40 MB, 9.8 against 16.1
+  // at 189 MB, 104 against 157 at 10 GB.
   static constexpr double LOOP_BYTES = 64e6;
 
   template <int LPE, int CPL>
-  void launch(const StepArgs &a, bool loop, double *b0, double *b1, uint32_t k, uint32_t k1, uint32_t under) {
+  void launch(const StepArgs &a, bool loop, double *b0, double *b1, uint32_t k, uint32_t k1, uint32_t under,
+              bool first) {
     if (loop) {
       const void *f = (const void *)k_ppr_steps<LPE, CPL>;
       StepArgs aa = a;
       uint32_t *r = ran();
-      void *args[] = {&aa, &b0, &b1, &k, &k1, &under, &r};
+      void *args[] = {&aa, &b0, &b1, &k, &k1, &under, &first, &r};
       // no more CTAs than items (idle ones only lengthen the barriers)
-      const uint64_t need = ((uint64_t)a.npieces + a.nv + THREADS / 32 - 1) / (THREADS / 32);
+      const uint64_t items = a.npieces + ((uint64_t)a.nv + a.per - 1) / a.per;
+      const uint64_t need = (items + THREADS / 32 - 1) / (THREADS / 32);
       const uint32_t gr = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(rgrid(f), need));
       ++n_launch;
       PCK(cudaLaunchCooperativeKernel(f, gr, THREADS, args, 0, s));
@@ -699,37 +900,49 @@ struct sgs_ppr {
     for (; k < k1; ++k) {
       ++n_launch;
       k_ppr_step<LPE, CPL><<<rgrid((const void *)k_ppr_step<LPE, CPL>), THREADS, 0, s>>>(a, k % 2 ? b1 : b0,
-                                                                                       k % 2 ? b0 : b1, k);
+                                                                                       k % 2 ? b0 : b1, k, first);
+      first = false;
     }
   }
   // Steps k .. k1 - 1 (or, looping, up to the end of the iteration).
-  void steps(const StepArgs &a, bool loop, double *b0, double *b1, uint32_t k, uint32_t k1, uint32_t under) {
+  void steps(const StepArgs &a, bool loop, double *b0, double *b1, uint32_t k, uint32_t k1, uint32_t under,
+             bool first) {
     switch (a.K <= 32 ? lanes_per_edge(a.K) : 64) {
-      case 1: launch<1, 1>(a, loop, b0, b1, k, k1, under); break;
-      case 2: launch<2, 1>(a, loop, b0, b1, k, k1, under); break;
-      case 4: launch<4, 1>(a, loop, b0, b1, k, k1, under); break;
-      case 8: launch<8, 1>(a, loop, b0, b1, k, k1, under); break;
-      case 16: launch<16, 1>(a, loop, b0, b1, k, k1, under); break;
-      case 32: launch<32, 1>(a, loop, b0, b1, k, k1, under); break;
-      default: launch<32, 2>(a, loop, b0, b1, k, k1, under); break;
+      case 1: launch<1, 1>(a, loop, b0, b1, k, k1, under, first); break;
+      case 2: launch<2, 1>(a, loop, b0, b1, k, k1, under, first); break;
+      case 4: launch<4, 1>(a, loop, b0, b1, k, k1, under, first); break;
+      case 8: launch<8, 1>(a, loop, b0, b1, k, k1, under, first); break;
+      case 16: launch<16, 1>(a, loop, b0, b1, k, k1, under, first); break;
+      case 32: launch<32, 1>(a, loop, b0, b1, k, k1, under, first); break;
+      default: launch<32, 2>(a, loop, b0, b1, k, k1, under, first); break;
     }
     PCK(cudaGetLastError());
   }
 
-  // The fixed point of x = c B + alpha A x from the state in b0, b1 as the
-  // second buffer: steps until one changes the state by less than tol in L1
+  // Light vertices per item: 8 from the counter (32 left the last items to few
+  // warps), in the loop as many as give every warp one item; at least what the
+  // lane groups of a narrow form take at a time, at most 32.
+  uint32_t items_per_warp(bool loop, uint32_t K) const {
+    const uint32_t warps = (uint32_t)nsm * 32, neg = 32u / (uint32_t)lanes_per_edge(std::min(K, 32u));
+    uint32_t per = loop ? (nv + warps - 1) / warps : 8u;
+    return std::min(32u, std::max(per, neg));
+  }
+
+  // The fixed point of x = c B + alpha A x from c B in b0, b1 as the second
+  // buffer: steps until one changes the state by less than tol in L1
   // (ppr_ends).  `cur` = the buffer with the result.  Returns the steps run, -1
   // when max_iter did not suffice.
   int iterate(const Adj &adj, const double *p, uint32_t K, double alpha, double c, const double *B, double *b0,
               double *b1, double tol, uint32_t max_iter, double *&cur) {
     const double bytes = step_bytes(K);
     const bool loop = bytes < LOOP_BYTES;
-    StepArgs a{adj.ptr, adj.nbr, p, nv, adj.pv.p, adj.poff.p, adj.npieces, K, alpha, c, B, part.p, done(),
-               sgs::StepHist{work.p, HIST}, tol};
+    StepArgs a{adj.ptr, adj.nbr, p, nv, adj.pv.p, adj.poff.p, adj.npieces, piece, K, alpha, c, B, part.p, done(), next(),
+               items_per_warp(loop, K), sgs::StepHist{work.p, HIST}, tol};
     const size_t row = sizeof(double);
-    PCK(cudaMemsetAsync(work.p, 0, row * sgs::StepHist::FIELDS * HIST, s));
+    PCK(cudaMemsetAsync(work.p, 0, row * sgs::StepHist::FIELDS * HIST + sizeof(uint32_t) * HIST, s));
     uint32_t it = 0, k = 0, under = 0;
     bool below = false;  // the last plain step was below tol
+    double prev = 0.0;   // its change
     std::vector<double> hd;
     while (it < max_iter) {
       if (k == HIST) {
@@ -741,6 +954,7 @@ struct sgs_ppr {
           PCK(cudaMemcpyAsync(q, q + HIST - keep, row * keep, cudaMemcpyDeviceToDevice, s));
           PCK(cudaMemsetAsync(q + keep, 0, row * (HIST - keep), s));
         }
+        PCK(cudaMemsetAsync(next(), 0, sizeof(uint32_t) * HIST, s));
         k = keep;
       }
       // A launch per step: 8 steps before the first host read (never fewer are
@@ -749,7 +963,7 @@ struct sgs_ppr {
       uint32_t nb = std::min<uint32_t>(HIST - k, max_iter - it);
       if (!loop) nb = std::min<uint32_t>(nb, it == 0 ? 8 : bytes > 256e6 ? 2 : 4);
       if (timing) PCK(cudaEventRecord(ev[0], s));
-      steps(a, loop, b0, b1, k, k + nb, under);
+      steps(a, loop, b0, b1, k, k + nb, under, it == 0);
       if (timing) PCK(cudaEventRecord(ev[1], s));
       hd.resize(sgs::StepHist::FIELDS * (size_t)nb);
       uint32_t n = nb;
@@ -766,7 +980,8 @@ struct sgs_ppr {
       const sgs::StepHist h{hd.data(), nb};
       bool end = false;
       for (uint32_t b = 0; b < n; ++b) {
-        end = end || ppr_ends(h.step()[b], h.l1()[b], (int)h.state()[b], tol, under);
+        end = end || ppr_ends(h.step()[b], h.l1()[b], prev, (int)h.state()[b], tol, alpha, under);
+        prev = h.step()[b] == 1.0 ? h.l1()[b] : 0.0;
         below = h.step()[b] == 1.0 && h.l1()[b] < tol;
       }
       it += n;
@@ -816,12 +1031,15 @@ struct sgs_ppr {
         dst = tmp.p;
       }
       switch (lanes_per_edge(K)) {
-        case 1: launch_grad<1>(K, alpha, cur, dst); break;
-        case 2: launch_grad<2>(K, alpha, cur, dst); break;
-        case 4: launch_grad<4>(K, alpha, cur, dst); break;
-        case 8: launch_grad<8>(K, alpha, cur, dst); break;
-        case 16: launch_grad<16>(K, alpha, cur, dst); break;
-        default: launch_grad<32>(K, alpha, cur, dst); break;
+        case 1: launch_grad<1, 1>(K, alpha, cur, dst); break;
+        case 2: launch_grad<2, 1>(K, alpha, cur, dst); break;
+        case 4: launch_grad<4, 1>(K, alpha, cur, dst); break;
+        case 8: launch_grad<8, 1>(K, alpha, cur, dst); break;
+        case 16: launch_grad<16, 1>(K, alpha, cur, dst); break;
+        default:
+          if (K <= 32) launch_grad<32, 1>(K, alpha, cur, dst);
+          else launch_grad<32, 2>(K, alpha, cur, dst);
+          break;
       }
       PCK(cudaGetLastError());
       if (mem == SGS_MEM_HOST) PCK(cudaMemcpyAsync(gw, dst, sizeof(double) * ne, kout(mem), s));
@@ -974,7 +1192,7 @@ SGS_API int sgs_ppr_forward(sgs_ppr *p, const double *w, const double *T, uint32
   if (bad_args(alpha, K)) return SGS_ERR_INVALID;
   return pguard([&] {
     PCK(cudaSetDevice(p->dev));
-    p->set_weights(w, mem);
+    p->set_weights(w, false, mem);
     p->call_begin();
     p->st.bytes_alg_step = p->step_bytes(K);
     const int it = p->forward(T, K, alpha, tol, max_iter, X, mem);
@@ -994,7 +1212,7 @@ SGS_API int sgs_ppr_backward(sgs_ppr *p, const double *w, const double *X, const
   if (bad_args(alpha, K)) return SGS_ERR_INVALID;
   return pguard([&] {
     PCK(cudaSetDevice(p->dev));
-    p->set_weights(w, mem);
+    p->set_weights(w, true, mem);
     p->call_begin();
     p->st.bytes_alg_step = p->step_bytes(K);
     const int it = p->backward(X, G, K, alpha, tol, max_iter, gw, gT, mem);
