@@ -342,29 +342,45 @@ __global__ void k_pr_warm_res(const double *x, double *r, uint32_t nv, double ba
 // 1.61 ms and 28.3 -> 9.6 ms.
 // Coherent: r was written earlier in the same launch by other CTAs (the
 // persistent round kernel), so it is read through L2.
-template <bool Coherent>
+template <bool Coherent, int N>
 __device__ __forceinline__ StepRule pr_absorb_body(const GraphView &g, double *x, double *r, double *pv,
                                                    double alpha, double tol, const StepHist &h, uint32_t k) {
   const StepRule rule = step_rule(h, k, alpha, tol);
   const double w = rule.w;
   const double back = rule.mu / alpha;  // push value * outdeg * back = mu * previous residual
   double acc = 0.0, fit = 0.0;
+  // N vertices per thread and step, everything they need requested before
+  // anything is used.  Four in a launch of its own (one at a time it was bound by
+  // that latency: 45 us at two million vertices, 38 now); one in the launch that
+  // runs all rounds, whose graphs have about a vertex per thread, and where the
+  // registers of four would halve the CTAs that fit.
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < g.nv; v += stride) {
-    const double rv = Coherent ? __ldcg(r + v) : r[v];
-    double p = 0.0;
-    const double prev = rule.mu > 0.0 ? pv[v] : 0.0;
-    if (rv != 0.0 || prev != 0.0) {
-      const uint32_t l = g.live[v];
-      if (rv != 0.0) {
-        r[v] = w == 1.0 ? 0.0 : (1.0 - w) * rv;
-        x[v] += w * rv;
-        acc += fabs(rv);
-        if (l) p = w * alpha * rv / (double)l;
-      }
-      if (rule.mu > 0.0 && l) fit += fabs(rv - back * prev * (double)l);
+  for (uint64_t v0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v0 < g.nv; v0 += N * stride) {
+    double rv[N], xv[N], prev[N];
+    uint32_t l[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      const uint64_t v = v0 + i * stride;
+      const bool in = v < g.nv;
+      rv[i] = in ? (Coherent ? __ldcg(r + v) : r[v]) : 0.0;
+      xv[i] = in ? x[v] : 0.0;
+      prev[i] = in && rule.mu > 0.0 ? pv[v] : 0.0;
+      l[i] = in ? g.live[v] : 0u;
     }
-    pv[v] = p;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      const uint64_t v = v0 + i * stride;
+      if (v >= g.nv) break;
+      double p = 0.0;
+      if (rv[i] != 0.0) {
+        r[v] = w == 1.0 ? 0.0 : (1.0 - w) * rv[i];
+        x[v] = xv[i] + w * rv[i];
+        acc += fabs(rv[i]);
+        if (l[i]) p = w * alpha * rv[i] / (double)l[i];
+      }
+      if (rule.mu > 0.0 && l[i]) fit += fabs(rv[i] - back * prev[i] * (double)l[i]);
+      pv[v] = p;
+    }
   }
   __shared__ double s_acc[RELAX_THREADS / 32], s_fit[RELAX_THREADS / 32];
   acc = warp_sum(acc);
@@ -390,7 +406,7 @@ __device__ __forceinline__ StepRule pr_absorb_body(const GraphView &g, double *x
 
 __global__ void k_pr_absorb(GraphView g, double *x, double *r, double *pv,
                             double alpha, double tol, StepHist h, uint32_t k) {
-  pr_absorb_body<false>(g, x, r, pv, alpha, tol, h, k);
+  pr_absorb_body<false, 4>(g, x, r, pv, alpha, tol, h, k);
 }
 
 // PageRank rounds r0, r0+1, ... (at most `limit`) of the pull form in one
@@ -408,11 +424,9 @@ __global__ void __launch_bounds__(RELAX_THREADS)
   cooperative_groups::grid_group grid = cooperative_groups::this_grid();
   uint32_t k = 0;
   while (k < limit) {
-    const StepRule rule = pr_absorb_body<true>(g, x, r, pv, alpha, tol, h, r0 + k);
-    __threadfence();
+    const StepRule rule = pr_absorb_body<true, 1>(g, x, r, pv, alpha, tol, h, r0 + k);
     grid.sync();
     pull_pr_body<true>(fin, gi, pv, r, rule.w != 1.0, edge_stat);
-    __threadfence();
     grid.sync();
     const double l1v = __ldcg(h.l1() + r0 + k);
     ++k;
