@@ -36,7 +36,7 @@ constexpr uint64_t HOST_BIT = 1ull << 63;
 constexpr uint64_t OFF_MASK = HOST_BIT - 1;
 constexpr int CNT_SHIFT = 37;                 // packed frontier counter
 constexpr uint64_t EDGE_MASK = (1ull << CNT_SHIFT) - 1;
-constexpr uint32_t UNIT = 2048;               // edges per load-balanced unit
+constexpr uint32_t UNIT = 1024;               // edges per load-balanced unit (a window for each warp of a CTA)
 constexpr int RELAX_THREADS = 256;
 
 enum Algo : int { A_BFS = 0, A_SSSP = 1, A_CC = 2, A_PR = 3 };
@@ -324,12 +324,13 @@ __device__ __forceinline__ void frontier_append(const FrontierView &f, bool want
 
 // Block-aggregated append: one atomic per CTA instead of one per warp, for
 // builders where most threads append.  Every thread of the CTA (blockDim.x ==
-// RELAX_THREADS) must call it the same number of times.
+// THREADS) must call it the same number of times.
+template <int THREADS = RELAX_THREADS>
 __device__ __forceinline__ void frontier_append_block(const FrontierView &f, bool want,
                                                       uint32_t v, uint32_t d,
                                                       uint32_t *aux = nullptr,
                                                       uint32_t aux_val = 0) {
-  constexpr int NW = RELAX_THREADS / 32;
+  constexpr int NW = THREADS / 32;
   __shared__ unsigned long long s_warp[NW];
   __shared__ unsigned long long s_base;
   const unsigned full = 0xFFFFFFFFu;
@@ -374,47 +375,56 @@ __device__ __forceinline__ void frontier_append_block(const FrontierView &f, boo
 // A walk's step finds up to four per thread; appending them as they come took
 // one counter atomic per step and slot of the quad, all on one address, and
 // that address set the pace of rounds that improve many vertices.  The queue
-// hands them over 32 at a time: one scan, one atomic, coalesced length reads.
+// hands them over 32 at a time: one scan, one atomic.
 // SSSP and BFS from scratch on a million vertices: the rounds 2163 -> 1085 us,
 // the query 2.6 -> 1.7 ms.
 struct WarpQueue {
-  static constexpr int CAP = 31 + 4 * 32;
-  uint32_t *v;     // [CAP] of this warp
+  static constexpr int CAP = 31 + 4 * 32, CAP1 = 31 + 32;  // entries for push4, for push alone
+  uint2 *e;        // (vertex, slots) of this warp
   uint32_t n = 0;  // warp-uniform
-  __device__ __forceinline__ explicit WarpQueue(uint32_t *mine) : v(mine) {}
-  // Bit k of `app`: append dst[k].  All 32 lanes, converged.
-  template <class Len>
+  __device__ __forceinline__ explicit WarpQueue(uint2 *mine) : e(mine) {}
+  // Bit k of `app`: append dst[k], whose block has len[k] slots.  All 32 lanes,
+  // converged.
   __device__ __forceinline__ void push4(const FrontierView &f, uint32_t app, const uint32_t (&dst)[4],
-                                        const Len &len) {
+                                        const uint32_t (&len)[4]) {
     if (!__ballot_sync(0xFFFFFFFFu, app != 0u)) return;
     const uint32_t below = (1u << (threadIdx.x & 31)) - 1u;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       const uint32_t m = __ballot_sync(0xFFFFFFFFu, app >> k & 1u);
-      if (app >> k & 1u) v[n + __popc(m & below)] = dst[k];
+      if (app >> k & 1u) e[n + __popc(m & below)] = make_uint2(dst[k], len[k]);
       n += __popc(m);
     }
     __syncwarp();
-    while (n >= 32) flush(f, 32, len);
+    while (n >= 32) flush(f, 32);
   }
-  template <class Len>
-  __device__ __forceinline__ void push(const FrontierView &f, bool want, uint32_t dst, const Len &len) {
+  __device__ __forceinline__ void push(const FrontierView &f, bool want, uint32_t dst, uint32_t len) {
     const uint32_t m = __ballot_sync(0xFFFFFFFFu, want);
     if (!m) return;
-    if (want) v[n + __popc(m & ((1u << (threadIdx.x & 31)) - 1u))] = dst;
+    if (want) e[n + __popc(m & ((1u << (threadIdx.x & 31)) - 1u))] = make_uint2(dst, len);
     n += __popc(m);
     __syncwarp();
-    while (n >= 32) flush(f, 32, len);
+    while (n >= 32) flush(f, 32);
+  }
+  // What the queues of the CTA's warps still hold (fewer than 32 each), with one
+  // atomic: a round in which every warp finds a little would otherwise send one
+  // per warp to the one counter.  All threads of the CTA.
+  template <int THREADS>
+  __device__ __forceinline__ void finish(const FrontierView &f) {
+    if (!__syncthreads_or(n != 0u)) return;
+    const bool want = (threadIdx.x & 31) < n;
+    const uint2 x = want ? e[threadIdx.x & 31] : make_uint2(0, 0);
+    n = 0;
+    frontier_append_block<THREADS>(f, want, x.x, x.y);
   }
   // Appends the last min(n, most) of the queue (most <= 32).
-  template <class Len>
-  __device__ __forceinline__ void flush(const FrontierView &f, uint32_t most, const Len &len) {
+  __device__ __forceinline__ void flush(const FrontierView &f, uint32_t most) {
     const uint32_t c = min(n, most), lane = threadIdx.x & 31;
     const bool want = lane < c;
-    const uint32_t x = want ? v[n - c + lane] : 0u;
+    const uint2 x = want ? e[n - c + lane] : make_uint2(0, 0);
     n -= c;
     __syncwarp();  // read before the next push writes the places
-    frontier_append(f, want, x, want ? len(x) : 0u);
+    frontier_append(f, want, x.x, x.y);
   }
 };
 

@@ -17,6 +17,8 @@
 #pragma once
 #include <cooperative_groups.h>
 
+#include <algorithm>
+
 #include "sgs_device.cuh"
 #include "sgs_segmap.cuh"
 
@@ -115,6 +117,8 @@ struct RPay {
 
 template <int S>
 struct GroupRelaxOp {
+  static constexpr int kBlocks = 4;
+  static constexpr bool kResets = false;
   using Payload = RPay<S>;
   GraphView g;
   unsigned long long *st;
@@ -144,8 +148,6 @@ struct GroupRelaxOp {
   struct Quad {
     uint4 ids, ws;
   };
-  // slots of an appended vertex (its range in the next frontier)
-  __device__ __forceinline__ uint32_t append_len(uint32_t v) const { return g.slots[v]; }
   // H: the graph has a host tier (blocks may be host-resident or cached)
   template <bool H>
   __device__ __forceinline__ Quad fetch(const Payload &p, uint32_t j0) const {
@@ -169,9 +171,11 @@ struct GroupRelaxOp {
   __device__ __forceinline__ uint32_t weight_of(const uint4 &ws, int k, uint32_t u, uint32_t d) const {
     return g.wmode == W_EXPLICIT ? quad_at(ws, k) : g.wmode == W_SYNTH ? (u + d) % 128u + 1u : 1u;
   }
-  // Returns a 4-bit mask of destinations to append; dst[] holds them.
+  // Returns a 4-bit mask of destinations to append; dst[] holds them, sl[] their
+  // slots.
   __device__ __forceinline__ uint32_t visit4(uint32_t u, const Payload &pr, uint32_t j0, uint32_t len,
-                                             const Quad &qd, uint32_t (&dst)[4]) const {
+                                             const Quad &qd, uint32_t (&dst)[4], uint32_t (&sl)[4],
+                                             uint32_t *) const {
     const uint4 ids = qd.ids;
     const uint4 ws = qd.ws;
     uint32_t okm = 0;
@@ -196,30 +200,66 @@ struct GroupRelaxOp {
         lt |= (cand_of(pr.base[q], w, q) < cur[k][q] ? 1u : 0u) << (4 * k + q);
     }
     if (!lt) return 0;
-    uint32_t app = 0;
+    // The atomics go out together, then their answers are looked at: with a
+    // wait after each (up to 16 per quad, one lane's improvement holding up the
+    // whole warp) a round's length was that chain.  (With units of 1024 slots
+    // and one append per CTA at a round's end, scale 16, 20,000 updates:
+    // relaxation rounds 140 -> 91 us, invalidation rounds 148 -> 93 us.)
+    uint32_t old[4][S];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      const uint32_t lk = lt >> (4 * k) & 0xFu;
-      if (!lk) continue;
+      const uint32_t w = weight_of(ws, k, u, dst[k]);
+#pragma unroll
+      for (int q = 0; q < S; ++q) {
+        old[k][q] = 0;
+        if (lt >> (4 * k + q) & 1u)
+          old[k][q] = atomicMin(&val[(uint64_t)dst[k] * S + q], cand_of(pr.base[q], w, q));
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) sl[k] = lt >> (4 * k) & 0xFu ? g.slots[dst[k]] : 0u;
+    uint32_t app = 0, seen[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
       const uint32_t w = weight_of(ws, k, u, dst[k]);
       uint32_t bits = 0;
 #pragma unroll
       for (int q = 0; q < S; ++q) {
-        if (!(lk >> q & 1u)) continue;
-        const uint64_t idx = (uint64_t)dst[k] * S + q;
-        if (relax_mirror_packed(&val[idx], &st[idx], cand_of(pr.base[q], w, q), u)) bits |= 1u << q;
+        const uint32_t cand = cand_of(pr.base[q], w, q);
+        if (old[k][q] > cand) {  // strictly lowered (0 where no candidate was offered)
+          atomicMin(&st[(uint64_t)dst[k] * S + q], ((unsigned long long)cand << 32) | u);
+          bits |= 1u << q;
+        }
       }
-      if (bits && g.slots[dst[k]] && atomicOr(&m_out[dst[k]], bits) == 0u) app |= 1u << k;
+      seen[k] = 1u;
+      if (bits && sl[k]) seen[k] = atomicOr(&m_out[dst[k]], bits);
     }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) app |= (seen[k] == 0u ? 1u : 0u) << k;
     return app;
   }
 };
+
+// S packed words of vertex v (two 16-B loads for S = 4).
+template <int S>
+__device__ __forceinline__ void load_row(const unsigned long long *st, uint32_t v, unsigned long long (&o)[S]) {
+  if constexpr (S == 4) {
+    const ulonglong2 a = __ldcg(reinterpret_cast<const ulonglong2 *>(st + (uint64_t)v * 4));
+    const ulonglong2 b = __ldcg(reinterpret_cast<const ulonglong2 *>(st + (uint64_t)v * 4 + 2));
+    o[0] = a.x; o[1] = a.y; o[2] = b.x; o[3] = b.y;
+  } else {
+#pragma unroll
+    for (int q = 0; q < S; ++q) o[q] = __ldcg(st + (uint64_t)v * S + q);
+  }
+}
 
 // Parent-tree invalidation per lane: a child whose lane-q parent is u (and u
 // was reset in lane q) is reset exactly once (CAS on the packed word); the
 // mirror is reset with it.
 template <int S>
 struct GroupInvalidateOp {
+  static constexpr int kBlocks = 3;
+  static constexpr bool kResets = true;
   struct Payload {
     uint64_t off;
     uint32_t mask;
@@ -243,14 +283,14 @@ struct GroupInvalidateOp {
   struct Quad {
     uint4 ids;
   };
-  __device__ __forceinline__ uint32_t append_len(uint32_t v) const { return g.slots[v]; }
   template <bool H>
   __device__ __forceinline__ Quad fetch(const Payload &p, uint32_t j0) const {
     if constexpr (H) return Quad{ld_quad_stream(adj_at(g, p.off, j0))};
     else return Quad{ld_quad_stream(g.adj_d + p.off + j0)};
   }
   __device__ __forceinline__ uint32_t visit4(uint32_t u, const Payload &p, uint32_t j0, uint32_t len,
-                                             const Quad &qd, uint32_t (&dst)[4]) const {
+                                             const Quad &qd, uint32_t (&dst)[4], uint32_t (&sl)[4],
+                                             uint32_t *resets) const {
     const uint4 ids = qd.ids;
     uint32_t okm = 0;
 #pragma unroll
@@ -258,28 +298,47 @@ struct GroupInvalidateOp {
       dst[k] = quad_at(ids, k);
       if (j0 + k < len && dst[k] != SGS_TOMB) okm |= 1u << k;
     }
-    uint32_t app = 0;
+    // rows, then the resets, then the masks: each kind together (see GroupRelaxOp)
+    unsigned long long row[4][S];
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (okm >> k & 1u) load_row<S>(st, dst[k], row[k]);
+    uint32_t hit = 0;  // bit 4k+q: lane q's parent of destination k is u
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+#pragma unroll
+      for (int q = 0; q < S; ++q)
+        if ((okm >> k & 1u) && (p.mask >> q & 1u) && (uint32_t)row[k][q] == u) hit |= 1u << (4 * k + q);
+    if (!hit) return 0;
+    unsigned long long was[4][S];
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+#pragma unroll
+      for (int q = 0; q < S; ++q) {
+        was[k][q] = 0;
+        if (hit >> (4 * k + q) & 1u)
+          was[k][q] = atomicCAS(&st[(uint64_t)dst[k] * S + q], row[k][q],
+                                algo.at(q) == A_CC ? (((unsigned long long)dst[k] << 32) | INF32) : ~0ull);
+      }
+    uint32_t seen[4], app = 0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) sl[k] = hit >> (4 * k) & 0xFu ? g.slots[dst[k]] : 0u;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      if (!(okm >> k & 1u)) continue;
       uint32_t bits = 0;
 #pragma unroll
       for (int q = 0; q < S; ++q) {
-        if (!(p.mask >> q & 1u)) continue;
-        const uint64_t idx = (uint64_t)dst[k] * S + q;
-        const unsigned long long cu = __ldcg(&st[idx]);
-        if ((uint32_t)cu != u) continue;
-        const bool cc = algo.at(q) == A_CC;
-        const unsigned long long rst = cc ? (((unsigned long long)dst[k] << 32) | INF32) : ~0ull;
-        if (atomicCAS(&st[idx], cu, rst) == cu) {
-          val[idx] = cc ? dst[k] : INF32;
-          bits |= 1u << q;
-          atomicAdd(&inval[q], 1ull);
-        }
+        if (!(hit >> (4 * k + q) & 1u) || was[k][q] != row[k][q]) continue;
+        val[(uint64_t)dst[k] * S + q] = algo.at(q) == A_CC ? dst[k] : INF32;
+        bits |= 1u << q;
+        atomicAdd(&resets[q], 1u);
       }
       if (bits && mark) bit_set(mark, dst[k]);
-      if (bits && g.slots[dst[k]] && atomicOr(&m_out[dst[k]], bits) == 0u) app |= 1u << k;
+      seen[k] = 1u;
+      if (bits && sl[k]) seen[k] = atomicOr(&m_out[dst[k]], bits);
     }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) app |= (seen[k] == 0u ? 1u : 0u) << k;
     return app;
   }
 };
@@ -289,9 +348,9 @@ struct GroupInvalidateOp {
 // position adds live[v] for every lane of its mask, which counts exactly the
 // (query, edge) pairs relaxed.  The kernel also clears the previous
 // frontier's masks.
-#ifndef SGS_GROUP_MIN_BLOCKS
-#define SGS_GROUP_MIN_BLOCKS 4  // resident CTAs per SM the register budget allows
-#endif
+// (Op::kBlocks: resident CTAs per SM that the registers are budgeted for; 4 of
+// 64 registers for the relaxation, 3 for the invalidation, which holds four
+// 32-B rows per thread.)
 // H = false when every block is in HBM (no host tier): the host-tier logic
 // (hotness, cache lookups, link accounting) is compiled out.
 template <class Op, bool H>
@@ -300,7 +359,7 @@ __device__ __forceinline__ void group_map_body(FrontierView in, FrontierView out
                                                const unsigned long long *prev_cnt, uint32_t *prev_mask,
                                                unsigned long long *lane_edges,
                                                unsigned long long *edge_stat,
-                                               unsigned long long *host_stat) {
+                                               unsigned long long *host_stat, uint64_t packed) {
   using P = typename Op::Payload;
   constexpr int GC = GCHUNK;
   __shared__ uint64_t s_eb[GC + 1];
@@ -309,14 +368,15 @@ __device__ __forceinline__ void group_map_body(FrontierView in, FrontierView out
   __shared__ uint32_t s_vtx[GC];
   __shared__ unsigned long long s_lane[GMAX];
   __shared__ unsigned long long s_host, s_all;  // host-tier slots read over the link / owned
-  __shared__ uint32_t s_queue[RELAX_THREADS / 32][WarpQueue::CAP];
+  __shared__ uint32_t s_reset[GMAX];            // resets of an invalidation, per lane
+  __shared__ uint2 s_queue[RELAX_THREADS / 32][WarpQueue::CAP];
   WarpQueue queue(s_queue[threadIdx.x >> 5]);
-  auto len_of = [&](uint32_t v) { return op.append_len(v); };
-  clear_prev_masks(prev_vtx, prev_cnt, prev_mask);
-  if (threadIdx.x < GMAX) s_lane[threadIdx.x] = 0;
+  if (threadIdx.x < GMAX) {
+    s_lane[threadIdx.x] = 0;
+    s_reset[threadIdx.x] = 0;
+  }
   if (threadIdx.x == 0) s_host = s_all = 0;
   uint32_t host_acc = 0;
-  const uint64_t packed = __ldcg((const unsigned long long *)in.counter);
   const uint32_t n = (uint32_t)(packed >> CNT_SHIFT);
   const uint64_t T = packed & EDGE_MASK;
   const uint64_t nunits = (T + UNIT - 1) / UNIT;
@@ -436,9 +496,9 @@ __device__ __forceinline__ void group_map_body(FrontierView in, FrontierView out
             if (hn) qn = op.template fetch<H>(s_pay[on], jn);
           }
           uint32_t app = 0;
-          uint32_t dst[4] = {0, 0, 0, 0};
+          uint32_t dst[4] = {0, 0, 0, 0}, sl[4] = {0, 0, 0, 0};
           if (hc) {
-            app = op.visit4(s_vtx[oc], s_pay[oc], jc, s_len[oc], qc, dst);
+            app = op.visit4(s_vtx[oc], s_pay[oc], jc, s_len[oc], qc, dst, sl, s_reset);
             if (H && chunk_host) {
               const uint64_t o = s_pay[oc].off;
               if ((o & HOST_BIT) && cache_line(op.g, (o & OFF_MASK) + jc) == NO_LINE)
@@ -449,20 +509,33 @@ __device__ __forceinline__ void group_map_body(FrontierView in, FrontierView out
           jc = jn;
           qc = qn;
           hc = hn;
-          queue.push4(out, app, dst, len_of);
+          queue.push4(out, app, dst, sl);
         }
       }
       if (s_eb[GC] >= E1 || s + GC >= n) break;
       s += GC;
     }
-    queue.flush(out, 32, len_of);
+    queue.template finish<RELAX_THREADS>(out);
   }
+  // (after the walk: its loads would delay a CTA that has edges, and most have
+  // none in the small rounds)
+  clear_prev_masks(prev_vtx, prev_cnt, prev_mask);
   const unsigned long long hs = warp_sum((unsigned long long)host_acc);
   if ((threadIdx.x & 31) == 0 && hs) atomicAdd(&s_host, hs);
   __syncthreads();
   if (threadIdx.x < GMAX && s_lane[threadIdx.x]) {
     if (lane_edges) atomicAdd(&lane_edges[threadIdx.x], s_lane[threadIdx.x]);
-    if (edge_stat) atomicAdd(edge_stat, s_lane[threadIdx.x]);
+  }
+  // (one global atomic per CTA and lane; one per reset, all on the group's few
+  // counters, was most of a large snapshot's first rounds)
+  if constexpr (Op::kResets)
+    if (threadIdx.x < GMAX && s_reset[threadIdx.x])
+      atomicAdd(&op.inval[threadIdx.x], (unsigned long long)s_reset[threadIdx.x]);
+  if (threadIdx.x == 0 && edge_stat) {
+    unsigned long long all = 0;
+#pragma unroll
+    for (int q = 0; q < GMAX; ++q) all += s_lane[q];
+    if (all) atomicAdd(edge_stat, all);
   }
   if (threadIdx.x == 0 && s_host && host_stat) atomicAdd(host_stat, s_host);
   if (threadIdx.x == 0 && op.g.cstat) {
@@ -473,7 +546,7 @@ __device__ __forceinline__ void group_map_body(FrontierView in, FrontierView out
 }
 
 template <class Op, bool H>
-__global__ void __launch_bounds__(RELAX_THREADS, SGS_GROUP_MIN_BLOCKS)
+__global__ void __launch_bounds__(RELAX_THREADS, Op::kBlocks)
     group_map(FrontierView in, FrontierView out, Op op, const uint32_t *prev_vtx,
               const unsigned long long *prev_cnt, uint32_t *prev_mask,
               unsigned long long *lane_edges, unsigned long long *edge_stat,
@@ -481,7 +554,8 @@ __global__ void __launch_bounds__(RELAX_THREADS, SGS_GROUP_MIN_BLOCKS)
               const unsigned long long *resets = nullptr, unsigned long long restrict_max = 0) {
   // round 0 of a repair that k_group_sweep has done
   if (resets && repair_mode(resets, lanes, restrict_max) == REPAIR_RESTRICTED) return;
-  group_map_body<Op, H>(in, out, op, prev_vtx, prev_cnt, prev_mask, lane_edges, edge_stat, host_stat);
+  group_map_body<Op, H>(in, out, op, prev_vtx, prev_cnt, prev_mask, lane_edges, edge_stat, host_stat,
+                        __ldcg((const unsigned long long *)in.counter));
 }
 
 // The three rotating frontier buffers, their counters and lane masks, as one
@@ -515,13 +589,14 @@ struct RoundBufs {
 // kernel returns; *rounds_out = the first empty frontier's index (or
 // max_rounds when the limit is hit).
 template <class Op, bool H>
-__global__ void __launch_bounds__(RELAX_THREADS, SGS_GROUP_MIN_BLOCKS)
+__global__ void __launch_bounds__(RELAX_THREADS, Op::kBlocks)
     group_rounds(RoundBufs<uint32_t> rb, Op op, uint32_t r0, uint32_t max_rounds,
                  unsigned long long *lane_edges, unsigned long long *rstat, unsigned long long *hstat,
                  uint32_t *rounds_out) {
   cooperative_groups::grid_group grid = cooperative_groups::this_grid();
   uint32_t r = r0;
   bool conv = false;
+  uint64_t packed = __ldcg(rb.cnt + r0);
   for (; r < max_rounds; ++r) {
     Op o = op;
     o.m_in = rb.mask[r % 3];
@@ -529,10 +604,10 @@ __global__ void __launch_bounds__(RELAX_THREADS, SGS_GROUP_MIN_BLOCKS)
     const bool hp = r >= 1;
     group_map_body<Op, H>(rb.view(r), rb.view(r + 1), o, hp ? rb.vtx[(r - 1) % 3] : nullptr,
                    hp ? rb.cnt + r - 1 : nullptr, hp ? rb.mask[(r - 1) % 3] : nullptr, lane_edges,
-                   rstat + r, hstat + r);
-    __threadfence();
+                   rstat + r, hstat + r, packed);
     grid.sync();
-    if ((__ldcg(rb.cnt + r + 1) >> CNT_SHIFT) == 0) {
+    packed = __ldcg(rb.cnt + r + 1);
+    if ((packed >> CNT_SHIFT) == 0) {
       conv = true;
       ++r;
       break;
@@ -701,7 +776,7 @@ struct SweepWarp {
   // queues: up to 31 waiting and 32 new
   uint32_t q1_dst[63], q1_src[63], q1_j[63];
   uint32_t q2_dst[63], q2_src[63], q2_j[63];
-  uint32_t app[WarpQueue::CAP];
+  uint2 app[WarpQueue::CAP1];
 };
 inline size_t sweep_smem(uint32_t filter_words) {
   return sizeof(SweepWarp) * (SWEEP_THREADS / 32) + ((size_t)filter_words + 3) / 4 * 16;
@@ -731,7 +806,6 @@ __global__ void __launch_bounds__(SWEEP_THREADS, 1)
   const uint64_t W = (uint64_t)gridDim.x * (SWEEP_THREADS / 32);
   const uint64_t ub = w * nunits / W, ue = (w + 1) * nunits / W;
   WarpQueue queue(sw.app);
-  auto len_of = [&](uint32_t v) { return g.slots[v]; };
   uint32_t evald = 0, host_acc = 0;
   unsigned long long host_all = 0;
   uint32_t n1 = 0, n2 = 0;  // queued edges (warp-uniform)
@@ -772,7 +846,7 @@ __global__ void __launch_bounds__(SWEEP_THREADS, 1)
       }
       want = got && g.slots[d] && atomicOr(&op.m_out[d], got) == 0u;
     }
-    queue.push(out, want, d, len_of);
+    queue.push(out, want, d, want ? g.slots[d] : 0u);
   };
   // probes the exact bitmap for the last min(n1, 32) of queue 1
   auto probe = [&]() {
@@ -894,7 +968,7 @@ __global__ void __launch_bounds__(SWEEP_THREADS, 1)
     }
     if (n1) probe();
     if (n2) relax();
-    queue.flush(out, 32, len_of);
+    queue.flush(out, 32);
   }
   const unsigned long long ev = warp_sum((unsigned long long)evald);
   if (lane == 0 && ev && edge_stat) atomicAdd(edge_stat, ev);
@@ -925,6 +999,9 @@ __global__ void k_group_seed_deleted(GraphView g, unsigned long long *st, uint32
                                      unsigned long long *inval, uint32_t *mark, uint32_t *m_out,
                                      FrontierView out) {
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  __shared__ uint32_t s_reset[S];
+  if (threadIdx.x < S) s_reset[threadIdx.x] = 0;
+  __syncthreads();
   for (uint64_t b = (uint64_t)blockIdx.x * blockDim.x; b < n; b += stride) {
     const uint64_t i = b + threadIdx.x;
     bool want = false;
@@ -934,28 +1011,33 @@ __global__ void k_group_seed_deleted(GraphView g, unsigned long long *st, uint32
       const uint32_t u = (uint32_t)(k >> 32);
       v = (uint32_t)k;
       uint32_t bits = 0;
+      unsigned long long row[S], was[S];
+      load_row<S>(st, v, row);
+      d = g.slots[v];
 #pragma unroll
       for (int q = 0; q < S; ++q) {
-        if (!(lanes >> q & 1u)) continue;
-        const uint64_t idx = (uint64_t)v * S + q;
-        const unsigned long long cu = __ldcg(&st[idx]);
-        if ((uint32_t)cu != u) continue;
-        const bool cc = algo.at(q) == A_CC;
-        const unsigned long long rst = cc ? (((unsigned long long)v << 32) | INF32) : ~0ull;
-        if (atomicCAS(&st[idx], cu, rst) == cu) {
-          val[idx] = cc ? v : INF32;
-          bits |= 1u << q;
-          atomicAdd(&inval[q], 1ull);
-        }
+        was[q] = ~row[q];
+        if ((lanes >> q & 1u) && (uint32_t)row[q] == u)
+          was[q] = atomicCAS(&st[(uint64_t)v * S + q], row[q],
+                             algo.at(q) == A_CC ? (((unsigned long long)v << 32) | INF32) : ~0ull);
+      }
+#pragma unroll
+      for (int q = 0; q < S; ++q) {
+        if (was[q] != row[q]) continue;
+        val[(uint64_t)v * S + q] = algo.at(q) == A_CC ? v : INF32;
+        bits |= 1u << q;
+        atomicAdd(&s_reset[q], 1u);
       }
       if (bits) {
         if (mark) bit_set(mark, v);
-        d = g.slots[v];
         want = d && atomicOr(&m_out[v], bits) == 0u;
       }
     }
-    frontier_append(out, want, v, d);
+    frontier_append_block(out, want, v, d);
   }
+  __syncthreads();
+  if (threadIdx.x < S && s_reset[threadIdx.x])
+    atomicAdd(&inval[threadIdx.x], (unsigned long long)s_reset[threadIdx.x]);
 }
 
 // Relaxes just the kept inserted edges in the selected lanes: the whole
@@ -997,39 +1079,39 @@ __global__ void k_group_relax_inserted(GraphView g, unsigned long long *st, uint
       uint32_t su[S], sv[S];
       load_vals<S>(val, u, su);
       load_vals<S>(val, v, sv);
-      uint32_t bits = 0;
+      uint32_t bits = 0, cand[S], old[S];
+      d = g.slots[v];
+      const uint32_t wi = g.wmode == W_EXPLICIT ? (w ? w[i] : 1u) : g.wmode == W_SYNTH ? (u + v) % 128u + 1u : 1u;
 #pragma unroll
       for (int q = 0; q < S; ++q) {
-        if (!(lanes >> q & 1u)) continue;
         const int a = algo.at(q);
-        uint32_t cand;
-        if (a == A_CC) {
-          cand = su[q];
-        } else {
-          if (su[q] == INF32) continue;
-          uint32_t wt = 1;
-          if (a == A_SSSP)
-            wt = g.wmode == W_EXPLICIT ? w[i] : g.wmode == W_SYNTH ? (u + v) % 128u + 1u : 1u;
-          const uint64_t nd = (uint64_t)su[q] + wt;
-          if (nd >= INF32) continue;
-          cand = (uint32_t)nd;
-        }
-        if (cand >= sv[q]) continue;
-        const uint64_t idx = (uint64_t)v * S + q;
-        if (relax_mirror_packed(&val[idx], &st[idx], cand, u)) bits |= 1u << q;
+        uint64_t nd = su[q];
+        if (a != A_CC) nd += a == A_SSSP ? wi : 1u;
+        const bool ok = (lanes >> q & 1u) && (a == A_CC || su[q] != INF32) && nd < sv[q];
+        cand[q] = (uint32_t)nd;
+        old[q] = 0;
+        if (ok) old[q] = atomicMin(&val[(uint64_t)v * S + q], cand[q]);
       }
-      if (bits) {
-        d = g.slots[v];
-        want = d && atomicOr(&m_out[v], bits) == 0u;
-      }
-    }
-    frontier_append(out, want, v, d);
-  }
-  if (counted && lane_edges) {
 #pragma unroll
-    for (int q = 0; q < S; ++q)
-      if (lanes >> q & 1u) atomicAdd(&lane_edges[q], (unsigned long long)counted);
+      for (int q = 0; q < S; ++q)
+        if (old[q] > cand[q]) {  // strictly lowered
+          atomicMin(&st[(uint64_t)v * S + q], ((unsigned long long)cand[q] << 32) | u);
+          bits |= 1u << q;
+        }
+      if (bits) want = d && atomicOr(&m_out[v], bits) == 0u;
+    }
+    frontier_append_block(out, want, v, d);
   }
+  if (!lane_edges) return;
+  // one atomic per CTA and lane
+  __shared__ uint32_t s_count;
+  if (threadIdx.x == 0) s_count = 0;
+  __syncthreads();
+  counted = warp_sum(counted);
+  if ((threadIdx.x & 31) == 0 && counted) atomicAdd(&s_count, counted);
+  __syncthreads();
+  if (threadIdx.x < S && (lanes >> threadIdx.x & 1u) && s_count)
+    atomicAdd(&lane_edges[threadIdx.x], (unsigned long long)s_count);
 }
 
 // One lane of every vertex: its values from the mirror (between snapshots

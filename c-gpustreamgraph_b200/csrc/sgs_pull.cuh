@@ -310,6 +310,8 @@ __global__ void __launch_bounds__(RELAX_THREADS)
 // map's graph; a vertex is appended with its out-slots.
 template <int S>
 struct GroupPullOp {
+  static constexpr int kBlocks = 4;
+  static constexpr bool kResets = false;
   using Payload = GPay<S>;
   GraphView g;                 // the in-edge store
   const uint32_t *out_slots;   // out-store slots (append lengths)
@@ -329,7 +331,6 @@ struct GroupPullOp {
   struct Quad {
     uint4 ids, ws;
   };
-  __device__ __forceinline__ uint32_t append_len(uint32_t v) const { return out_slots[v]; }
   template <bool H>
   __device__ __forceinline__ Quad fetch(const Payload &p, uint32_t j0) const {
     Quad q;
@@ -338,7 +339,8 @@ struct GroupPullOp {
     return q;
   }
   __device__ __forceinline__ uint32_t visit4(uint32_t v, const Payload &p, uint32_t j0, uint32_t len,
-                                             const Quad &qd, uint32_t (&dst)[4]) const {
+                                             const Quad &qd, uint32_t (&dst)[4], uint32_t (&sl)[4],
+                                             uint32_t *) const {
     uint32_t best[S], bu[S];
 #pragma unroll
     for (int q = 0; q < S; ++q) {
@@ -382,7 +384,8 @@ struct GroupPullOp {
     }
     dst[0] = v;
     dst[1] = dst[2] = dst[3] = 0;
-    return bits && out_slots[v] && atomicOr(&m_out[v], bits) == 0u ? 1u : 0u;
+    sl[0] = bits ? out_slots[v] : 0u;
+    return sl[0] && atomicOr(&m_out[v], bits) == 0u ? 1u : 0u;
   }
 };
 

@@ -159,9 +159,8 @@ __device__ __forceinline__ void wide_map_body(const GraphView &g, FrontierView i
   uint32_t miss_acc = 0;  // host-tier slots this thread read over the link
   __shared__ unsigned long long s_host;  // host-tier slots of the entries this CTA owns
   if (threadIdx.x == 0) s_host = 0;
-  __shared__ uint32_t s_queue[NW][WarpQueue::CAP];
+  __shared__ uint2 s_queue[NW][WarpQueue::CAP1];
   WarpQueue queue(s_queue[warp]);
-  auto len_of = [&](uint32_t v) { return g.slots[v]; };
   __shared__ unsigned long long s_eval;
   if (threadIdx.x == 0) s_eval = 0;
   const uint64_t packed = __ldcg((const unsigned long long *)in.counter);
@@ -297,7 +296,7 @@ __device__ __forceinline__ void wide_map_body(const GraphView &g, FrontierView i
                 want = atomicOr(&m_out[vi[q]], bits) == 0ull;
             }
           }
-          queue.push(out, want, v, len_of);
+          queue.push(out, want, v, want ? g.slots[v] : 0u);
         } else if (total) {
           const uint32_t nonempty = __ballot_sync(0xFFFFFFFFu, c > 0);
           for (uint32_t ib = 0; ib < total; ib += 32) {
@@ -332,7 +331,7 @@ __device__ __forceinline__ void wide_map_body(const GraphView &g, FrontierView i
                 want = g.slots[vj] && atomicOr(&m_out[vj], 1ull << q) == 0ull;
               }
             }
-            queue.push(out, want, vj, len_of);
+            queue.push(out, want, vj, want ? g.slots[vj] : 0u);
           }
         }
       };
@@ -485,7 +484,7 @@ __device__ __forceinline__ void wide_map_body(const GraphView &g, FrontierView i
       if (s_eb[GC] >= E1 || s + GC >= n) break;
       s += GC;
     }
-    queue.flush(out, 32, len_of);
+    queue.template finish<RELAX_THREADS>(out);
   }
   // per-lane sums (thread t holds lanes t and t + 32): shared, then 64
   // global atomics per CTA
@@ -534,7 +533,6 @@ __global__ void __launch_bounds__(RELAX_THREADS, 3)
     wide_map_body<Op, H>(g, rb.view(r), rb.view(r + 1), op, rb.mask[r % 3], rb.mask[(r + 1) % 3],
                   hp ? rb.vtx[(r - 1) % 3] : nullptr, hp ? rb.cnt + r - 1 : nullptr,
                   hp ? rb.mask[(r - 1) % 3] : nullptr, lane_edges, lane_changes, rstat + r);
-    __threadfence();
     grid.sync();
     if ((__ldcg(rb.cnt + r + 1) >> CNT_SHIFT) == 0) {
       conv = true;
