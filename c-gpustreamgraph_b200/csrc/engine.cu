@@ -248,7 +248,7 @@ struct sgs_engine {
                    CTL_BIG, CTL_FIT, CTL_ZERO, CTL_ROUNDS = CTL_ZERO, CTL_TOP, CTL_INTOP = CTL_TOP + 2,
                    CTL_N = CTL_INTOP + 2 };
   DBuf<unsigned long long> ctl;
-  unsigned long long *h_ctl = nullptr;  // pinned
+  unsigned long long *h_ctl = nullptr;  // pinned, after h_cnt's
   void read_ctl() {
     CK(cudaMemcpyAsync(h_ctl, ctl.p, sizeof(unsigned long long) * CTL_N, cudaMemcpyDeviceToHost, s));
     sync();
@@ -291,7 +291,7 @@ struct sgs_engine {
   uint64_t frun = 0;                 // lanes with work in flight
   uint64_t fsusp = 0;                // lanes suspended while an update applies
   uint32_t fadmit[WLANES] = {};      // round at which each lane joined
-  DBuf<unsigned long long> flc;      // per-lane entry counts of the next frontier
+  Part<unsigned long long> flc;      // the lanes present in the next frontier, after b_lane and b_inval
   int next_qid = 1;
   sgs_engine_stats est{};
   Events ev_batch, ev_apply, ev_q;
@@ -366,7 +366,6 @@ struct sgs_engine {
     for (auto ev : kev) cudaEventDestroy(ev);
     for (auto ev : gev) cudaEventDestroy(ev);
     if (h_cnt) cudaFreeHost(h_cnt);
-    if (h_ctl) cudaFreeHost(h_ctl);
     if (s) cudaStreamDestroy(s);
   }
 
@@ -450,18 +449,19 @@ struct sgs_engine {
     CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
     CK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
     const size_t nr = (size_t)cfg.max_rounds + 2;
-    phase_len = nr + kSpecial + 2 * nr + 2 * WLANES;
+    phase_len = nr + kSpecial + 2 * nr + 2 * WLANES + 1;
     phase.ensure(phase_len);
     cnt.p = phase.p;
     rstat.p = cnt.p + nr + kSpecial;
     hstat.p = rstat.p + nr;
     b_lane.p = hstat.p + nr;
     b_inval.p = b_lane.p + WLANES;
-    CK(cudaHostAlloc((void **)&h_cnt, (cfg.max_rounds + 2 + kSpecial) * sizeof(unsigned long long),
+    flc.p = b_inval.p + WLANES;
+    CK(cudaHostAlloc((void **)&h_cnt, (cfg.max_rounds + 2 + kSpecial + CTL_N + 2 * WLANES + 1) * sizeof(unsigned long long),
                      cudaHostAllocDefault));
+    h_ctl = h_cnt + cfg.max_rounds + 2 + kSpecial;
     ctl.ensure(CTL_N);
     CK(cudaMemsetAsync(ctl.p, 0, sizeof(unsigned long long) * CTL_N, s));
-    CK(cudaHostAlloc((void **)&h_ctl, sizeof(unsigned long long) * CTL_N, cudaHostAllocDefault));
     b_err.p = (unsigned int *)(ctl.p + CTL_ERR);
     b_nkept.p = (uint32_t *)(ctl.p + CTL_NKEPT);
     b_stat.p = ctl.p + CTL_STAT;
@@ -1800,7 +1800,6 @@ struct sgs_engine {
       fg = ng.get();
       groups.push_back(std::move(ng));
     }
-    flc.ensure(WLANES);
     return *fg;
   }
   uint32_t flight_lanes() const {
@@ -1962,20 +1961,20 @@ struct sgs_engine {
                                             G.algo(), anyw});
     }
     const uint32_t nf = fr + rounds;  // the next input frontier
-    CK(cudaMemsetAsync(flc.p, 0, sizeof(unsigned long long) * WLANES, s));
+    CK(cudaMemsetAsync(flc.p, 0, sizeof(unsigned long long), s));
     if (G.wide())
-      { ++n_launch; k_lane_counts<unsigned long long><<<grid_elem(nv), 256, 0, s>>>(
+      { ++n_launch; k_lanes_present<unsigned long long><<<grid_elem(nv), 256, 0, s>>>(
           fb[nf % 3].vtx.p, cnt.p + nf, wm[nf % 3].p, flc.p); }
     else
-      { ++n_launch; k_lane_counts<uint32_t><<<grid_elem(nv), 256, 0, s>>>(fb[nf % 3].vtx.p, cnt.p + nf,
-                                                                      gm[nf % 3].p, flc.p); }
+      { ++n_launch; k_lanes_present<uint32_t><<<grid_elem(nv), 256, 0, s>>>(fb[nf % 3].vtx.p, cnt.p + nf,
+                                                                        gm[nf % 3].p, flc.p); }
     CK(cudaGetLastError());
-    unsigned long long lc[WLANES], le[WLANES];
+    unsigned long long *le = h_ctl + CTL_N;  // pinned: edges per lane, (resets), lanes present
     CK(cudaMemcpyAsync(h_cnt, cnt.p + fr, sizeof(unsigned long long) * (rounds + 1),
                        cudaMemcpyDeviceToHost, s));
-    CK(cudaMemcpyAsync(lc, flc.p, sizeof(lc), cudaMemcpyDeviceToHost, s));
-    CK(cudaMemcpyAsync(le, b_lane.p, sizeof(le), cudaMemcpyDeviceToHost, s));
+    CK(cudaMemcpyAsync(le, b_lane.p, sizeof(unsigned long long) * (2 * WLANES + 1), cudaMemcpyDeviceToHost, s));
     sync();
+    const unsigned long long present = le[2 * WLANES];
     uint32_t z = 0;  // first empty frontier of the batch, if any
     for (uint32_t k = 1; k <= rounds && !z; ++k)
       if ((h_cnt[k] >> CNT_SHIFT) == 0) z = fr + k;
@@ -1985,7 +1984,7 @@ struct sgs_engine {
       fin = frun;
     } else {
       for (int l = 0; l < G.width; ++l)
-        if ((frun >> l & 1ull) && lc[l] == 0) fin |= 1ull << l;
+        if ((frun >> l & 1ull) && !(present >> l & 1ull)) fin |= 1ull << l;
     }
     const uint32_t end = z ? z : nf;
     for (auto &q : queries) {

@@ -1202,26 +1202,18 @@ __global__ void k_group_summary_lanes(const unsigned long long *st, uint32_t nv,
   }
 }
 
-// Lanes present in a frontier: per-lane counts of its entries' mask bits
-// (narrow u32 or wide u64 masks), for a serving loop that retires a lane as
-// soon as no entry carries it.
+// Lanes present in a frontier: the OR of its entries' masks (narrow u32 or wide
+// u64), for a serving loop that retires a lane as soon as no entry carries it.
 template <class M>
-__global__ void k_lane_counts(const uint32_t *vtx, const unsigned long long *cnt, const M *mask,
-                              unsigned long long *out) {
-  __shared__ unsigned long long s[64];
-  if (threadIdx.x < 64) s[threadIdx.x] = 0;
-  __syncthreads();
+__global__ void k_lanes_present(const uint32_t *vtx, const unsigned long long *cnt, const M *mask,
+                                unsigned long long *out) {
   const uint32_t n = (uint32_t)(__ldcg(cnt) >> CNT_SHIFT);
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    unsigned long long m = (unsigned long long)__ldcg(&mask[__ldcg(&vtx[i])]);
-    while (m) {
-      const int q = __ffsll((long long)m) - 1;
-      atomicAdd(&s[q], 1ull);
-      m &= m - 1;
-    }
-  }
-  __syncthreads();
-  if (threadIdx.x < 64 && s[threadIdx.x]) atomicAdd(&out[threadIdx.x], s[threadIdx.x]);
+  unsigned long long m = 0;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    m |= (unsigned long long)__ldcg(&mask[__ldcg(&vtx[i])]);
+  const uint32_t lo = __reduce_or_sync(0xFFFFFFFFu, (uint32_t)m);
+  const uint32_t hi = sizeof(M) == 8 ? __reduce_or_sync(0xFFFFFFFFu, (uint32_t)(m >> 32)) : 0u;
+  if ((threadIdx.x & 31) == 0 && (lo | hi)) atomicOr(out, (unsigned long long)hi << 32 | lo);
 }
 
 // Dense seeding of CC lanes into a frontier that may already hold entries:
