@@ -1014,12 +1014,20 @@ struct sgs_engine {
   // Whether a narrow group's relaxation runs its round 0 as a launch of its own
   // (cfg.persistent bit 2), which a repair may then restrict to the edges into
   // reset vertices.
+  // (Not with an explicit host policy, which judges by round 0's frontier and
+  // stages the blocks it reads.)
   bool own_round0() const { return (cfg.persistent & 4u) && !(cfg.persistent & 1u); }
-  // Up to this many (lane, vertex) resets the restricted sweep is used: an
-  // eighth of the vertices, where about that share of the edges passes the
-  // filter.  (The update streams measured here reset 0.5 to 10 % of it.)
-  unsigned long long restrict_max() const { return std::max<uint32_t>(nv / 8, 1); }
+  bool may_restrict() const { return own_round0() && !cfg.host_policy; }
+  // Up to this many (lane, vertex) resets the restricted sweep is used: half
+  // the vertices.  Measured with three lanes, a snapshot with the full sweep
+  // against the restricted one: at 2^22 vertices 1234 against 767 us with
+  // 0.0025 resets per vertex, 1814 against 1310 with 0.054, 2708 against 2243
+  // with 0.18, 5303 against 5245 with 0.64; at 2^20 667 against 566 with
+  // 0.0027, 1142 against 1051 with 0.18, 1773 against 1699 with 0.61; at 2^16
+  // equal within 2 % throughout.
+  unsigned long long restrict_max() const { return std::max<uint32_t>(nv / 2, 1); }
   DBuf<uint32_t> b_coarse;  // folded reset bitmap
+  DBuf<uint2> b_slices;     // k_group_sweep's slices of large blocks
   void launch_sweep(Group &G, const GroupRelaxOp<GMAX> &op, unsigned long long rmax) {
     uint32_t shift = 0;
     while (((nv - 1) >> shift) >= SWEEP_FILTER_BITS) ++shift;
@@ -1029,12 +1037,40 @@ struct sgs_engine {
       { ++n_launch; k_fold_bits<<<grid_elem(words), 256, 0, s>>>(G.ibits.p, (nv - 1) / 32 + 1, shift, b_coarse.p,
                                                                  words); }
     }
-    auto k = host_tier() ? k_group_sweep<true> : k_group_sweep<false>;
-    const size_t smem = sweep_smem(words);
-    CK(cudaFuncSetAttribute((const void *)k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    { ++n_launch; k<<<(uint32_t)nsm, SWEEP_THREADS, smem, s>>>(
-        fview(0, cnt.p), fview(1, cnt.p + 1), op, G.ibits.p, b_coarse.p, words, shift, (uint32_t)G.used, G.resets(),
-        rmax, rstat.p, hstat.p); }
+    SweepCtx c{};
+    c.bits = G.ibits.p;
+    c.coarse = b_coarse.p;
+    uint32_t kept = 16;
+    while (kept < words) kept *= 2;
+    c.filter_words = words;
+    c.filter_mask = kept - 1;
+    c.shift = shift;
+    c.lanes = (uint32_t)G.used;
+    c.resets = G.resets();
+    c.restrict_max = rmax;
+    c.next = special(0);
+    c.n_slices = special(1);
+    c.walked = special(2);
+    // a block of more than SWEEP_BIG slots has at most one slice per SWEEP_BIG
+    b_slices.ensure((arena_cap[0] + arena_cap[1]) / SWEEP_BIG + 1);
+    c.slices = b_slices.p;
+    // a few batches per warp, but not so many that the counter sets the pace;
+    // fewer than 32 vertices at a time where that would leave warps without any
+    const uint32_t per_warp = nv / ((uint32_t)nsm * (SWEEP_THREADS / 32));
+    c.step = 32;
+    while (c.step > 4 && c.step > per_warp) c.step /= 2;
+    c.batch = std::min<uint32_t>(128, std::max<uint32_t>(c.step, per_warp / 16 / 32 * 32));
+    c.lane_edges = b_lane.p;
+    c.edge_stat = rstat.p;
+    c.host_stat = hstat.p;
+    const void *k = host_tier() ? (const void *)k_group_sweep<true> : (const void *)k_group_sweep<false>;
+    const size_t smem = sweep_smem(kept);
+    CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    FrontierView out = fview(1, cnt.p + 1);
+    GroupRelaxOp<GMAX> o = op;
+    void *args[] = {&out, &o, &c};
+    ++n_launch;
+    CK(cudaLaunchCooperativeKernel(k, nsm, SWEEP_THREADS, args, smem, s));
     CK(cudaGetLastError());
   }
 
@@ -1295,7 +1331,8 @@ struct sgs_engine {
       launch_group(0, op0, (uint32_t)G.used, rmax ? G.resets() : nullptr, rmax);
       if (ktiming) {
         CK(cudaEventRecord(kev[1], s));
-        unsigned long long c0 = 0, r0s = 0, h0 = 0, rs[GMAX] = {}, nr = 0;
+        unsigned long long c0 = 0, cw = 0, r0s = 0, h0 = 0, rs[GMAX] = {}, nr = 0;
+        CK(cudaMemcpyAsync(&cw, special(2), sizeof(cw), cudaMemcpyDeviceToHost, s));
         if (rmax) CK(cudaMemcpyAsync(rs, G.resets(), sizeof(rs), cudaMemcpyDeviceToHost, s));
         CK(cudaMemcpyAsync(&c0, cnt.p, sizeof(c0), cudaMemcpyDeviceToHost, s));
         CK(cudaMemcpyAsync(&r0s, rstat.p, sizeof(r0s), cudaMemcpyDeviceToHost, s));
@@ -1304,7 +1341,7 @@ struct sgs_engine {
         for (int q = 0; q < GMAX; ++q) nr += (G.used >> q & 1u) ? rs[q] : 0;
         // the restricted sweep reads weights only for the pairs it relaxes
         const bool restricted = rmax && nr && nr <= rmax;
-        account(SGS_K_GROUP_SWEEP, c0, r0s, anyw && !restricted ? 8.0 : 4.0, 8.0, kev[0], kev[1], h0);
+        account(SGS_K_GROUP_SWEEP, restricted ? cw : c0, r0s, anyw && !restricted ? 8.0 : 4.0, 8.0, kev[0], kev[1], h0);
       }
       if (round0) nvtxRangePop();
       return run_group_persistent(GroupRelaxOp<GMAX>{g, G.st.p, G.val.p, nullptr, nullptr, G.algo(), anyw}, 1,
@@ -2386,12 +2423,12 @@ struct sgs_engine {
       if (G.wide()) {  // the lanes this invalidation resets, per vertex
         G.wreset.ensure(nv);
         CK(cudaMemsetAsync(G.wreset.p, 0, sizeof(unsigned long long) * nv, s));
-      } else if (prep || own_round0()) {  // bitmap of the vertices this invalidation resets
+      } else if (prep || may_restrict()) {  // bitmap of the vertices this invalidation resets
         const size_t nw = (size_t)nv / 32 + 1;
         G.ibits.ensure(nw);
         CK(cudaMemsetAsync(G.ibits.p, 0, sizeof(uint32_t) * nw, s));
       }
-      uint32_t *nmark = prep || own_round0() ? G.ibits.p : nullptr;
+      uint32_t *nmark = prep || may_restrict() ? G.ibits.p : nullptr;
       bool conv = false;
       if (G.wide()) {
         { ++n_launch; k_wide_seed_deleted<<<grid_elem(nd), 256, 0, s>>>(
@@ -2501,7 +2538,7 @@ struct sgs_engine {
       // the path is chosen on the device from the group's reset counts: the
       // dense frontier only if a lane was reset
       const unsigned long long *resets = G.resets();
-      const unsigned long long rmax = !G.wide() && gdel[i] && own_round0() ? restrict_max() : 0;
+      const unsigned long long rmax = !G.wide() && gdel[i] && may_restrict() ? restrict_max() : 0;
       if (!G.wide() && prep) {  // work-efficient repair: pull into the reset vertices
         bool conv = false;
         grounds[i] = pull_repair(G, gdel[i] != 0, ni, explicit_w);
@@ -2516,7 +2553,7 @@ struct sgs_engine {
                                                                fview(0, cnt.p), resets); }
       else
         { ++n_launch; k_group_dense<GMAX><<<grid_elem(nv), 256, 0, s>>>(g, G.val.p, (uint32_t)G.used, G.algo(),
-                                                            gm[0].p, fview(0, cnt.p), resets, rmax, b_lane.p); }
+                                                            gm[0].p, fview(0, cnt.p), resets, rmax); }
       if (ni && !G.wide())  // narrow, the sweep does not cover them
         { ++n_launch; k_group_relax_inserted<GMAX><<<grid_elem(ni), 256, 0, s>>>(
             g, G.st.p, G.val.p, (uint32_t)G.used, G.algo(), b_ikept.p, explicit_w ? b_iw_kept.p : nullptr,

@@ -636,97 +636,43 @@ __global__ void k_group_init_lane(unsigned long long *st, uint32_t *val, uint32_
 }
 
 // Every vertex with a non-empty block; mask = selected lanes whose value is
-// finite there (CC lanes always).  One writer per vertex: plain stores.  With
-// `resets`: nothing in mode NONE; in mode RESTRICTED no masks (k_group_sweep
-// reads none) but the (lane, edge) pairs of the sweep added to lane_edges.
-// Bound by memory: 20 B read and 16-20 B written per vertex.  A warp takes 32
-// consecutive vertices per step (one 512-B read of their values) and scans
-// the eight steps of its 256 one after the other; the block appends its 2048
-// vertices, in order, with one atomic.
+// finite there (CC lanes always).  One writer per vertex: plain stores.
+// With `resets`, only in repair mode FULL.
 template <int S>
-__global__ void __launch_bounds__(RELAX_THREADS)
-    k_group_dense(GraphView g, const uint32_t *val, uint32_t lanes, LaneAlgo algo, uint32_t *m_out,
-                  FrontierView out, const unsigned long long *resets = nullptr,
-                  unsigned long long restrict_max = 0, unsigned long long *lane_edges = nullptr) {
-  constexpr int N = 8, NW = RELAX_THREADS / 32;
-  __shared__ unsigned long long s_warp[NW], s_base;
-  const int mode = resets ? repair_mode(resets, lanes, restrict_max) : REPAIR_FULL;
-  if (mode == REPAIR_NONE) return;
-  const unsigned full = 0xFFFFFFFFu;
-  const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  unsigned long long edges[S] = {};
-  const uint64_t stride = (uint64_t)gridDim.x * RELAX_THREADS * N;
-  for (uint64_t b = (uint64_t)blockIdx.x * RELAX_THREADS * N; b < g.nv; b += stride) {
-    const uint64_t v0 = b + (uint64_t)wid * 32 * N + lane;
-    uint32_t d[N], m[N];
-    uint32_t blk[N][S];
-#pragma unroll
-    for (int i = 0; i < N; ++i) d[i] = v0 + 32 * i < g.nv ? g.slots[v0 + 32 * i] : 0u;
-#pragma unroll
-    for (int i = 0; i < N; ++i)
-      if (d[i]) load_vals<S>(val, (uint32_t)(v0 + 32 * i), blk[i]);
+__global__ void k_group_dense(GraphView g, const uint32_t *val, uint32_t lanes,
+                              LaneAlgo algo, uint32_t *m_out, FrontierView out,
+                              const unsigned long long *resets = nullptr,
+                              unsigned long long restrict_max = 0) {
+  if (resets && repair_mode(resets, lanes, restrict_max) != REPAIR_FULL) return;
+  // eight consecutive vertices per thread, one block append per 2048
+  constexpr int N = 8;
+  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x * N;
+  for (uint64_t b = (uint64_t)blockIdx.x * blockDim.x * N; b < g.nv; b += stride) {
+    const uint64_t v0 = b + (uint64_t)threadIdx.x * N;
+    bool want[N];
+    uint32_t d[N];
 #pragma unroll
     for (int i = 0; i < N; ++i) {
-      m[i] = 0;
-      if (d[i]) {
+      const uint64_t v = v0 + i;
+      want[i] = false;
+      d[i] = 0;
+      if (v < g.nv) {
+        d[i] = g.slots[v];
+        if (d[i]) {
+          uint32_t blk[S];
+          load_vals<S>(val, (uint32_t)v, blk);
+          uint32_t m = 0;
 #pragma unroll
-        for (int q = 0; q < S; ++q)
-          if ((lanes >> q & 1u) && (algo.at(q) == A_CC || blk[i][q] != INF32)) m[i] |= 1u << q;
-        if (mode == REPAIR_RESTRICTED && m[i]) {
-          const uint32_t l = g.live[v0 + 32 * i];
-#pragma unroll
-          for (int q = 0; q < S; ++q) edges[q] += (m[i] >> q & 1u) ? l : 0u;
+          for (int q = 0; q < S; ++q)
+            if ((lanes >> q & 1u) && (algo.at(q) == A_CC || blk[q] != INF32)) m |= 1u << q;
+          if (m) {
+            m_out[v] = m;
+            want[i] = true;
+          }
         }
       }
     }
-    // inclusive scans of the (count, padded slots) words, step after step
-    unsigned long long x[N], run = 0;
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-      x[i] = m[i] ? (1ull << CNT_SHIFT) | (unsigned long long)((d[i] + 3u) & ~3u) : 0ull;
-#pragma unroll
-      for (int s = 1; s < 32; s <<= 1) {
-        const unsigned long long y = __shfl_up_sync(full, x[i], s);
-        if (lane >= (uint32_t)s) x[i] += y;
-      }
-      x[i] += run;
-      run = __shfl_sync(full, x[i], 31);
-    }
-    if (lane == 0) s_warp[wid] = run;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      unsigned long long t = 0;
-      for (int w = 0; w < NW; ++w) {
-        const unsigned long long y = s_warp[w];
-        s_warp[w] = t;
-        t += y;
-      }
-      s_base = t ? atomicAdd((unsigned long long *)out.counter, t) : 0ull;
-    }
-    __syncthreads();
-    const unsigned long long base = s_base + s_warp[wid];
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-      if (!m[i]) continue;
-      const uint32_t v = (uint32_t)(v0 + 32 * i), dp = (d[i] + 3u) & ~3u;
-      const unsigned long long pos = base + x[i] - ((1ull << CNT_SHIFT) | (unsigned long long)dp);
-      const uint32_t slot = (uint32_t)(pos >> CNT_SHIFT);
-      const uint64_t eb = pos & EDGE_MASK;
-      out.vtx[slot] = v;
-      out.len[slot] = d[i];
-      out.ebase[slot] = eb;
-      const uint64_t u0 = (eb + UNIT - 1) / UNIT, u1 = (eb + dp - 1) / UNIT;
-      for (uint64_t u = u0; u <= u1 && u < out.ucap; ++u) out.ustart[u] = slot;
-      if (mode == REPAIR_FULL) m_out[v] = m[i];
-    }
-    __syncthreads();  // s_warp / s_base are rewritten by the next step
-  }
-  if (lane_edges && mode == REPAIR_RESTRICTED) {
-#pragma unroll
-    for (int q = 0; q < S; ++q) {
-      const unsigned long long e = warp_sum(edges[q]);
-      if (lane == 0 && e) atomicAdd(&lane_edges[q], e);
-    }
+    frontier_append_block_n<N>(out, want, (uint32_t)v0, d);
   }
 }
 
@@ -751,234 +697,387 @@ __global__ void k_fold_bits(const uint32_t *bits, uint32_t nwords, uint32_t shif
 }
 
 // Round 0 of a narrow group's repair in mode RESTRICTED: a walk of the ids of
-// every reached vertex's block (the dense frontier), in which only the edges
-// into reset vertices are relaxed.
+// every reached vertex's block in which only the edges into reset vertices are
+// relaxed.
 //
-// The full sweep reads a random 16-B mirror row per slot, and that gather
-// (one L1 tag per slot, and DRAM for the rows that miss L2), not the id
-// stream, sets its time.  Here a slot costs one bit of a filter in shared
-// memory: the reset bitmap, for up to 2^20 vertices exactly, above that one bit
-// per 2^shift consecutive vertices, with the exact bitmap probed for the slots
-// that pass.  What passes goes through per-warp queues and is handled 32
-// edges at a time, so the few edges per window that need the rows of both
-// ends do not stall the walk with mostly idle warps.
-// One CTA of 32 warps per SM (the filter takes 128 KB); every warp walks its
-// own run of units with 32 staged entries, two windows of ids in flight, and
-// no barrier.  With 65 % of a million-vertex graph in host memory a snapshot
-// goes from 4.9 to 3.6 ms, since weights are read for the few relaxed edges only;
-// with all of it in HBM the sweep takes as long as the full one (1.56 and 1.67 ms
-// at scale 24).
+// The full sweep reads a random 16-B mirror row per slot, and that gather, not
+// the id stream, sets its time.  Here a slot costs one bit of a filter in
+// shared memory: the reset bitmap, for up to 2^20 vertices exactly, above that
+// one bit per 2^shift consecutive vertices, with the exact bitmap probed for
+// the slots that pass.  What passes goes through per-warp queues and is
+// handled 32 edges at a time, so the few edges per window that need the rows
+// of both ends do not stall the walk with mostly idle warps.  The walk is then
+// bound by the instructions per slot, so it goes over the vertices themselves,
+// 32 consecutive ones per warp and step, instead of a frontier built and read
+// back (that was 0.2 ms of scale 24's 1.9): their blocks' starts come from
+// a warp scan, a quad's owner from the OR of starts (as in group_map, in 32
+// bits).  Blocks of more than SWEEP_BIG slots are cut into slices, listed by the
+// first phase and walked by all warps after a grid barrier, without owners.
+// Warps take vertices from a counter, since blocks differ widely in size.
+// One CTA of 32 warps per SM (the filter takes 128 KB).
+// Scale 24, three lanes, a million updates: 1.06 ms; 1.55 and 0.26 for the
+// frontier when it took its blocks from one, 1.67 and 0.21 as the full sweep.
+// Scale 16: 38 us against 37 + 12.  With the blocks behind the host link
+// (2^20 vertices, 0.35 of the graph in HBM) 1.36 ms either way: the link.
 constexpr int SWEEP_THREADS = 1024;
 constexpr uint32_t SWEEP_FILTER_BITS = 1u << 20;
+constexpr uint32_t SWEEP_SLICE = 1024;
+constexpr uint32_t SWEEP_BIG = 256;  // a step's 32 blocks then hold 64 windows at most
 struct SweepWarp {
-  uint64_t eb[33], off[32];
-  uint32_t len[32], vtx[32];
-  // queues: up to 31 waiting and 32 new
-  uint32_t q1_dst[63], q1_src[63], q1_j[63];
-  uint32_t q2_dst[63], q2_src[63], q2_j[63];
+  uint64_t off[32];
+  uint32_t eb[33], len[32], vtx[32];
+  // queue 1: slots that passed the filter; queue 2: edges into reset vertices
+  // (up to 31 waiting, 32 new)
+  uint32_t d1[63], s1[63], j1[63];
+  uint32_t d2[63], s2[63], j2[63];
   uint2 app[WarpQueue::CAP1];
 };
-inline size_t sweep_smem(uint32_t filter_words) {
-  return sizeof(SweepWarp) * (SWEEP_THREADS / 32) + ((size_t)filter_words + 3) / 4 * 16;
+inline size_t sweep_smem(uint32_t filter_words) {  // (a power of two, at least 16)
+  return sizeof(SweepWarp) * (SWEEP_THREADS / 32) + (size_t)filter_words * 4;
 }
+// Counters (zero before the launch) and lists of a sweep.
+struct SweepCtx {
+  const uint32_t *bits, *coarse;  // reset bitmap and its folded form (shift > 0)
+  uint32_t filter_words, filter_mask, shift, lanes;  // words given; words kept - 1 (all ones)
+  const unsigned long long *resets;
+  unsigned long long restrict_max;
+  unsigned long long *next;       // next vertex to take
+  unsigned long long *n_slices;   // slices listed
+  unsigned long long *walked;     // packed (vertices << CNT_SHIFT | padded slots)
+  uint2 *slices;                  // (vertex, slice)
+  uint32_t batch, step;           // vertices taken at a time, and walked at a time (at most 32)
+  unsigned long long *lane_edges, *edge_stat, *host_stat;
+};
 
 template <bool H>
 __global__ void __launch_bounds__(SWEEP_THREADS, 1)
-    k_group_sweep(FrontierView in, FrontierView out, GroupRelaxOp<GMAX> op, const uint32_t *bits,
-                  const uint32_t *coarse, uint32_t filter_words, uint32_t shift, uint32_t lanes,
-                  const unsigned long long *resets, unsigned long long restrict_max,
-                  unsigned long long *edge_stat, unsigned long long *host_stat) {
-  if (repair_mode(resets, lanes, restrict_max) != REPAIR_RESTRICTED) return;
+    k_group_sweep(FrontierView out, GroupRelaxOp<GMAX> op, SweepCtx c) {
+  if (repair_mode(c.resets, c.lanes, c.restrict_max) != REPAIR_RESTRICTED) return;
   extern __shared__ __align__(16) unsigned char s_raw[];
   SweepWarp &sw = reinterpret_cast<SweepWarp *>(s_raw)[threadIdx.x >> 5];
   uint32_t *filter = reinterpret_cast<uint32_t *>(s_raw + sizeof(SweepWarp) * (SWEEP_THREADS / 32));
-  const uint32_t *f_src = shift ? coarse : bits;
-  for (uint32_t i = threadIdx.x; i < filter_words; i += SWEEP_THREADS) filter[i] = f_src[i];
+  // (its length is a power of two, so that any id, a tombstone too, can be
+  // masked into it; what a false hit of that kind leads to checks the id)
+  {
+    const uint32_t *f_src = c.shift ? c.coarse : c.bits;
+    for (uint32_t i = threadIdx.x; i <= c.filter_mask; i += SWEEP_THREADS)
+      filter[i] = i < c.filter_words ? f_src[i] : 0u;
+  }
   __syncthreads();
   const GraphView &g = op.g;
-  const uint32_t lane = threadIdx.x & 31;
-  const uint64_t packed = __ldcg((const unsigned long long *)in.counter);
-  const uint32_t n = (uint32_t)(packed >> CNT_SHIFT);
-  const uint64_t T = packed & EDGE_MASK;
-  const uint64_t nunits = (T + UNIT - 1) / UNIT;
-  // a small frontier's units go to warps of different SMs
-  const uint64_t w = (uint64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
-  const uint64_t W = (uint64_t)gridDim.x * (SWEEP_THREADS / 32);
-  const uint64_t ub = w * nunits / W, ue = (w + 1) * nunits / W;
+  const uint32_t lane = threadIdx.x & 31, below = (1u << lane) - 1u, full = 0xFFFFFFFFu;
+  const uint32_t shift = c.shift, shift5 = shift + 5, mask = c.filter_mask;
   WarpQueue queue(sw.app);
-  uint32_t evald = 0, host_acc = 0;
-  unsigned long long host_all = 0;
-  uint32_t n1 = 0, n2 = 0;  // queued edges (warp-uniform)
-  // relaxes the last min(n2, 32) of queue 2
-  auto relax = [&]() {
-    const uint32_t c = min(n2, 32u);
-    const bool on = lane < c;
-    uint32_t d = 0, u = 0, j = 0;
-    if (on) {
-      d = sw.q2_dst[n2 - c + lane];
-      u = sw.q2_src[n2 - c + lane];
-      j = sw.q2_j[n2 - c + lane];
-    }
-    n2 -= c;
-    __syncwarp();
-    bool want = false;
-    if (on) {
-      uint32_t su[GMAX], cur[GMAX];
-      load_vals<GMAX>(op.val, u, su);
-      load_vals<GMAX>(op.val, d, cur);
-      uint32_t wt = 1;
-      if (op.any_w) {
-        if (g.wmode == W_EXPLICIT) wt = H ? *wgt_at(g, g.off[u], j) : g.wgt_d[g.off[u] + j];
-        else if (g.wmode == W_SYNTH) wt = (u + d) % 128u + 1u;
-      } else if (g.wmode == W_SYNTH) {
-        wt = (u + d) % 128u + 1u;
+  uint32_t evald = 0, host_acc = 0, n1 = 0, n2 = 0;  // n1, n2: queued (warp-uniform)
+  unsigned long long host_all = 0, walked = 0, edges[GMAX] = {};
+  // Takes the last 32 (or fewer) of queue 1: relaxes them when the filter is
+  // exact, else probes the bitmap, queues those that lead into reset vertices and
+  // relaxes these 32 at a time.  `all`: both queues, to the end.
+  auto drain = [&](bool all) {
+    const uint32_t *qd = shift ? sw.d2 : sw.d1, *qs = shift ? sw.s2 : sw.s1, *qj = shift ? sw.j2 : sw.j1;
+#pragma unroll 1
+    do {
+      uint32_t d = 0, u = 0, j = 0;
+      if (shift && n1) {
+        const uint32_t k = min(n1, 32u);
+        bool on = false;
+        if (lane < k) {
+          d = sw.d1[n1 - k + lane];
+          u = sw.s1[n1 - k + lane];
+          j = sw.j1[n1 - k + lane];
+          on = d != SGS_TOMB && (__ldg(c.bits + (d >> 5)) >> (d & 31) & 1u);
+        }
+        n1 -= k;
+        const uint32_t m = __ballot_sync(full, on);
+        if (on) {
+          const uint32_t at = n2 + __popc(m & below);
+          sw.d2[at] = d;
+          sw.s2[at] = u;
+          sw.j2[at] = j;
+        }
+        n2 += __popc(m);
+        __syncwarp();
       }
-      uint32_t got = 0;
+      // edges to relax: queue 2, or queue 1 itself when the filter is exact
+      uint32_t n = shift ? n2 : n1;
+      if (n >= 32 || (all && n)) {
+        const uint32_t k = min(n, 32u);
+        bool want = false;
+        uint32_t sd = 0;
+        if (lane < k) {
+          d = qd[n - k + lane];
+          u = qs[n - k + lane];
+          j = qj[n - k + lane];
+        }
+        __syncwarp();
+        n -= k;
+        if (shift) n2 = n;
+        else n1 = n;
+        if (lane < k && d != SGS_TOMB) {
+          uint32_t su[GMAX], cv[GMAX], cand[GMAX], old[GMAX];
+          load_vals<GMAX>(op.val, u, su);
+          load_vals<GMAX>(op.val, d, cv);
+          sd = g.slots[d];
+          uint32_t wt = 1;
+          if (g.wmode == W_EXPLICIT) {
+            if (op.any_w) wt = H ? *wgt_at(g, g.off[u], j) : g.wgt_d[g.off[u] + j];
+          } else if (g.wmode == W_SYNTH) {
+            wt = (u + d) % 128u + 1u;
+          }
+          uint32_t got = 0;
 #pragma unroll
-      for (int q = 0; q < GMAX; ++q) {
-        if (!(lanes >> q & 1u)) continue;
-        if (su[q] == INF32 && !(op.algo.cc >> q & 1u)) continue;
-        ++evald;
-        const uint32_t cand = op.cand_of(su[q] + (op.algo.inc >> q & 1u), wt, q);
-        if (cand >= cur[q]) continue;
-        const uint64_t idx = (uint64_t)d * GMAX + q;
-        if (relax_mirror_packed(&op.val[idx], &op.st[idx], cand, u)) got |= 1u << q;
-      }
-      want = got && g.slots[d] && atomicOr(&op.m_out[d], got) == 0u;
-    }
-    queue.push(out, want, d, want ? g.slots[d] : 0u);
-  };
-  // probes the exact bitmap for the last min(n1, 32) of queue 1
-  auto probe = [&]() {
-    const uint32_t c = min(n1, 32u);
-    bool on = lane < c;
-    uint32_t d = 0, u = 0, j = 0;
-    if (on) {
-      d = sw.q1_dst[n1 - c + lane];
-      u = sw.q1_src[n1 - c + lane];
-      j = sw.q1_j[n1 - c + lane];
-      on = __ldg(bits + (d >> 5)) >> (d & 31) & 1u;
-    }
-    n1 -= c;
-    const uint32_t m = __ballot_sync(0xFFFFFFFFu, on);
-    if (on) {
-      const uint32_t at = n2 + __popc(m & ((1u << lane) - 1u));
-      sw.q2_dst[at] = d;
-      sw.q2_src[at] = u;
-      sw.q2_j[at] = j;
-    }
-    n2 += __popc(m);
-    __syncwarp();
-    if (n2 >= 32) relax();
-  };
-  if (n != 0 && ub < ue) {
-    const uint64_t E0 = ub * UNIT, E1 = min(ue * (uint64_t)UNIT, T);
-    uint32_t s = __ldcg(&in.ustart[ub]);
-    for (;;) {
-      const uint32_t idx = s + lane;
-      const uint64_t eb = idx < n ? __ldcg((const unsigned long long *)&in.ebase[idx]) : T;
-      if (lane == 0) sw.eb[32] = s + 32 < n ? __ldcg((const unsigned long long *)&in.ebase[s + 32]) : T;
-      sw.eb[lane] = eb;
-      if (idx < n && eb < E1) {
-        const uint32_t v = __ldcg(&in.vtx[idx]), l = __ldcg(&in.len[idx]);
-        uint64_t o = g.off[v];
-        if constexpr (H) {
-          if (o & HOST_BIT) {
-            if (eb >= E0) {
-              hot_bump(g, v, o);
-              host_all += l;
+          for (int q = 0; q < GMAX; ++q) {
+            const bool on_q = (c.lanes >> q & 1u) && (su[q] != INF32 || (op.algo.cc >> q & 1u));
+            evald += on_q;
+            cand[q] = op.cand_of(su[q] + (op.algo.inc >> q & 1u), wt, q);
+            old[q] = 0;
+            if (on_q && cand[q] < cv[q]) old[q] = atomicMin(&op.val[(uint64_t)d * GMAX + q], cand[q]);
+          }
+#pragma unroll
+          for (int q = 0; q < GMAX; ++q)
+            if (old[q] > cand[q]) {  // strictly lowered
+              atomicMin(&op.st[(uint64_t)d * GMAX + q], ((unsigned long long)cand[q] << 32) | u);
+              got |= 1u << q;
             }
-            o = resolve_block(g, o, l);
+          want = got && sd && atomicOr(&op.m_out[d], got) == 0u;
+        }
+        __syncwarp();
+        queue.push(out, want, d, sd);
+      }
+    } while (all ? (n1 | n2) != 0 : n1 >= 32);
+  };
+  // ---- where windows come from.  Phase 1: `step` consecutive vertices at a
+  // time, their blocks' quads one after the other; phase 2, after a grid barrier:
+  // slices of the large blocks.  One loop over both, so that the test, the queues
+  // and the relaxation are in the code once (inlined at several places they
+  // overflowed the instruction cache).
+  bool slices = false;                          // phase 2
+  uint32_t v0 = 0, ve = 0;                      // vertices of the batch
+  uint32_t p = 0, total = 0, s0 = 0;            // positions of the step (phase 2: of the slice)
+  uint32_t si = (threadIdx.x >> 5) * gridDim.x + blockIdx.x, ns = 0;  // slice, slices
+  uint2 cur = make_uint2(0, 0), nxs = make_uint2(0, 0);
+  uint64_t co = 0, nxo = 0;
+  uint32_t nxl = 0;
+  struct Win {
+    uint32_t u, j, left;
+    uint4 ids;
+  };
+  // loads the next window of the positions at hand; false: none is left
+  auto fetch = [&](Win &w) -> bool {
+    w.left = 0;
+    if (p >= total) return false;
+    const uint32_t at = p + 4 * lane;
+    uint64_t o = co;
+    if (slices) {
+      w.u = cur.x;
+      w.j = cur.y * SWEEP_SLICE + at;
+      if (at < total) w.left = total - at;
+    } else {
+      const uint32_t pe = p + 128u, j = s0 + lane;
+      const uint32_t bj = j <= 32u ? sw.eb[j] : total;
+      const uint32_t m = __reduce_or_sync(full, (lane && bj < pe) ? 1u << ((bj - p) >> 2) : 0u);
+      const uint32_t own = s0 + __popc(m & (full >> (31 - lane)));
+      uint32_t nx = s0 + __popc(m);
+      if (nx < 32u && sw.eb[nx + 1] <= pe) ++nx;  // an entry starting exactly at pe
+      s0 = nx;
+      if (at < total) {
+        w.u = sw.vtx[own];
+        w.j = at - sw.eb[own];
+        w.left = sw.len[own] - w.j;
+        o = sw.off[own];
+      }
+    }
+    if (w.left) {
+      w.ids = ld_quad_stream(H ? adj_at(g, o, w.j) : g.adj_d + o + w.j);
+      if constexpr (H)
+        if ((o & HOST_BIT) && cache_line(g, (o & OFF_MASK) + w.j) == NO_LINE) host_acc += min(4u, w.left);
+    }
+    p += 128u;
+    return true;
+  };
+  for (;;) {
+    // ---- the next positions
+    if (!slices) {
+      if (v0 >= ve) {
+        unsigned long long b = 0;
+        if (lane == 0) b = atomicAdd(c.next, (unsigned long long)c.batch);
+        b = __shfl_sync(full, b, 0);
+        if (b >= g.nv) {
+          cooperative_groups::this_grid().sync();
+          slices = true;
+          ns = (uint32_t)__ldcg(c.n_slices);
+          if (si < ns) {
+            nxs = __ldcg(&c.slices[si]);
+            nxl = g.slots[nxs.x];
+            nxo = g.off[nxs.x];
+          }
+          continue;
+        }
+        v0 = (uint32_t)b;
+        ve = (uint32_t)min(b + c.batch, (unsigned long long)g.nv);
+      }
+      const uint32_t v = v0 + lane;
+      uint32_t len = lane < c.step && v < ve ? g.slots[v] : 0u;
+      v0 += c.step;
+      uint64_t o = 0;
+      if (len) {
+        uint32_t x[GMAX];
+        load_vals<GMAX>(op.val, v, x);
+        o = g.off[v];
+        const uint32_t l = g.live[v];
+        uint32_t m = 0;
+#pragma unroll
+        for (int q = 0; q < GMAX; ++q) {
+          const bool r = (c.lanes >> q & 1u) && (x[q] != INF32 || (op.algo.cc >> q & 1u));
+          m |= (r ? 1u : 0u) << q;
+          edges[q] += r ? l : 0u;
+        }
+        if (!m) len = 0;
+        else walked += (1ull << CNT_SHIFT) | ((len + 3u) & ~3u);
+        if constexpr (H) {
+          if (len && (o & HOST_BIT)) {
+            hot_bump(g, v, o);
+            host_all += len;
+            o = resolve_block(g, o, len);
           }
         }
-        sw.vtx[lane] = v;
-        sw.len[lane] = l;
-        sw.off[lane] = o;
+      }
+      // slices of large blocks
+      for (uint32_t big = __ballot_sync(full, len > SWEEP_BIG); big; big &= big - 1) {
+        const int from = __ffs(big) - 1;
+        const uint32_t n = (__shfl_sync(full, len, from) + SWEEP_SLICE - 1) / SWEEP_SLICE;
+        unsigned long long at = 0;
+        if (lane == 0) at = atomicAdd(c.n_slices, (unsigned long long)n);
+        at = __shfl_sync(full, at, 0);
+        const uint32_t bv = __shfl_sync(full, v, from);
+        for (uint32_t i = lane; i < n; i += 32) c.slices[at + i] = make_uint2(bv, i);
+      }
+      if (len > SWEEP_BIG) len = 0;
+      const uint32_t some = __ballot_sync(full, len != 0u);
+      if (!some) continue;
+      const uint32_t pad = (len + 3u) & ~3u;
+      uint32_t x = pad;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t y = __shfl_up_sync(full, x, d);
+        if (lane >= (uint32_t)d) x += y;
+      }
+      total = __shfl_sync(full, x, 31);
+      const uint32_t ne = __popc(some);
+      __syncwarp();  // the last step's entries are read
+      if (lane >= ne) sw.eb[lane] = total;
+      if (lane == 0) sw.eb[32] = total;
+      if (len) {
+        const uint32_t at = __popc(some & below);
+        sw.eb[at] = x - pad;
+        sw.off[at] = o;
+        sw.len[at] = len;
+        sw.vtx[at] = v;
       }
       __syncwarp();
-      WindowWalk<32> walk(sw.eb, sw.len, max(E0, sw.eb[0]), min(E1, sw.eb[32]), 0, 1);
-      struct Win {
-        int own;
-        uint32_t j;
-        bool has;
-        uint4 ids;
-      };
-      auto fetch = [&](Win &x) -> bool {
-        if (walk.q >= walk.end) return false;
-        x.has = walk.next(x.own, x.j);
-        if (x.has) x.ids = ld_quad_stream(H ? adj_at(g, sw.off[x.own], x.j) : g.adj_d + sw.off[x.own] + x.j);
-        return true;
-      };
-      Win a{}, b{};
-      bool more = fetch(a), more_b = more && fetch(b);
-      while (more) {
-        Win c{};
-        const bool more_c = more_b && fetch(c);
-        const uint32_t left = a.has ? sw.len[a.own] - a.j : 0u;
-        const uint32_t u = a.has ? sw.vtx[a.own] : 0u;
-        if constexpr (H) {
-          if (a.has) {
-            const uint64_t o = sw.off[a.own];
-            if ((o & HOST_BIT) && cache_line(g, (o & OFF_MASK) + a.j) == NO_LINE) host_acc += min(4u, left);
-          }
-        }
-        uint32_t hit = 0;
+      s0 = 0;
+    } else {
+      if (si >= ns) break;
+      cur = nxs;
+      co = nxo;
+      total = min(nxl - cur.y * SWEEP_SLICE, SWEEP_SLICE);
+      si += gridDim.x * (SWEEP_THREADS / 32);
+      if (si < ns) {  // the next slice's place, while this one is walked
+        nxs = __ldcg(&c.slices[si]);
+        nxl = g.slots[nxs.x];
+        nxo = g.off[nxs.x];
+      }
+    }
+    p = 0;
+    // ---- its windows, two in flight ahead of the one tested
+    Win wa{}, wb{};
+    bool more = fetch(wa), more_b = fetch(wb);
+#pragma unroll 1
+    while (more) {
+      Win wc{};
+      const bool more_c = fetch(wc);
+      uint32_t hit = 0;
+      if (wa.left) {
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-          const uint32_t d = quad_at(a.ids, k), f = d >> shift;
-          if ((uint32_t)k < left && d != SGS_TOMB && (filter[f >> 5] >> (f & 31) & 1u)) hit |= 1u << k;
+          const uint32_t d = quad_at(wa.ids, k);
+          hit |= (__funnelshift_r(filter[d >> shift5 & mask], 0u, d >> shift) & 1u) << k;
         }
-        if (__ballot_sync(0xFFFFFFFFu, hit != 0u)) {
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            const bool h = hit >> k & 1u;
-            const uint32_t m = __ballot_sync(0xFFFFFFFFu, h);
-            if (!m) continue;
-            const uint32_t at = __popc(m & ((1u << lane) - 1u));
-            if (shift) {
-              if (h) {
-                sw.q1_dst[n1 + at] = quad_at(a.ids, k);
-                sw.q1_src[n1 + at] = u;
-                sw.q1_j[n1 + at] = a.j + k;
-              }
-              n1 += __popc(m);
-              __syncwarp();
-              if (n1 >= 32) probe();
-            } else {
-              if (h) {
-                sw.q2_dst[n2 + at] = quad_at(a.ids, k);
-                sw.q2_src[n2 + at] = u;
-                sw.q2_j[n2 + at] = a.j + k;
-              }
-              n2 += __popc(m);
-              __syncwarp();
-              if (n2 >= 32) relax();
-            }
-          }
-        }
-        a = b;
-        b = c;
-        more = more_b;
-        more_b = more_c;
+        hit &= wa.left >= 4u ? 0xFu : (1u << wa.left) - 1u;
       }
-      __syncwarp();  // the staged entries are rewritten below
-      if (sw.eb[32] >= E1 || s + 32 >= n) break;
-      s += 32;
-      __syncwarp();
+      // the hits into queue 1: all together where they fit, else quad slot by
+      // quad slot
+      const uint32_t nh = __popc(hit);
+      const uint32_t h0 = __ballot_sync(full, nh & 1u), h1 = __ballot_sync(full, nh & 2u);
+      uint32_t ks = 0;
+      const uint32_t all = __popc(h0) + 2 * __popc(h1);  // (a lane with four hits counts none here)
+      if (__any_sync(full, nh == 4u) || all > 32u) {
+        ks = __reduce_or_sync(full, hit);
+      } else if (all) {
+        uint32_t at = n1 + __popc(h0 & below) + 2 * __popc(h1 & below);
+        for (uint32_t h = hit; h; h &= h - 1) {
+          const int k = __ffs(h) - 1;
+          sw.d1[at] = quad_at(wa.ids, k);
+          sw.s1[at] = wa.u;
+          sw.j1[at] = wa.j + k;
+          ++at;
+        }
+        n1 += all;
+        __syncwarp();
+        if (n1 >= 32) drain(false);
+      }
+#pragma unroll 1
+      while (ks) {
+        const int k = __ffs(ks) - 1;
+        ks &= ks - 1;
+        const bool h = hit >> k & 1u;
+        const uint32_t m = __ballot_sync(full, h);
+        if (h) {
+          const uint32_t at = n1 + __popc(m & below);
+          sw.d1[at] = quad_at(wa.ids, k);
+          sw.s1[at] = wa.u;
+          sw.j1[at] = wa.j + k;
+        }
+        n1 += __popc(m);
+        __syncwarp();
+        if (n1 >= 32) drain(false);
+      }
+      wa = wb;
+      wb = wc;
+      more = more_b;
+      more_b = more_c;
     }
-    if (n1) probe();
-    if (n2) relax();
-    queue.flush(out, 32);
   }
-  const unsigned long long ev = warp_sum((unsigned long long)evald);
-  if (lane == 0 && ev && edge_stat) atomicAdd(edge_stat, ev);
+  if (n1 | n2) drain(true);
+  queue.template finish<SWEEP_THREADS>(out);
+  // ---- counts: one atomic per CTA and counter
+  __syncthreads();  // the filter is done with; its first words hold the sums
+  unsigned long long *sum = reinterpret_cast<unsigned long long *>(filter);
+  constexpr int NS = GMAX + 4;
+  if (threadIdx.x < NS) sum[threadIdx.x] = 0;
+  __syncthreads();
+  auto add = [&](int k, unsigned long long x) {
+    x = warp_sum(x);
+    if (lane == 0 && x) atomicAdd(&sum[k], x);
+  };
+#pragma unroll
+  for (int q = 0; q < GMAX; ++q) add(q, edges[q]);
+  add(GMAX, walked);
+  add(GMAX + 1, evald);
   if constexpr (H) {
-    const unsigned long long hs = warp_sum((unsigned long long)host_acc), ha = warp_sum(host_all);
-    if (lane == 0 && hs && host_stat) atomicAdd(host_stat, hs);
-    if (lane == 0 && g.cstat) {
-      if (ha) atomicAdd(&g.cstat[0], ha);
-      if (hs) atomicAdd(&g.cstat[1], hs);
-    }
+    add(GMAX + 2, host_acc);
+    add(GMAX + 3, host_all);
+  }
+  __syncthreads();
+  if (threadIdx.x < NS && sum[threadIdx.x]) {
+    const unsigned long long x = sum[threadIdx.x];
+    const int k = threadIdx.x;
+    if (k < GMAX) atomicAdd(&c.lane_edges[k], x);
+    else if (k == GMAX) atomicAdd(c.walked, x);
+    else if (k == GMAX + 1) atomicAdd(c.edge_stat, x);
+    else if (k == GMAX + 2) atomicAdd(c.host_stat, x);
+    if (k == GMAX + 2 && g.cstat) atomicAdd(&g.cstat[1], x);
+    if (k == GMAX + 3 && g.cstat) atomicAdd(&g.cstat[0], x);
   }
 }
 
