@@ -72,14 +72,19 @@ __global__ void k_cache_hist(const uint32_t *score, uint64_t nlines, uint32_t *h
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t c = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; c < nlines; c += stride) {
     const uint32_t s = score[c];
-    if (s >= LINE_MIN_SCORE) atomicAdd(&hist[min(s, HOT_BINS - 1)], 1u);
+    if (s < LINE_MIN_SCORE) continue;
+    // whole lines of equally hot vertices share their score, so the lanes with
+    // one bin add together (2^20 vertices: 33 -> 19 us)
+    const uint32_t b = min(s, HOT_BINS - 1), act = __activemask(), same = __match_any_sync(act, b);
+    if ((threadIdx.x & 31) == (uint32_t)__ffs(same) - 1u) atomicAdd(&hist[b], (uint32_t)__popc(same));
   }
 }
 
 // Threshold for a capacity of `cap` lines (one block of 1024 threads, 128
 // bins each, highest scores first): every line with score >= t_hi fits, and
 // `rem` more of those with score == t_tie.  When all candidates fit, t_hi is
-// the minimum score and no tie is taken.
+// the minimum score and no tie is taken.  (One block, so its latency is its time:
+// bins four at a time and the crossing found by all threads, 77 -> 21 us.)
 __global__ void __launch_bounds__(1024) k_cache_threshold(const uint32_t *hist, uint64_t cap,
                                                           unsigned long long *cc) {
   constexpr int PER = HOT_BINS / 1024;
@@ -88,7 +93,12 @@ __global__ void __launch_bounds__(1024) k_cache_threshold(const uint32_t *hist, 
   const int k = threadIdx.x;
   const uint32_t top = HOT_BINS - (uint32_t)k * PER;  // bins [top - PER, top)
   unsigned long long mine = 0;
-  for (int i = 1; i <= PER; ++i) mine += hist[top - i];
+  const uint4 *bins = reinterpret_cast<const uint4 *>(hist + (top - PER));
+#pragma unroll 8
+  for (int i = 0; i < PER / 4; ++i) {
+    const uint4 q = bins[i];
+    mine += (unsigned long long)q.x + q.y + q.z + q.w;
+  }
   unsigned long long before = 0;
   BS(tmp).ExclusiveSum(mine, before);
   if (k == 0) {
@@ -96,20 +106,27 @@ __global__ void __launch_bounds__(1024) k_cache_threshold(const uint32_t *hist, 
     cc[CC_TTIE] = 0xFFFFFFFFull;
     cc[CC_REM] = 0;
   }
+  // the thread whose bins hold the crossing hands them to the block, one bin
+  // per thread (at most one thread's do)
+  __shared__ uint32_t s_top;
+  __shared__ unsigned long long s_before;
+  if (k == 0) s_top = 0;
   __syncthreads();
-  if (before <= cap && before + mine > cap) {  // the crossing is in my bins
-    unsigned long long cum = before;
-    for (int i = 1; i <= PER; ++i) {
-      const uint32_t b = top - i;
-      const uint32_t hb = hist[b];
-      if (cum + hb > cap) {
-        cc[CC_THI] = b + 1;
-        cc[CC_TTIE] = b;
-        cc[CC_REM] = cap - cum;
-        break;
-      }
-      cum += hb;
-    }
+  if (before <= cap && before + mine > cap) {
+    s_top = top;
+    s_before = before;
+  }
+  __syncthreads();
+  if (!s_top) return;
+  const unsigned long long hb = k < PER ? hist[s_top - 1 - k] : 0u;
+  unsigned long long cum = 0;
+  BS(tmp).ExclusiveSum(hb, cum);
+  cum += s_before;
+  if (cum <= cap && cum + hb > cap) {
+    const uint32_t b = s_top - 1 - (uint32_t)k;
+    cc[CC_THI] = b + 1;
+    cc[CC_TTIE] = b;
+    cc[CC_REM] = cap - cum;
   }
 }
 

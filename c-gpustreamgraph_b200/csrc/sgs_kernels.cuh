@@ -818,7 +818,8 @@ __global__ void k_compact_blocks(GraphView g, FrontierView f, unsigned long long
         const bool keep = st.id != SGS_TOMB;
         const uint32_t b = __ballot_sync(0xFFFFFFFFu, keep);
         __syncwarp();
-        if (keep) store_slot(g, o, out + __popc(b & ((1u << lane) - 1u)), st.id, ew, st.w);
+        const uint32_t to = out + __popc(b & ((1u << lane) - 1u));
+        if (keep && to != j + lane) store_slot(g, o, to, st.id, ew, st.w);  // (not those that stay)
         out += __popc(b);
         st = nx;
         __syncwarp();
@@ -903,7 +904,10 @@ __global__ void __launch_bounds__(COMPACT_THREADS)
       uint32_t pos = out + s_warp[wid] + x - c;
 #pragma unroll
       for (int k = 0; k < 4; ++k)
-        if (keep >> k & 1u) store_slot(g, o, pos++, quad_at(ids, k), ew, quad_at(ws, k));
+        if (keep >> k & 1u) {
+          if (pos != k0 + k) store_slot(g, o, pos, quad_at(ids, k), ew, quad_at(ws, k));
+          ++pos;
+        }
       out += s_tot;
       __syncthreads();  // s_warp / s_tot are rewritten by the next tile
       ids = nids;
