@@ -1450,12 +1450,16 @@ struct sgs_engine {
       }
       return ran;
     }
+    // Vertices a thread takes at a time: four where it has more than that (two
+    // million vertices: 38 us a launch, 45 with one at a time), else one (half a
+    // million, less than two per thread: 21 us, 24 with four).
+    const auto absorb = nv > 4ull * RELAX_THREADS * grid_elem(nv) ? k_pr_absorb<4> : k_pr_absorb<1>;
     while (r < limit) {
       const uint32_t nb = std::min(rb, limit - r);
       if (ktiming) ensure_kev(2 * nb);
       for (uint32_t k = 0; k < nb; ++k) {
-        { ++n_launch; k_pr_absorb<<<grid_elem(nv), RELAX_THREADS, 0, s>>>(g, q.x.p, q.r.p, q.pv.p, cfg.pr_alpha,
-                                                           cfg.pr_tol, h, r0 + r + k); }
+        { ++n_launch; absorb<<<grid_elem(nv), RELAX_THREADS, 0, s>>>(g, q.x.p, q.r.p, q.pv.p, cfg.pr_alpha,
+                                                      cfg.pr_tol, h, r0 + r + k); }
         if (ktiming) CK(cudaEventRecord(kev[2 * k], s));
         if (pull)
           { ++n_launch; k_pull_pr<<<grid_map(), RELAX_THREADS, 0, s>>>(fin, gi, q.pv.p, q.r.p, h.step() + r0 + r + k,
@@ -1478,10 +1482,10 @@ struct sgs_engine {
       r += nb;
       // A round queued past the end takes as long as any other: 0.2 ms at 32 M
       // slots, where a host read is a fifth of that (two million vertices: 9.19
-      // -> 8.92 ms with reads every other round near the end).  At 2.4 M slots
-      // the read is the longer of the two (1.97 -> 2.10 ms), and around 15 M it
-      // makes no difference.
-      rb = r >= 16 && (pr_in & EDGE_MASK) > 1u << 24 ? 2 : 4;
+      // -> 8.92 ms with reads every other round near the end; half a million,
+      // 9.5 M slots: 26 rounds instead of 28, 3.42 -> 3.29 ms).  At 2.4 M slots
+      // the read is the longer of the two (1.97 -> 2.10 ms).
+      rb = r >= 16 && (pr_in & EDGE_MASK) > 1u << 23 ? 2 : 4;
     }
     return r;
   }

@@ -350,10 +350,9 @@ __device__ __forceinline__ StepRule pr_absorb_body(const GraphView &g, double *x
   const double back = rule.mu / alpha;  // push value * outdeg * back = mu * previous residual
   double acc = 0.0, fit = 0.0;
   // N vertices per thread and step, everything they need requested before
-  // anything is used.  Four in a launch of its own (one at a time it was bound by
-  // that latency: 45 us at two million vertices, 38 now); one in the launch that
-  // runs all rounds, whose graphs have about a vertex per thread, and where the
-  // registers of four would halve the CTAs that fit.
+  // anything is used: four where a thread has more than that, one in the
+  // launch that runs all rounds, whose graphs have about a vertex per thread, and
+  // where the registers of four would halve the CTAs that fit.
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t v0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v0 < g.nv; v0 += N * stride) {
     double rv[N], xv[N], prev[N];
@@ -404,9 +403,10 @@ __device__ __forceinline__ StepRule pr_absorb_body(const GraphView &g, double *x
   return rule;
 }
 
+template <int N>
 __global__ void k_pr_absorb(GraphView g, double *x, double *r, double *pv,
                             double alpha, double tol, StepHist h, uint32_t k) {
-  pr_absorb_body<false, 4>(g, x, r, pv, alpha, tol, h, k);
+  pr_absorb_body<false, N>(g, x, r, pv, alpha, tol, h, k);
 }
 
 // PageRank rounds r0, r0+1, ... (at most `limit`) of the pull form in one

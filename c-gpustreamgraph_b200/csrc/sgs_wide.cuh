@@ -118,7 +118,7 @@ struct WideInvalidateOp {
   }
 };
 
-// Load-balanced map for wide ops: CTAs take ranges of 2048-slot units of
+// Load-balanced map for wide ops: CTAs take ranges of units of
 // the frontier's edge space (as seg_map / group_map); entries are staged in
 // shared memory, then each warp takes 32 consecutive slots per step.  Per
 // lane counts: the CTA that holds an entry's first slot adds live[v] for

@@ -7,6 +7,7 @@
 * the batch sort at the edges of a vertex id's bits, with inserts only,
   deletes only and inserts that the same batch deletes;
 * step lengths: PageRank and PPR on graphs with and without a spectral gap;
+* PageRank's absorb with one and with four vertices per thread;
 * PPR in the looping launch and in a launch per step, with light vertices and
   pieces of either size;
 * results gathered by several threads at once.
@@ -146,6 +147,22 @@ def test_pagerank_step_lengths(shape, pull, persistent):
             u = np.repeat(np.arange(nv), np.diff(m.row).astype(np.int64))[d]
             _apply(e, m, ([1, 2, nv - 1], [nv - 1, 5 + k, 0]), (u, m.col[d]))
             check_query(q, m, sgs.W_EXPLICIT)
+
+
+@pytest.mark.parametrize("nv", [1184 * 1024, 1184 * 1024 + 1, 1184 * 2048 - 1])
+@pytest.mark.parametrize("pull", [0, 1])
+def test_pagerank_absorb_widths(nv, pull):
+    """Sizes around the one from which an absorb launch takes four vertices per
+    thread at a time (more than four for each of 1184 * 256 threads)."""
+    rng = np.random.default_rng(nv)
+    src, dst = rng.integers(0, nv, (2, 30000))
+    tail = np.arange(nv - 300, nv - 1)
+    e, m = _load(nv, np.concatenate([src, tail]), np.concatenate([dst, tail + 1]), pull=pull, persistent=6)
+    with e:
+        q = e.add_query(sgs.PR)
+        check_query(q, m, sgs.W_EXPLICIT)
+        _apply(e, m, ([nv - 1, 0], [0, nv - 1]), (tail[::7], tail[::7] + 1))
+        check_query(q, m, sgs.W_EXPLICIT)
 
 
 @pytest.mark.parametrize("K", [1, 2, 16, 17, 65])
