@@ -464,9 +464,11 @@ def engine_arm(a, R):
         hs = kd.get("max_host_slots", 0)
         if hs:
             # blocks in the pinned-host tier are read over the host link: 4-B
-            # ids (+4-B weights) per slot against the measured pinned H2D rate
+            # ids per slot (the restricted sweep reads the weights of the few
+            # edges it relaxes only; with a host policy every edge is relaxed:
+            # + 4-B weights) against the measured pinned H2D rate
             h2d = measure_h2d_gbs(dev)
-            hb = hs * 8  # explicit weights: the SSSP lane reads them
+            hb = hs * (8 if a.host_policy else 4)
             got = hb / (kd["max_ms"] * 1e-3) / 1e9
             roof["largest_launch"]["host_link"] = {
                 "host_slots": int(hs), "host_bytes": int(hb), "achieved": round(got, 1),
@@ -1016,7 +1018,7 @@ def ppr_arm(a, R):
     value = R.sum(relax) / (T_ms * 1e6)
     peak, peak_src = measured_peak_hbm()
     achieved = nbytes / (steps_ms * 1e-3) / 1e9
-    roof = {"bound": "hbm", "kernel": "k_ppr_step (+ k_ppr_finalize for hub pieces)",
+    roof = {"bound": "hbm", "kernel": "k_ppr_step",
             "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
             "frac": round(achieved / peak, 4), "peak_source": peak_src, "traffic": None,
             "launches": nsteps, "avg_launch_ms": round(steps_ms / nsteps, 4),
