@@ -1028,15 +1028,26 @@ struct sgs_engine {
   unsigned long long restrict_max() const { return std::max<uint32_t>(nv / 2, 1); }
   DBuf<uint32_t> b_coarse;  // folded reset bitmap
   DBuf<uint2> b_slices;     // k_group_sweep's slices of large blocks
+  // The sweep's buffers for the arenas as they are; without room for them (the
+  // batch is applied by then) the repair takes the full sweep.
+  bool sweep_scratch() {
+    try {
+      b_coarse.ensure(SWEEP_FILTER_BITS / 32);
+      // a block of more than SWEEP_BIG slots has at most one slice per SWEEP_BIG
+      b_slices.ensure((arena_cap[0] + arena_cap[1]) / SWEEP_BIG + 1);
+    } catch (const SgsError &) {
+      cudaGetLastError();
+      return false;
+    }
+    return true;
+  }
   void launch_sweep(Group &G, const GroupRelaxOp<GMAX> &op, unsigned long long rmax) {
     uint32_t shift = 0;
     while (((nv - 1) >> shift) >= SWEEP_FILTER_BITS) ++shift;
     const uint32_t words = ((nv - 1) >> shift) / 32 + 1;
-    if (shift) {
-      b_coarse.ensure(words);
+    if (shift)
       { ++n_launch; k_fold_bits<<<grid_elem(words), 256, 0, s>>>(G.ibits.p, (nv - 1) / 32 + 1, shift, b_coarse.p,
                                                                  words); }
-    }
     SweepCtx c{};
     c.bits = G.ibits.p;
     c.coarse = b_coarse.p;
@@ -1051,8 +1062,6 @@ struct sgs_engine {
     c.next = special(0);
     c.n_slices = special(1);
     c.walked = special(2);
-    // a block of more than SWEEP_BIG slots has at most one slice per SWEEP_BIG
-    b_slices.ensure((arena_cap[0] + arena_cap[1]) / SWEEP_BIG + 1);
     c.slices = b_slices.p;
     // a few batches per warp, but not so many that the counter sets the pace;
     // fewer than 32 vertices at a time where that would leave warps without any
@@ -2542,7 +2551,7 @@ struct sgs_engine {
       // the path is chosen on the device from the group's reset counts: the
       // dense frontier only if a lane was reset
       const unsigned long long *resets = G.resets();
-      const unsigned long long rmax = !G.wide() && gdel[i] && may_restrict() ? restrict_max() : 0;
+      const unsigned long long rmax = !G.wide() && gdel[i] && may_restrict() && sweep_scratch() ? restrict_max() : 0;
       if (!G.wide() && prep) {  // work-efficient repair: pull into the reset vertices
         bool conv = false;
         grounds[i] = pull_repair(G, gdel[i] != 0, ni, explicit_w);
