@@ -138,6 +138,11 @@ struct Group {
   uint64_t used = 0;            // lanes in use
   uint32_t algo_packed = 0;     // narrow: 8 bits per lane
   uint64_t sssp = 0, cc = 0;    // lanes per algorithm (both widths)
+  // A snapshot began and has not repaired this group to the end: it runs, or it
+  // ended with an error (a round limit, a user algorithm, no memory).  Edges
+  // outside what the next one resets and inserts may be unrelaxed then, so its
+  // repair re-pushes from every reached vertex.
+  bool unrepaired = false;
   uint64_t inval[WLANES] = {};  // resets per lane in the last deletion phase
   DBuf<uint32_t> ibits;         // narrow: bitmap of vertices reset in the last deletion phase
   DBuf<unsigned long long> wreset;  // wide: per vertex, the lanes reset in the last deletion phase
@@ -2111,7 +2116,10 @@ struct sgs_engine {
       if (queries[i]->id == qid) {
         sync();
         Query &q = *queries[i];
-        if (q.grp) q.grp->used &= ~(1ull << q.lane);
+        if (q.grp) {
+          q.grp->used &= ~(1ull << q.lane);
+          if (!q.grp->used) q.grp->unrepaired = false;  // the next lanes start from scratch
+        }
         if (job.q == &q) job.q = nullptr;
         if (q.algo == SGS_PR && cfg.pr_warm) {  // keep its vector for the next start
           std::swap(pr_warm.p, q.x.p);
@@ -2412,6 +2420,22 @@ struct sgs_engine {
     bool any_narrow = false;
     for (size_t i = 0; i < ng; ++i) any_narrow |= groups[i]->used && !groups[i]->wide();
     const bool prep = (cfg.repair & 1u) && any_narrow && nd && ensure_in();
+    // what the phases need is allocated before any of them changes a value
+    const size_t iwords = (size_t)nv / 32 + 1;
+    const bool nmarks = prep || may_restrict();  // narrow groups note the vertices they reset
+    for (size_t i = 0; i < ng; ++i) {
+      Group &G = *groups[i];
+      if (!G.used) continue;
+      if (G.wide()) G.wreset.ensure(nv);
+      else if (nd && nmarks) G.ibits.ensure(iwords);
+    }
+    if (nd && any_narrow && may_restrict()) (void)sweep_scratch();
+    std::vector<char> whole(ng, 0);  // the snapshot before was not repaired to the end
+    for (size_t i = 0; i < ng; ++i)
+      if (groups[i]->used) {
+        whole[i] = groups[i]->unrepaired;
+        groups[i]->unrepaired = true;
+      }
 
     // ---- PR cancel over the old out-lists of touched sources
     if (any_pr) {
@@ -2433,15 +2457,11 @@ struct sgs_engine {
       gdel[i] = 1;
       CK(cudaEventRecord(gev[4 * i], s));
       reset_phase();
-      if (G.wide()) {  // the lanes this invalidation resets, per vertex
-        G.wreset.ensure(nv);
+      if (G.wide())  // the lanes this invalidation resets, per vertex
         CK(cudaMemsetAsync(G.wreset.p, 0, sizeof(unsigned long long) * nv, s));
-      } else if (prep || may_restrict()) {  // bitmap of the vertices this invalidation resets
-        const size_t nw = (size_t)nv / 32 + 1;
-        G.ibits.ensure(nw);
-        CK(cudaMemsetAsync(G.ibits.p, 0, sizeof(uint32_t) * nw, s));
-      }
-      uint32_t *nmark = prep || may_restrict() ? G.ibits.p : nullptr;
+      else if (nmarks)  // bitmap of the vertices this invalidation resets
+        CK(cudaMemsetAsync(G.ibits.p, 0, sizeof(uint32_t) * iwords, s));
+      uint32_t *nmark = nmarks ? G.ibits.p : nullptr;
       bool conv = false;
       if (G.wide()) {
         { ++n_launch; k_wide_seed_deleted<<<grid_elem(nd), 256, 0, s>>>(
@@ -2538,24 +2558,25 @@ struct sgs_engine {
     // rounds are unrestricted, so the fixed point is the same.  (A narrow group
     // does so unless much was reset, see RepairMode.)  Without invalidation
     // only the inserted edges are relaxed.  Then rounds to convergence.
+    // All of that rests on a group whose last snapshot was repaired to the end;
+    // one whose was not (`whole`) takes the reference's re-push, whatever was
+    // reset.
     for (size_t i = 0; i < ng; ++i) {
       Group &G = *groups[i];
       if (!G.used) continue;
       Range rg("sgs:repair");
       CK(cudaEventRecord(gev[4 * i + 2], s));
       reset_phase();
-      if (G.wide() && !gdel[i]) {  // no deletion phase ran: no lane was reset
-        G.wreset.ensure(nv);
+      if (G.wide() && !gdel[i])  // no deletion phase ran: no lane was reset
         CK(cudaMemsetAsync(G.wreset.p, 0, sizeof(unsigned long long) * nv, s));
-      }
       // the path is chosen on the device from the group's reset counts: the
       // dense frontier only if a lane was reset
-      const unsigned long long *resets = G.resets();
-      const unsigned long long rmax = !G.wide() && gdel[i] && may_restrict() && sweep_scratch() ? restrict_max() : 0;
-      if (!G.wide() && prep) {  // work-efficient repair: pull into the reset vertices
-        bool conv = false;
+      const unsigned long long *resets = whole[i] ? nullptr : G.resets();
+      const unsigned long long rmax =
+          !G.wide() && gdel[i] && !whole[i] && may_restrict() && sweep_scratch() ? restrict_max() : 0;
+      if (!G.wide() && prep && !whole[i]) {  // work-efficient repair: pull into the reset vertices
         grounds[i] = pull_repair(G, gdel[i] != 0, ni, explicit_w);
-        (void)conv;
+        G.unrepaired = false;
         CK(cudaEventRecord(gev[4 * i + 3], s));
         CK(cudaMemcpyAsync(G.dstat.p + 2 * WLANES, b_lane.p, sizeof(unsigned long long) * WLANES,
                            cudaMemcpyDeviceToDevice, s));
@@ -2567,7 +2588,7 @@ struct sgs_engine {
       else
         { ++n_launch; k_group_dense<GMAX><<<grid_elem(nv), 256, 0, s>>>(g, G.val.p, (uint32_t)G.used, G.algo(),
                                                             gm[0].p, fview(0, cnt.p), resets, rmax); }
-      if (ni && !G.wide())  // narrow, the sweep does not cover them
+      if (ni && !G.wide() && !whole[i])  // narrow, the sweep does not cover them
         { ++n_launch; k_group_relax_inserted<GMAX><<<grid_elem(ni), 256, 0, s>>>(
             g, G.st.p, G.val.p, (uint32_t)G.used, G.algo(), b_ikept.p, explicit_w ? b_iw_kept.p : nullptr,
             b_nkept.p, gm[0].p, fview(0, cnt.p), b_lane.p, resets, rmax, gm[1].p, fview(1, cnt.p + 1)); }
@@ -2581,9 +2602,11 @@ struct sgs_engine {
             b_nkept.p, wm[1].p, fview(1, cnt.p + 1), b_lane.p); }
       };
       bool conv = false;
-      grounds[i] = G.wide() ? group_relax(G, conv, "sgs:sweep", G.wreset.p, ni ? &ins_after0 : nullptr)
-                            : group_relax(G, conv, "sgs:sweep", nullptr, nullptr, rmax);
+      grounds[i] = G.wide() && !whole[i]
+                       ? group_relax(G, conv, "sgs:sweep", G.wreset.p, ni ? &ins_after0 : nullptr)
+                       : group_relax(G, conv, "sgs:sweep", nullptr, nullptr, rmax);
       if (!conv) fail(SGS_ERR_NOCONV, "round limit reached before convergence");
+      G.unrepaired = false;
       CK(cudaEventRecord(gev[4 * i + 3], s));
       CK(cudaMemcpyAsync(G.dstat.p + 2 * WLANES, b_lane.p, sizeof(unsigned long long) * WLANES,
                          cudaMemcpyDeviceToDevice, s));
