@@ -25,7 +25,9 @@
 // (R-MAT hubs reach 10^5 in-edges) is cut into pieces of that many edges whose
 // partial sums go to a scratch row each and are added up, in piece order, by
 // the warp that finishes the vertex's last piece -- so no warp walks more than
-// `piece` edges of a vertex and the sums are deterministic.  Inside a warp, LPE
+// `piece` edges of a vertex and a step's result does not depend on the order of
+// its items.  Only the norms do, by their last bits, which the step lengths
+// leave out (sgs_steplen.cuh).  Inside a warp, LPE
 // lanes cover the columns of one neighbour row (CPL columns per lane) and
 // 32/LPE neighbours are gathered at once, four deep, so one neighbour row is
 // one coalesced read for any K.

@@ -72,7 +72,12 @@ __device__ __forceinline__ StepRule step_rule(const StepHist &h, uint32_t k, dou
     return s;
   }
   if (w1 != 1.0 || w2 != 1.0 || !(b > 0.0)) return s;
-  const double mu = a / b;
+  // mu to 16 bits: the norms' sums are added in any order, and their last bits
+  // must not reach the state, so that equal calls give equal bits.  (The rest of
+  // mu is far below the fit.  A sum's order would have to move a / b across the
+  // middle of two such values, 1 in 10^11.)
+  const double mu =
+      __longlong_as_double((__double_as_longlong(a / b) + (1ll << 35)) & ~((1ll << 36) - 1));
   // (below 0.3 a plain step is as good; M's spectral radius is at most alpha)
   if (!(mu > 0.3 && mu <= alpha * 1.0001)) return s;
   // no long step near the end: a step queued past it must not raise d

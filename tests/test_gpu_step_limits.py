@@ -1,0 +1,119 @@
+"""PPR's and PageRank's iterations:
+
+* two runs give the same bits;
+* PPR's launch per step: the adjoint and the edge gradient, all column
+  layouts, and more steps than the step history holds, in both launch forms.
+"""
+import numpy as np
+import pytest
+import scipy.sparse as sp
+
+import oracle as O
+import sgs
+
+pytestmark = pytest.mark.gpu
+
+ALPHA = 0.85
+
+
+def _p(nv, row, col, w):
+    """Row-normalised transition matrix, sparse."""
+    src = np.repeat(np.arange(nv), np.diff(row).astype(np.int64))
+    s = np.bincount(src, weights=w, minlength=nv)
+    return sp.csr_matrix((w / s[src], (src, col.astype(np.int64))), shape=(nv, nv))
+
+
+def _inputs(nv, ne, K, seed):
+    rng = np.random.default_rng(seed)
+    T = np.zeros((nv, K))
+    T[rng.integers(0, nv, 32), np.arange(32) % K] = 1.0
+    return np.exp(rng.uniform(-1, 1, ne)), T, rng.standard_normal((nv, K))
+
+
+@pytest.mark.parametrize("scale,K", [(12, 8), (13, 40), (17, 8), (17, 40)])
+def test_ppr_repeats_itself(scale, K):
+    """Equal bits from run to run (torch's gradcheck asks for them), many CTAs,
+    both launch forms."""
+    nv, row, col = O.rmat_csr(scale, 16, 7)
+    w, T, G = _inputs(nv, len(col), K, scale)
+    with sgs.Ppr(nv, row, col) as g:
+        X = g.forward(w, T)
+        gw, gT = g.backward(w, X, G)
+        for _ in range(6):
+            assert np.array_equal(g.forward(w, T), X)
+            gw2, gT2 = g.backward(w, X, G)
+            assert np.array_equal(gT2, gT) and np.array_equal(gw2, gw)
+
+
+@pytest.mark.parametrize("K", [3, 8, 16, 20, 40])
+def test_ppr_launch_per_step_adjoint(K):
+    """Scale 17, pieces of 128 edges: 64 MB a step or more from K = 3 on."""
+    nv, row, col = O.rmat_csr(17, 20, 5)
+    w, T, G = _inputs(nv, len(col), K, K)
+    P = _p(nv, row, col, w)
+    tol = 1e-10
+    with sgs.Ppr(nv, row, col) as g:
+        X = g.forward(w, T, tol=tol)
+        gw, gT = g.backward(w, X, G, tol=tol)
+    # one more step changes the states by less than tol, and the rounding of
+    # a row's sum
+    d = (1 - ALPHA) * T + ALPHA * (P.T @ X) - X
+    assert np.abs(d).sum() <= tol + 64 * 1e-15 * np.abs(X).sum()
+    Y = gT / (1 - ALPHA)
+    d = G + ALPHA * (P @ Y) - Y
+    assert np.abs(d).sum() <= tol + 64 * 1e-15 * np.abs(Y).sum()
+    # gw_uv = X[u] . (alpha Y[v] - Y[u] + G[u]) / s_u: edges at random and all of
+    # the largest row's
+    src = np.repeat(np.arange(nv), np.diff(row).astype(np.int64))
+    s = np.bincount(src, weights=w, minlength=nv)
+    hub = int(np.argmax(np.diff(row)))
+    pick = np.concatenate([np.random.default_rng(1).integers(0, len(col), 5000),
+                           np.arange(row[hub], row[hub + 1]).astype(np.int64)])
+    u, v = src[pick], col[pick].astype(np.int64)
+    ref = np.einsum("ek,ek->e", X[u], ALPHA * Y[v] - Y[u] + G[u]) / s[u]
+    mag = np.einsum("ek,ek->e", np.abs(X[u]), np.abs(Y[v]) + np.abs(Y[u]) + np.abs(G[u])) / s[u]
+    assert np.all(np.abs(gw[pick] - ref) <= 1e-13 * mag)
+
+
+@pytest.mark.parametrize("nv", [600, 1 << 19])
+def test_ppr_more_steps_than_the_history(nv):
+    """A cycle at alpha = 0.98 takes some 1,300 steps, all plain; its solution
+    is a geometric series."""
+    alpha, K = 0.98, 8
+    a = np.arange(nv)
+    row, col = O.csr_from_edges(nv, a.astype(np.uint32), ((a + 1) % nv).astype(np.uint32))
+    T = np.zeros((nv, K))
+    T[np.arange(K) * 7, np.arange(K)] = 1.0
+    tol = 1e-11
+    with sgs.Ppr(nv, row, col) as g:
+        X = g.forward(np.ones(nv), T, alpha=alpha, tol=tol)
+        assert g.last_iters > 1024
+    ref = np.zeros_like(T)
+    for k in range(K):
+        ref[(np.arange(nv) + 7 * k) % nv, k] = (1 - alpha) * alpha ** np.arange(nv) / (1 - alpha**nv)
+    assert np.abs(X - ref).sum() <= alpha / (1 - alpha) * tol
+
+
+@pytest.mark.parametrize("nv0", [1 << 10, 1 << 17])
+def test_ppr_long_steps_and_more_steps_than_the_history(nv0):
+    """An R-MAT part, whose Perron vector one long step removes, beside a
+    cycle with a thousandth of the mass, which keeps the rest of the steps
+    plain and takes more of them than the history holds."""
+    alpha, K, ring = 0.98, 4, 3000
+    n0, row, col = O.rmat_csr(int(np.log2(nv0)), 16, 3)
+    src = np.repeat(np.arange(n0), np.diff(row).astype(np.int64))
+    a = np.arange(ring)
+    nv = n0 + ring
+    row, col = O.csr_from_edges(nv, np.concatenate([src, n0 + a]).astype(np.uint32),
+                                np.concatenate([col.astype(np.int64), n0 + (a + 1) % ring]).astype(np.uint32))
+    w = np.ones(len(col))
+    T = np.zeros((nv, K))
+    T[:n0] = 1.0
+    T[n0 + np.arange(K), np.arange(K)] = 1e-3 * n0
+    tol = 1e-9
+    with sgs.Ppr(nv, row, col) as g:
+        X = g.forward(w, T, alpha=alpha, tol=tol)
+        assert g.last_iters > 512
+    P = _p(nv, row, col, w)
+    d = (1 - alpha) * T + alpha * (P.T @ X) - X
+    assert np.abs(d).sum() <= tol + 64 * 1e-15 * np.abs(X).sum()
