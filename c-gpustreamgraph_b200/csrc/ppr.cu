@@ -980,6 +980,9 @@ struct sgs_ppr {
         st.steps_ms += ms;
       }
       const sgs::StepHist h{hd.data(), nb};
+      // Vertices without edges have their say in step 0 only; one that is not a
+      // number there never comes to rest.
+      const bool lost = it == 0 && !(h.l1()[0] == h.l1()[0]);
       bool end = false;
       for (uint32_t b = 0; b < n; ++b) {
         end = end || ppr_ends(h.step()[b], h.l1()[b], prev, (int)h.state()[b], tol, alpha, under);
@@ -990,6 +993,7 @@ struct sgs_ppr {
       k += n;
       st.iters = (int32_t)it;
       cur = k % 2 ? b1 : b0;
+      if (lost) return -1;
       if (end) return (int)it;
     }
     return below ? (int)it : -1;

@@ -1,5 +1,6 @@
 """PPR's and PageRank's iterations:
 
+* input that is not a number is refused wherever it stands;
 * two runs give the same bits;
 * PPR's launch per step: the adjoint and the edge gradient, all column
   layouts, and more steps than the step history holds, in both launch forms.
@@ -14,6 +15,7 @@ import sgs
 pytestmark = pytest.mark.gpu
 
 ALPHA = 0.85
+NOCONV = -5
 
 
 def _p(nv, row, col, w):
@@ -28,6 +30,32 @@ def _inputs(nv, ne, K, seed):
     T = np.zeros((nv, K))
     T[rng.integers(0, nv, 32), np.arange(32) % K] = 1.0
     return np.exp(rng.uniform(-1, 1, ne)), T, rng.standard_normal((nv, K))
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+@pytest.mark.parametrize("nv", [50, 1 << 19])
+def test_ppr_refuses_what_is_not_a_number(nv, bad):
+    """Also at a vertex without any edge, in a launch per step (2^19 vertices,
+    K = 8: 109 MB a step) and in the looping launch."""
+    K = 8
+    a = np.arange(40)
+    row, col = O.csr_from_edges(nv, np.concatenate([a, a]).astype(np.uint32),
+                                np.concatenate([(a + 1) % 41, (a * 7 + 3) % 41]).astype(np.uint32))
+    w = np.ones(len(col))
+    T = np.zeros((nv, K))
+    T[:41] = 1.0
+    with sgs.Ppr(nv, row, col) as g:
+        X = g.forward(w, T)
+        for v in (5, 45):
+            T2 = T.copy()
+            T2[v, 3] = bad
+            with pytest.raises(sgs.SgsError) as err:
+                g.forward(w, T2, max_iter=300)
+            assert err.value.code == NOCONV
+            with pytest.raises(sgs.SgsError) as err:
+                g.backward(w, X, T2, max_iter=300)
+            assert err.value.code == NOCONV
+        assert np.array_equal(g.forward(w, T), X)
 
 
 @pytest.mark.parametrize("scale,K", [(12, 8), (13, 40), (17, 8), (17, 40)])
