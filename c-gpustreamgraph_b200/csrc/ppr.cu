@@ -930,21 +930,36 @@ struct sgs_ppr {
     return std::min(32u, std::max(per, neg));
   }
 
-  // The fixed point of x = c B + alpha A x from c B in b0, b1 as the second
-  // buffer: steps until one changes the state by less than tol in L1
-  // (ppr_ends).  `cur` = the buffer with the result.  Returns the steps run, -1
-  // when max_iter did not suffice.
+  // The fixed point of x = c B + alpha A x from c B, in the buffers b0 and b1:
+  // steps until one changes the state by less than tol in L1 (ppr_ends).
+  // `cur` = the buffer with the result.  Returns the steps run, -1 when max_iter
+  // did not suffice: plain steps alone are tried too before that is said, since
+  // a long step may fall on the last one permitted, or not keep its promise.
   int iterate(const Adj &adj, const double *p, uint32_t K, double alpha, double c, const double *B, double *b0,
               double *b1, double tol, uint32_t max_iter, double *&cur) {
+    bool longs = false;
+    st.iters = 0;
+    const int it = run_steps(adj, p, K, alpha, c, B, b0, b1, tol, max_iter, false, cur, longs);
+    return it >= 0 || !longs ? it : run_steps(adj, p, K, alpha, c, B, b0, b1, tol, max_iter, true, cur, longs);
+  }
+  int run_steps(const Adj &adj, const double *p, uint32_t K, double alpha, double c, const double *B, double *b0,
+                double *b1, double tol, uint32_t max_iter, bool plain, double *&cur, bool &longs) {
     const double bytes = step_bytes(K);
     const bool loop = bytes < LOOP_BYTES;
     StepArgs a{adj.ptr, adj.nbr, p, nv, adj.pv.p, adj.poff.p, adj.npieces, piece, K, alpha, c, B, part.p, done(), next(),
                items_per_warp(loop, K), sgs::StepHist{work.p, HIST}, tol};
     const size_t row = sizeof(double);
     PCK(cudaMemsetAsync(work.p, 0, row * sgs::StepHist::FIELDS * HIST + sizeof(uint32_t) * HIST, s));
+    { ++n_launch; k_scale<<<grid(), THREADS, 0, s>>>(B, c, (uint64_t)nv * K, b0); }
+    cur = b0;
     uint32_t it = 0, k = 0, under = 0;
-    bool below = false;  // the last plain step was below tol
-    double prev = 0.0;   // its change
+    if (plain) {  // after a failed long step none follows
+      static const double failed = sgs::ST_FAILED;
+      k = 2;
+      PCK(cudaMemcpyAsync(sgs::StepHist{work.p, HIST}.state() + 1, &failed, row, cudaMemcpyHostToDevice, s));
+    }
+    bool below = false;  // a plain step was below tol, and no long one came after it
+    double prev = 0.0;   // the last plain step's change
     std::vector<double> hd;
     while (it < max_iter) {
       if (k == HIST) {
@@ -987,11 +1002,12 @@ struct sgs_ppr {
       for (uint32_t b = 0; b < n; ++b) {
         end = end || ppr_ends(h.step()[b], h.l1()[b], prev, (int)h.state()[b], tol, alpha, under);
         prev = h.step()[b] == 1.0 ? h.l1()[b] : 0.0;
-        below = h.step()[b] == 1.0 && h.l1()[b] < tol;
+        below = h.step()[b] == 1.0 && (below || h.l1()[b] < tol);
+        longs = longs || h.step()[b] != 1.0;
       }
       it += n;
       k += n;
-      st.iters = (int32_t)it;
+      st.iters += (int32_t)n;
       cur = k % 2 ? b1 : b0;
       if (lost) return -1;
       if (end) return (int)it;
@@ -1007,7 +1023,6 @@ struct sgs_ppr {
     xn.ensure(n);
     part.ensure((uint64_t)std::max(in.npieces, out.npieces) * K);
     PCK(cudaMemcpyAsync(t.p, T, sizeof(double) * n, kin(mem), s));
-    { ++n_launch; k_scale<<<grid(), THREADS, 0, s>>>(t.p, 1.0 - alpha, n, x.p); }
     double *cur = x.p;
     const int it = iterate(in, pc.p, K, alpha, 1.0 - alpha, t.p, x.p, xn.p, tol, max_iter, cur);
     PCK(cudaMemcpyAsync(X, cur, sizeof(double) * n, kout(mem), s));
@@ -1025,7 +1040,6 @@ struct sgs_ppr {
     part.ensure((uint64_t)std::max(in.npieces, out.npieces) * K);
     PCK(cudaMemcpyAsync(x.p, X, sizeof(double) * n, kin(mem), s));
     PCK(cudaMemcpyAsync(g.p, G, sizeof(double) * n, kin(mem), s));
-    PCK(cudaMemcpyAsync(y.p, g.p, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
     double *cur = y.p;
     const int it = iterate(out, pr.p, K, alpha, 1.0, g.p, y.p, yn.p, tol, max_iter, cur);
     if (it < 0) return it;

@@ -536,10 +536,15 @@ SGS_API int sgs_serve(sgs_engine *e, const sgs_request *req, uint32_t n,
  * pass has no counterpart in the reference.  Layout: X, T, G, gT are
  * vertex-major [nv][K] doubles; w and gw are per edge in the CSR order of
  * the prepared graph (sgs_ppr_export).  `mem` says where all arrays live.
- * Convergence: Jacobi steps until the L1 change summed over all nv*K entries
- * is below tol; SGS_ERR_NOCONV after max_iter steps.  *iters (optional) gets
- * the steps taken.  Weights must be positive and finite (else
- * SGS_ERR_INVALID).  A handle is not thread-safe. */
+ * Convergence: steps until the L1 change of a Jacobi step, summed over all
+ * nv*K entries, is below tol.  Some steps are longer than a Jacobi step; with
+ * steps to spare the end is a sixteenth of tol (a 256th after a long step),
+ * so that the error left is no larger than that of plain steps some way past
+ * tol.  SGS_ERR_NOCONV when neither these nor plain steps alone are below tol
+ * within max_iter steps, and for input that is not a number.  *iters (optional)
+ * gets the steps taken.  Weights must be positive and finite (else
+ * SGS_ERR_INVALID).  Equal calls give equal bits.  A handle is not
+ * thread-safe. */
 typedef struct sgs_ppr sgs_ppr;
 SGS_API int sgs_ppr_create_csr(int device, uint32_t nv, const uint64_t *row,
                                const uint32_t *col, int mem, sgs_ppr **out);
@@ -561,16 +566,16 @@ SGS_API int sgs_ppr_backward(sgs_ppr *p, const double *w, const double *X,
                              double *gT, int *iters, int mem);
 /* Device timing of the last forward/backward call (CUDA events on the
  * handle's stream).  steps_ms is filled only while sgs_ppr_timing is on
- * (events around every Jacobi step).  bytes_alg_step = algorithmic bytes of
+ * (events around every batch of steps).  bytes_alg_step = algorithmic bytes of
  * one step: per edge the 4-B neighbour id, 8-B probability and 8K-B neighbour
  * row; per vertex 16 B of offsets and 24K B of state (B, x read; out written). */
 typedef struct sgs_ppr_stats {
-  int32_t iters;             /* Jacobi steps of the last call              */
+  int32_t iters;             /* steps of the last call, of both tries      */
   uint32_t pieces_in;        /* work pieces of hub vertices, CSC and CSR   */
   uint32_t pieces_out;
   uint32_t reserved;
   double ms;                 /* device time of the whole last call         */
-  double steps_ms;           /* device time of its Jacobi steps            */
+  double steps_ms;           /* device time of its steps                   */
   double bytes_alg_step;
   uint64_t kernel_launches;  /* own kernel launches since the handle was made */
 } sgs_ppr_stats;

@@ -1,5 +1,7 @@
-"""PPR's and PageRank's iterations:
+"""PPR's iterations at their limits:
 
+* the documented end (one step's L1 change below the tolerance) is found within the steps that plain iteration
+  needs, also when one of them is a long step;
 * input that is not a number is refused wherever it stands;
 * two runs give the same bits;
 * PPR's launch per step: the adjoint and the edge gradient, all column
@@ -10,7 +12,9 @@ import pytest
 import scipy.sparse as sp
 
 import oracle as O
+import ppr_dense as D
 import sgs
+import step_rule as S
 
 pytestmark = pytest.mark.gpu
 
@@ -30,6 +34,33 @@ def _inputs(nv, ne, K, seed):
     T = np.zeros((nv, K))
     T[rng.integers(0, nv, 32), np.arange(32) % K] = 1.0
     return np.exp(rng.uniform(-1, 1, ne)), T, rng.standard_normal((nv, K))
+
+
+@pytest.mark.parametrize("scale,K", [(8, 1), (10, 3), (12, 20)])
+def test_ppr_limit_where_plain_steps_suffice(scale, K):
+    """Plain steps are below tol at step k, where the rule takes a long one."""
+    nv, row, col = O.rmat_csr(scale, 16, 2)
+    w, T, G = _inputs(nv, len(col), K, scale)
+    P = _p(nv, row, col, w)
+    with sgs.Ppr(nv, row, col) as g:
+        k, n = S.first_long_step(P.T.tocsr(), 1 - ALPHA, T, ALPHA)
+        assert k is not None and n[k] < n[k - 1]
+        tol = 0.5 * (n[k] + n[k - 1])
+        X = g.forward(w, T, tol=tol, max_iter=k + 1)
+        assert g.last_iters <= k + 1
+        # the L1 error is at most alpha / (1 - alpha) times the last change
+        assert np.abs(X - D.ppr_dense(nv, row, col, w, T)).sum() <= ALPHA / (1 - ALPHA) * tol
+        with pytest.raises(sgs.SgsError) as err:  # one step fewer never was enough
+            g.forward(w, T, tol=0.5 * n[-1] * 1e-3, max_iter=3)
+        assert err.value.code == NOCONV
+        # the adjoint; a positive G has a Perron part, so a long step comes
+        k, n = S.first_long_step(P, 1.0, np.abs(G), ALPHA)
+        assert k is not None and n[k] < n[k - 1]
+        tol = 0.5 * (n[k] + n[k - 1])
+        _, gT = g.backward(w, X, np.abs(G), tol=tol, max_iter=k + 1)
+        Y = np.linalg.solve(np.eye(nv) - ALPHA * P.toarray(), np.abs(G))
+        # row sums of alpha P are at most alpha: the same bound for the maximum
+        assert np.abs(gT / (1 - ALPHA) - Y).max() <= ALPHA / (1 - ALPHA) * tol
 
 
 @pytest.mark.parametrize("bad", [np.nan, np.inf])
