@@ -1395,17 +1395,43 @@ struct sgs_engine {
     unsigned long long pr_in = 0;
     CK(cudaMemcpyAsync(&pr_in, cnt.p, sizeof(pr_in), cudaMemcpyDeviceToHost, s));
     sync();
-    return pr_steps(q, fview(0, cnt.p), fview(1, cnt.p + 1), pull, StepHist{prh.p, maxr + 2}, 0, maxr, edge_stat,
-                    pr_in, conv, last_l1);
+    const StepHist h{prh.p, maxr + 2};
+    PrEnd end;
+    uint32_t r = pr_steps(q, fview(0, cnt.p), fview(1, cnt.p + 1), pull, h, 0, maxr, edge_stat, pr_in, end);
+    if (pr_tries_plain(end, h))
+      r += pr_steps(q, fview(0, cnt.p), fview(1, cnt.p + 1), pull, h, 1, maxr, edge_stat, pr_in, end);
+    conv = end.conv;
+    last_l1 = end.l1;
+    return r;
+  }
+
+  // How a run of PageRank rounds ended: its last round's norm and length, and
+  // whether any round was a long one.
+  struct PrEnd {
+    bool conv = false, longs = false;
+    double l1 = 0, w = 0;
+  };
+  // At the round limit: a plain round below pr_tol is an end (the sixteenth that
+  // rounds after a long one go on to is for rounds to spare); without one, true
+  // when long rounds were taken.  The history is then set up for up to as many
+  // rounds again from its entry 1, all plain: the last round permitted may have
+  // been a long one, or one may not have kept its promise, where plain rounds
+  // alone would have ended within the limit.
+  bool pr_tries_plain(PrEnd &end, const StepHist &h) {
+    if (end.w == 1.0 && end.l1 < cfg.pr_tol) end.conv = true;
+    if (end.conv || !end.longs) return false;
+    static const double failed = ST_FAILED;
+    CK(cudaMemsetAsync(h.p, 0, sizeof(double) * StepHist::FIELDS * h.n, s));
+    CK(cudaMemcpyAsync(h.state(), &failed, sizeof(failed), cudaMemcpyHostToDevice, s));
+    return true;
   }
 
   // Rounds r0, r0+1, ... (at most `limit`) over a prebuilt dense frontier
   // `fin` of the store the sweep reads (in-edge store when `pull`); per-round
-  // history in h[r].  Returns the rounds run; conv when a round's L1 falls
+  // history in h[r].  Returns the rounds run; end.conv when a round's L1 falls
   // below the tolerance (pr_tol; less after a long round, sgs_steplen.cuh).
   uint32_t pr_steps(Query &q, FrontierView fin, FrontierView fout, bool pull, StepHist h, uint32_t r0,
-                    uint32_t limit, unsigned long long *edge_stat, unsigned long long pr_in, bool &conv,
-                    double &last_l1) {
+                    uint32_t limit, unsigned long long *edge_stat, unsigned long long pr_in, PrEnd &end) {
     const GraphView g = view();
     const GraphView gi = pull ? in_view() : g;
     // one strided copy reads the fields of a batch of rounds
@@ -1415,13 +1441,18 @@ struct sgs_engine {
       CK(cudaMemcpy2DAsync(hl.data(), n * sizeof(double), h.p + first, h.n * sizeof(double), n * sizeof(double),
                            StepHist::FIELDS, cudaMemcpyDeviceToHost, s));
     };
+    // notes round k of the n read; true when it ends the iteration
     auto ends = [&](uint32_t k, uint32_t n) {
       const StepHist f{hl.data(), n};
-      return StepRule::ends(f.step()[k], f.l1()[k], (int)f.state()[k], cfg.pr_tol);
+      end.l1 = f.l1()[k];
+      end.w = f.step()[k];
+      end.longs |= end.w != 1.0;
+      end.conv = StepRule::ends(end.w, end.l1, (int)f.state()[k], cfg.pr_tol);
+      return end.conv;
     };
     uint32_t r = 0, rb = 8;
-    conv = false;
-    last_l1 = 0;
+    end.conv = false;
+    end.l1 = end.w = 0;
     PrPushOp op{g, q.pv.p, q.r.p};
     const unsigned long long pr_inst = (pr_in & EDGE_MASK);
     // all rounds in one cooperative launch (k_pr_rounds, one host read) when
@@ -1431,7 +1462,7 @@ struct sgs_engine {
     const void *fn = (const void *)k_pr_rounds;
     const uint64_t units = ((pr_in & EDGE_MASK) + CTA_SLOTS - 1) / CTA_SLOTS;
     if (pull && (cfg.persistent & 8u) && limit && units <= (uint64_t)coop_grid(fn)) {
-        GraphView ga = g, gb = gi;
+      GraphView ga = g, gb = gi;
       FrontierView f = fin;
       double *x = q.x.p, *rp = q.r.p, *pv = q.pv.p;
       StepHist hh = h;
@@ -1453,10 +1484,7 @@ struct sgs_engine {
       read_ctl();
       const uint32_t ran = (uint32_t)h_ctl[CTL_ROUNDS];
       if (ran > limit) fail(SGS_ERR_CUDA, "PageRank round kernel returned a bad round count");
-      if (ran) {
-        last_l1 = hl[ran - 1];
-        conv = ends(ran - 1, limit);
-      }
+      for (uint32_t k = 0; k < ran; ++k) ends(k, limit);
       if (ktiming && ran) {
         float ms = 0;
         CK(cudaEventElapsedTime(&ms, kev[0], kev[1]));
@@ -1489,10 +1517,8 @@ struct sgs_engine {
         for (uint32_t k = 0; k < nb; ++k)
           account(pull ? SGS_K_PR_PULL : SGS_K_PR_PUSH, pr_in, pr_inst, 4.0, 16.0, kev[2 * k],
                   kev[2 * k + 1]);
-      for (uint32_t k = 0; k < nb; ++k) {
-        last_l1 = hl[k];
-        if (ends(k, nb)) { conv = true; return r + k + 1; }
-      }
+      for (uint32_t k = 0; k < nb; ++k)
+        if (ends(k, nb)) return r + k + 1;
       r += nb;
       // A round queued past the end takes as long as any other: 0.2 ms at 32 M
       // slots, where a host read is a fifth of that (two million vertices: 9.19
@@ -1512,6 +1538,8 @@ struct sgs_engine {
     Query *q = nullptr;
     bool pull = false;
     uint32_t r = 0;
+    uint32_t before = 0;  // rounds of the first try, once plain rounds alone are tried
+    bool longs = false;
     Frontier f;
     uint32_t ucap = 0;
     DBuf<unsigned long long> c;  // [0] frontier counter, [1] output counter, [2] edge count
@@ -1574,7 +1602,8 @@ struct sgs_engine {
     CK(cudaEventRecord(ev_q.b, s));
     sync();
     CK(cudaEventElapsedTime(&job.ms, ev_q.a, ev_q.b));
-    job.r = 0;
+    job.r = job.before = 0;
+    job.longs = false;
     job.q = q.get();
     q->stats = sgs_query_stats{};
     const int id = q->id;
@@ -1593,28 +1622,36 @@ struct sgs_engine {
       job.stale = false;
     }
     Query &q = *job.q;
-    const uint32_t lim = std::min(rounds, cfg.max_rounds - job.r);
-    bool conv = false;
-    double l1v = 0;
+    const StepHist h{job.prh.p, cfg.max_rounds + 2};
+    // (the second try starts at entry 1 of the history)
+    const uint32_t last = cfg.max_rounds + (job.before ? 1 : 0), lim = std::min(rounds, last - job.r);
+    PrEnd end;
     CK(cudaEventRecord(ev_q.a, s));
-    const uint32_t ran = pr_steps(q, job_view(0), job_view(1), job.pull,
-                                  StepHist{job.prh.p, cfg.max_rounds + 2}, job.r, lim, job.c.p + 2,
-                                  job.pr_in, conv, l1v);
+    const uint32_t ran = pr_steps(q, job_view(0), job_view(1), job.pull, h, job.r, lim, job.c.p + 2, job.pr_in, end);
     CK(cudaEventRecord(ev_q.b, s));
     sync();
     float ms = 0;
     CK(cudaEventElapsedTime(&ms, ev_q.a, ev_q.b));
     job.ms += ms;
     job.r += ran;
-    q.stats.pr_residual_l1 = l1v;
-    if (!conv && job.r < cfg.max_rounds) return false;
+    job.longs |= end.longs;
+    q.stats.pr_residual_l1 = end.l1;
+    if (!end.conv && job.r < last) return false;
+    if (!end.conv) {
+      end.longs = job.longs && !job.before;
+      if (pr_tries_plain(end, h)) {
+        job.before = job.r;
+        job.r = 1;
+        return false;
+      }
+    }
     unsigned long long e = 0;
     CK(cudaMemcpyAsync(&e, job.c.p + 2, sizeof(e), cudaMemcpyDeviceToHost, s));
     sync();
     q.stats.edges_traversed = e;
     q.stats.edges_total += e;
-    q.stats.rounds = job.r;
-    q.stats.converged = conv ? 1 : 0;
+    q.stats.rounds = job.before ? job.before + job.r - 1 : job.r;
+    q.stats.converged = end.conv ? 1 : 0;
     q.stats.ms = job.ms;
     job.q = nullptr;
     return true;

@@ -100,9 +100,11 @@ typedef struct sgs_config {
                              Segments beyond it live in pinned host memory
                              and are read over the host link              */
   int weight_mode;        /* SGS_W_*                                        */
-  uint32_t max_rounds;    /* round limit per convergence (reference: 1000) */
+  uint32_t max_rounds;    /* round limit per convergence (reference: 1000);
+                             PageRank: again, all plain, if long rounds failed */
   double pr_alpha;        /* damping, 0.85 (hybrid_pr_common.h:39)         */
-  double pr_tol;          /* stop when sum|residual| < pr_tol              */
+  double pr_tol;          /* stop when sum|residual| < pr_tol (rounds to spare
+                             go on to a sixteenth of it after a long round) */
   uint32_t slack_div;     /* per-block slack: cap = deg + deg/slack_div + 2 */
   double arena_headroom;  /* extra arena fraction for relocated blocks    */
   uint32_t group_size;    /* BFS/SSSP/CC queries relaxed together per edge

@@ -1,6 +1,7 @@
-"""PPR's iterations at their limits:
+"""PPR's and PageRank's iterations at their limits:
 
-* the documented end (one step's L1 change below the tolerance) is found within the steps that plain iteration
+* the documented end (one step's L1 change below the tolerance, or the sum of
+  the residuals for PageRank) is found within the steps that plain iteration
   needs, also when one of them is a long step;
 * input that is not a number is refused wherever it stands;
 * two runs give the same bits;
@@ -61,6 +62,30 @@ def test_ppr_limit_where_plain_steps_suffice(scale, K):
         Y = np.linalg.solve(np.eye(nv) - ALPHA * P.toarray(), np.abs(G))
         # row sums of alpha P are at most alpha: the same bound for the maximum
         assert np.abs(gT / (1 - ALPHA) - Y).max() <= ALPHA / (1 - ALPHA) * tol
+
+
+@pytest.mark.parametrize("pull,persistent", [(1, 14), (1, 6), (0, 14)])
+@pytest.mark.parametrize("scale", [8, 11])
+def test_pagerank_limit_where_plain_rounds_suffice(scale, pull, persistent):
+    nv, row, col = O.rmat_csr(scale, 16, 2)
+    P = _p(nv, row, col, np.ones(len(col)))
+    k, n = S.first_long_round(P.T.tocsr(), nv, ALPHA, np.diff(row) > 0)
+    assert k is not None and n[k] < n[k - 1]
+    tol = 0.5 * (n[k] + n[k - 1])
+    ref = O.pagerank(nv, row, col)
+    with sgs.Engine(max_rounds=k + 1, pr_tol=tol, pull=pull, persistent=persistent) as e:
+        e.load_csr(nv, row, col, O.weights(nv, row, col, 1, 0))
+        q = e.add_query(sgs.PR)
+        assert q.stats()["converged"] == 1 and q.stats()["pr_residual_l1"] < tol
+        # what is left after the residual r is at most |r| / (1 - alpha)
+        assert np.abs(q.value() - ref).sum() <= ALPHA / (1 - ALPHA) * tol
+        e.remove_query(q)
+    with sgs.Engine(max_rounds=k + 1, pr_tol=tol, pull=pull, persistent=persistent, pr_warm=0) as e:
+        e.load_csr(nv, row, col, O.weights(nv, row, col, 1, 0))
+        out = np.empty(nv)
+        done = e.serve([{"kind": "query", "algo": sgs.PR, "value_out": out}], realtime=False)
+        assert done[0]["status"] == 0
+        assert np.abs(out - ref).sum() <= ALPHA / (1 - ALPHA) * tol
 
 
 @pytest.mark.parametrize("bad", [np.nan, np.inf])
