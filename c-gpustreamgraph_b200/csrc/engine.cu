@@ -453,6 +453,11 @@ struct sgs_engine {
     CK(cudaSetDevice(dev));
     CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
     CK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+    // A kernel's limit is one for all engines of the process, so it is the same
+    // from each: the largest that launch_sweep asks for.
+    for (const void *k : {(const void *)k_group_sweep<true>, (const void *)k_group_sweep<false>})
+      CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)sweep_smem(SWEEP_FILTER_BITS / 32)));
     const size_t nr = (size_t)cfg.max_rounds + 2;
     phase_len = nr + kSpecial + 2 * nr + 2 * WLANES + 1;
     phase.ensure(phase_len);
@@ -1079,7 +1084,6 @@ struct sgs_engine {
     c.host_stat = hstat.p;
     const void *k = host_tier() ? (const void *)k_group_sweep<true> : (const void *)k_group_sweep<false>;
     const size_t smem = sweep_smem(kept);
-    CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     FrontierView out = fview(1, cnt.p + 1);
     GroupRelaxOp<GMAX> o = op;
     void *args[] = {&out, &o, &c};

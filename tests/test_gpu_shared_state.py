@@ -1,0 +1,72 @@
+"""What engines and calls share: launch attributes of a kernel between engines
+of different sizes, and a PageRank job between two updates."""
+import threading
+
+import numpy as np
+import pytest
+
+import oracle as O
+import sgs
+from test_gpu_parity import Mirror, check_query
+
+pytestmark = pytest.mark.gpu
+
+
+def test_engines_of_two_sizes_in_two_threads():
+    """Their sweeps ask for different amounts of shared memory."""
+    errors = []
+
+    def work(scale):
+        try:
+            nv, row, col = O.rmat_csr(scale, 8, scale)
+            w = O.weights(nv, row, col, 1, 0)
+            src = np.repeat(np.arange(nv), np.diff(row).astype(np.int64)).astype(np.uint32)
+            with sgs.Engine() as e:
+                e.load_csr(nv, row, col, w)
+                qs = e.add_queries([(sgs.SSSP, 0), (sgs.BFS, 0), (sgs.CC, 0)])
+                for k in range(400):  # the same edges out and in again
+                    s = slice(37 * (k // 2), 37 * (k // 2) + 37)
+                    none = np.empty(0, np.uint32)
+                    if k % 2 == 0:
+                        e.apply_batch(none, none, none, src[s], col[s])
+                    else:
+                        e.apply_batch(src[s], col[s], w[s], none, none)
+                m = Mirror(nv, row, col, w)
+                for q in qs:
+                    check_query(q, m, sgs.W_EXPLICIT)
+        except Exception as ex:  # reported by the main thread
+            errors.append(ex)
+
+    ts = [threading.Thread(target=work, args=(s,)) for s in (10, 20)]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    assert not errors, errors
+
+
+def test_pagerank_job_amended_between_long_steps():
+    """Updates arrive while a served PageRank job runs: its residual changes
+    between two rounds, and the result is the fixed point of the graph it ended on."""
+    nv, row, col = O.rmat_csr(13, 16, 8)
+    w = O.weights(nv, row, col, 1, 0)
+    m = Mirror(nv, row, col, w)
+    graphs = [(row, col)]  # by the number of updates applied
+    with sgs.Engine() as e:
+        e.load_csr(nv, row, col, w)
+        i_s, i_d, d_s, d_d = O.gen_updates(nv, row, col, 3, 4000, 4000)
+        reqs = [{"kind": "query", "algo": sgs.PR, "value_out": np.empty(nv)}]
+        for k in range(8):
+            s = slice(500 * k, 500 * k + 500)
+            iw = O.weights_pairs(1, i_s[s], i_d[s])
+            reqs.append({"kind": "update", "ins_src": i_s[s], "ins_dst": i_d[s], "ins_w": iw,
+                         "del_src": d_s[s], "del_dst": d_d[s]})
+            m.apply(i_s[s], i_d[s], iw, d_s[s], d_d[s])
+            graphs.append((m.row, m.col))
+        done = e.serve(reqs, realtime=False)
+        assert all(c["status"] == 0 for c in done)
+        assert done[0]["version"] >= 2
+        ref = O.pagerank(nv, *graphs[done[0]["version"]])
+        assert np.max(np.abs(reqs[0]["value_out"] - ref)) <= 1e-6
+        q = e.add_query(sgs.SSSP, 0)
+        check_query(q, m, sgs.W_EXPLICIT)
