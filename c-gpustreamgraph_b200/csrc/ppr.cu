@@ -26,8 +26,7 @@
 // partial sums go to a scratch row each and are added up, in piece order, by
 // the warp that finishes the vertex's last piece -- so no warp walks more than
 // `piece` edges of a vertex and a step's result does not depend on the order of
-// its items.  Only the norms do, by their last bits, which the step lengths
-// leave out (sgs_steplen.cuh).  Inside a warp, LPE
+// its items, nor does a step's length (sgs_steplen.cuh).  Inside a warp, LPE
 // lanes cover the columns of one neighbour row (CPL columns per lane) and
 // 32/LPE neighbours are gathered at once, four deep, so one neighbour row is
 // one coalesced read for any K.
@@ -342,15 +341,15 @@ struct StepArgs {
   double tol;
 };
 
-// The new state of one entry; |d| and the fit (sgs_steplen.cuh) into dsum,
-// fsum.  out still holds the state before x, so x - out is the previous d.
+// The new state of one entry; |d|, so that the order of the additions does not
+// show, and the fit (sgs_steplen.cuh) into dsum, fsum.  out still holds the state before x, so x - out is the previous d.
 template <bool Coh>
 __device__ __forceinline__ void finish_entry(const StepArgs &a, const sgs::StepRule &rule, uint64_t o, double sum,
                                              const double *x, double *out, double &dsum, double &fsum) {
   const double nx = a.c * __ldg(a.B + o) + a.alpha * sum;
   const double xo = ld_row<Coh>(x + o);
   const double d = nx - xo;
-  dsum += fabs(d);
+  dsum += sgs::exact_term(fabs(d), rule.unit);
   if (rule.mu > 0.0) fsum += fabs(d - rule.mu * (xo - __ldcg(out + o)));
   out[o] = rule.w == 1.0 ? nx : fma(rule.w, d, xo);
 }
@@ -531,7 +530,19 @@ __device__ __forceinline__ void ppr_step_body(const StepArgs &a, const sgs::Step
 template <int LPE, int CPL>
 __global__ void __launch_bounds__(THREADS, LPE == 32 ? 4 : 5)
     k_ppr_step(StepArgs a, const double *__restrict__ x, double *out, uint32_t k, bool first) {
-  ppr_step_body<LPE, CPL, false>(a, sgs::step_rule(a.h, k, a.alpha, a.tol * sgs::LONG_TOL), x, out, k, first);
+  // The history is a few words, for which every warp would queue at one place in
+  // L2: one thread of the CTA reads it where the registers are short of keeping
+  // the rule too (2^18 vertices, K = 16: 140 -> 133 us); with narrower rows it
+  // arrives while the warps gather (K = 1: 49 us, 52 with one thread).
+  if constexpr (LPE >= 8) {
+    __shared__ sgs::StepRule s_rule;
+    if (threadIdx.x == 0) s_rule = sgs::step_rule<true>(a.h, k, a.alpha, a.tol * sgs::LONG_TOL);
+    __syncthreads();
+    ppr_step_body<LPE, CPL, false>(a, s_rule, x, out, k, first);
+  } else {
+    ppr_step_body<LPE, CPL, false>(a, sgs::step_rule<true>(a.h, k, a.alpha, a.tol * sgs::LONG_TOL), x, out, k,
+                                   first);
+  }
 }
 
 // The end of the iteration, the same on both sides: a plain step below the
@@ -554,20 +565,45 @@ __host__ __device__ inline bool ppr_ends(double w, double l1, double prev, int s
 // step takes about as long as a launch: forward and backward on 4,096 vertices
 // with K = 8 took 8.0 ms with two launches per step and 0.84 per step, 2.3 with
 // this loop and the long steps.
-template <int LPE, int CPL>
+template <int LPE, int CPL, bool One>
 __global__ void __launch_bounds__(THREADS, 4)
     k_ppr_steps(StepArgs a, double *x0, double *x1, uint32_t k0, uint32_t k1, uint32_t under, bool first,
                 uint32_t *ran) {
   cooperative_groups::grid_group grid = cooperative_groups::this_grid();
+  // One: as above, one thread of the CTA reads the history, a step's end and the
+  // next one's rule at once.
+  __shared__ sgs::StepRule s_rule;
+  __shared__ bool s_end;
+  auto rule_of = [&](uint32_t k) { return sgs::step_rule<true>(a.h, k, a.alpha, a.tol * sgs::LONG_TOL); };
+  auto ends = [&](const sgs::StepRule &rule, uint32_t k) {
+    const double norm = __ldcg(a.h.l1() + k), norm1 = __ldcg(a.h.l1() + (k ? k - 1 : 0));
+    const double w1 = __ldcg(a.h.step() + (k ? k - 1 : 0));
+    return ppr_ends(rule.w, norm + sgs::exact_slack(rule.unit, (double)a.nv * a.K), k && w1 == 1.0 ? norm1 : 0.0,
+                    rule.state, a.tol, a.alpha, under);
+  };
   uint32_t k = k0;
-  while (k < k1) {
-    const sgs::StepRule rule = sgs::step_rule(a.h, k, a.alpha, a.tol * sgs::LONG_TOL);
-    ppr_step_body<LPE, CPL, true>(a, rule, k % 2 ? x1 : x0, k % 2 ? x0 : x1, k, first && k == k0);
-    grid.sync();
-    const double l1 = __ldcg(a.h.l1() + k);
-    const double prev = k && __ldcg(a.h.step() + k - 1) == 1.0 ? __ldcg(a.h.l1() + k - 1) : 0.0;
-    ++k;
-    if (ppr_ends(rule.w, l1, prev, rule.state, a.tol, a.alpha, under)) break;
+  if constexpr (One) {
+    if (threadIdx.x == 0) s_rule = rule_of(k);
+    __syncthreads();
+    while (k < k1) {
+      ppr_step_body<LPE, CPL, true>(a, s_rule, k % 2 ? x1 : x0, k % 2 ? x0 : x1, k, first && k == k0);
+      grid.sync();
+      if (threadIdx.x == 0) {
+        const sgs::StepRule done = s_rule;
+        s_rule = rule_of(k + 1);
+        s_end = ends(done, k);
+      }
+      __syncthreads();
+      ++k;
+      if (s_end) break;
+    }
+  } else {
+    while (k < k1) {
+      const sgs::StepRule rule = rule_of(k);
+      ppr_step_body<LPE, CPL, true>(a, rule, k % 2 ? x1 : x0, k % 2 ? x0 : x1, k, first && k == k0);
+      grid.sync();
+      if (ends(rule, k++)) break;
+    }
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) *ran = k - k0;
 }
@@ -887,14 +923,24 @@ struct sgs_ppr {
   void launch(const StepArgs &a, bool loop, double *b0, double *b1, uint32_t k, uint32_t k1, uint32_t under,
               bool first) {
     if (loop) {
-      const void *f = (const void *)k_ppr_steps<LPE, CPL>;
+      const void *f = (const void *)k_ppr_steps<LPE, CPL, false>;
       StepArgs aa = a;
       uint32_t *r = ran();
       void *args[] = {&aa, &b0, &b1, &k, &k1, &under, &first, &r};
       // no more CTAs than items (idle ones only lengthen the barriers)
       const uint64_t items = a.npieces + ((uint64_t)a.nv + a.per - 1) / a.per;
       const uint64_t need = (items + THREADS / 32 - 1) / (THREADS / 32);
-      const uint32_t gr = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(rgrid(f), need));
+      uint32_t gr = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(rgrid(f), need));
+      // More than two CTAs per SM would queue for the history's words (4,096
+      // vertices, K = 32, 512 CTAs: 8.3 us a step with a thread each reading
+      // them, 12.0 with all; K = 8, 128 CTAs: 8.5 against 6.5).  Not with 16 lanes
+      // per row, where R-MAT graphs' hubs wait for the later start (2^14 vertices,
+      // K = 16, forward and backward: 1.66 against 1.57 ms).
+      if constexpr (LPE != 16)
+        if (gr > 2u * (uint32_t)nsm) {
+          f = (const void *)k_ppr_steps<LPE, CPL, true>;
+          gr = std::min(gr, rgrid(f));
+        }
       ++n_launch;
       PCK(cudaLaunchCooperativeKernel(f, gr, THREADS, args, 0, s));
       return;
@@ -960,6 +1006,8 @@ struct sgs_ppr {
     }
     bool below = false;  // a plain step was below tol, and no long one came after it
     double prev = 0.0;   // the last plain step's change
+    double norm = 0.0;   // the last step's, whatever its length
+    const double entries = (double)nv * K;
     std::vector<double> hd;
     while (it < max_iter) {
       if (k == HIST) {
@@ -1000,9 +1048,11 @@ struct sgs_ppr {
       const bool lost = it == 0 && !(h.l1()[0] == h.l1()[0]);
       bool end = false;
       for (uint32_t b = 0; b < n; ++b) {
-        end = end || ppr_ends(h.step()[b], h.l1()[b], prev, (int)h.state()[b], tol, alpha, under);
-        prev = h.step()[b] == 1.0 ? h.l1()[b] : 0.0;
-        below = h.step()[b] == 1.0 && (below || h.l1()[b] < tol);
+        const double l1 = h.l1()[b] + sgs::exact_slack(sgs::exact_unit(norm), entries);
+        end = end || ppr_ends(h.step()[b], l1, prev, (int)h.state()[b], tol, alpha, under);
+        norm = h.l1()[b];
+        prev = h.step()[b] == 1.0 ? norm : 0.0;
+        below = h.step()[b] == 1.0 && (below || l1 < tol);
         longs = longs || h.step()[b] != 1.0;
       }
       it += n;

@@ -28,6 +28,7 @@
 // approach and the steps that were queued past its end.
 #pragma once
 #include <cstdint>
+#include <cstring>
 #include <cuda_runtime.h>
 
 namespace sgs {
@@ -51,33 +52,60 @@ struct StepHist {
   __host__ __device__ double *state() const { return p + 4 * (size_t)n; }
 };
 
+// A sum whose value must not depend on the order of its additions is made of
+// exact_terms: x >= 0 rounded to a multiple of 2^-47 of the last step's norm (of
+// its power of two, the unit), of which up to 2^53 add up without rounding.  The
+// last bit of a number of 48 units' size is such a multiple.  (Unit 0: no norm to
+// go by, x is left as it is.)  The sum of n terms is off by exact_slack at most.
+__host__ __device__ __forceinline__ double exact_unit(double norm) {
+  unsigned long long b;
+  memcpy(&b, &norm, sizeof(b));
+  b &= 0x7FF0000000000000ull;
+  double u;
+  memcpy(&u, &b, sizeof(u));
+  return u < 1e300 ? u : 0.0;
+}
+__device__ __forceinline__ double exact_term(double x, double unit) {
+  const double c = 48.0 * unit;
+  return __dsub_rn(__dadd_rn(x, c), c);
+}
+__host__ __device__ __forceinline__ double exact_slack(double unit, double n) {
+  return n * (unit * (1.0 / (double)(1ull << 48)));
+}
+
 struct StepRule {
   double w;   // step length
   double mu;  // > 0: take the fit with it
   int state;
+  double unit = 0.0;  // exact_term's
   // whether a step with norm l1 under this rule ends the iteration
   __host__ __device__ static bool ends(double w, double l1, int state, double tol) {
     return w == 1.0 && l1 < (state == ST_LONG ? tol * LONG_TOL : tol);
   }
 };
 
+// Exact: the norms are sums of exact_terms, so that a step's length, and with it
+// the state, is the same to the last bit in equal calls.  (The fit is not: it is
+// compared with a threshold only.)
+template <bool Exact = false>
 __device__ __forceinline__ StepRule step_rule(const StepHist &h, uint32_t k, double alpha, double tol) {
-  StepRule s{1.0, 0.0, k ? (int)__ldcg(h.state() + k - 1) : ST_PLAIN};
+  if (k == 0) return StepRule{1.0, 0.0, ST_PLAIN};
+  // (all that may be needed at once: one round trip)
+  const uint32_t k1 = k - 1, k2 = k > 1 ? k - 2 : 0, k3 = k > 2 ? k - 3 : 0;
+  const double a = __ldcg(h.l1() + k1), b = __ldcg(h.l1() + k2), c = Exact ? __ldcg(h.l1() + k3) : 0.0;
+  const double w1 = __ldcg(h.step() + k1), w2 = __ldcg(h.step() + k2);
+  const double f = __ldcg(h.fit() + k1), mu0 = __ldcg(h.mu() + k1);
+  StepRule s{1.0, 0.0, (int)__ldcg(h.state() + k1)};
+  if (Exact) s.unit = exact_unit(a);
   if (k < 2 || s.state == ST_FAILED) return s;
-  const double a = __ldcg(h.l1() + k - 1), b = __ldcg(h.l1() + k - 2);
-  const double w1 = __ldcg(h.step() + k - 1), w2 = __ldcg(h.step() + k - 2);
-  const double f = __ldcg(h.fit() + k - 1), mu0 = __ldcg(h.mu() + k - 1);
   if (w2 > 1.0 && !(a < 0.5 * b)) {
     s.state = ST_FAILED;
     return s;
   }
   if (w1 != 1.0 || w2 != 1.0 || !(b > 0.0)) return s;
-  // mu to 16 bits: the norms' sums are added in any order, and their last bits
-  // must not reach the state, so that equal calls give equal bits.  (The rest of
-  // mu is far below the fit.  A sum's order would have to move a / b across the
-  // middle of two such values, 1 in 10^11.)
-  const double mu =
-      __longlong_as_double((__double_as_longlong(a / b) + (1ll << 35)) & ~((1ll << 36) - 1));
+  // (sums of a step whose norm grew more than eightfold may have been rounded)
+  if (Exact && k > 2 && !(b <= 8.0 * c)) return s;
+  const double mu = a / b;
   // (below 0.3 a plain step is as good; M's spectral radius is at most alpha)
   if (!(mu > 0.3 && mu <= alpha * 1.0001)) return s;
   // no long step near the end: a step queued past it must not raise d
