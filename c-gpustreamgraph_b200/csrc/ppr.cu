@@ -448,9 +448,18 @@ __device__ __forceinline__ void ppr_step_body(const StepArgs &a, const sgs::Step
       }
       uint32_t todo = __ballot_sync(full, deg > 0 && deg <= a.piece);
       if constexpr (LPE < 32) {
-        // up to 32 edges: a lane group per vertex, NEG vertices at a time
+        // up to 32 edges: a lane group per vertex, NEG vertices at a time;
         uint32_t lo = __ballot_sync(full, deg > 0 && deg <= 32);
         todo &= ~lo;
+        // so with heavier ones if that takes fewer loads in a row than the warp on
+        // one after the other (20,000 vertices, a fifth of them with 64 in-edges,
+        // K = 1: 36 -> 19 us a step)
+        constexpr uint32_t D = Coh ? 8 : 4;
+        const uint32_t many = __popc(todo);
+        if ((many + NEG - 1) / NEG * ((a.piece + D - 1) / D) < many * ((a.piece + NEG * D - 1) / (NEG * D))) {
+          lo |= todo;
+          todo = 0;
+        }
         while (lo) {
           const int my = eg < __popc(lo) ? (int)__fns(lo, 0, eg + 1) : -1;
           const uint64_t b = __shfl_sync(full, rb, my & 31), e = __shfl_sync(full, re, my & 31);
@@ -530,19 +539,7 @@ __device__ __forceinline__ void ppr_step_body(const StepArgs &a, const sgs::Step
 template <int LPE, int CPL>
 __global__ void __launch_bounds__(THREADS, LPE == 32 ? 4 : 5)
     k_ppr_step(StepArgs a, const double *__restrict__ x, double *out, uint32_t k, bool first) {
-  // The history is a few words, for which every warp would queue at one place in
-  // L2: one thread of the CTA reads it where the registers are short of keeping
-  // the rule too (2^18 vertices, K = 16: 140 -> 133 us); with narrower rows it
-  // arrives while the warps gather (K = 1: 49 us, 52 with one thread).
-  if constexpr (LPE >= 8) {
-    __shared__ sgs::StepRule s_rule;
-    if (threadIdx.x == 0) s_rule = sgs::step_rule<true>(a.h, k, a.alpha, a.tol * sgs::LONG_TOL);
-    __syncthreads();
-    ppr_step_body<LPE, CPL, false>(a, s_rule, x, out, k, first);
-  } else {
-    ppr_step_body<LPE, CPL, false>(a, sgs::step_rule<true>(a.h, k, a.alpha, a.tol * sgs::LONG_TOL), x, out, k,
-                                   first);
-  }
+  ppr_step_body<LPE, CPL, false>(a, sgs::step_rule<true>(a.h, k, a.alpha, a.tol * sgs::LONG_TOL), x, out, k, first);
 }
 
 // The end of the iteration, the same on both sides: a plain step below the
@@ -570,8 +567,8 @@ __global__ void __launch_bounds__(THREADS, 4)
     k_ppr_steps(StepArgs a, double *x0, double *x1, uint32_t k0, uint32_t k1, uint32_t under, bool first,
                 uint32_t *ran) {
   cooperative_groups::grid_group grid = cooperative_groups::this_grid();
-  // One: as above, one thread of the CTA reads the history, a step's end and the
-  // next one's rule at once.
+  // One: one thread of the CTA reads the history, a step's end and the next one's
+  // rule at once.
   __shared__ sgs::StepRule s_rule;
   __shared__ bool s_end;
   auto rule_of = [&](uint32_t k) { return sgs::step_rule<true>(a.h, k, a.alpha, a.tol * sgs::LONG_TOL); };
@@ -968,11 +965,12 @@ struct sgs_ppr {
   }
 
   // Light vertices per item: 8 from the counter (32 left the last items to few
-  // warps), in the loop as many as give every warp one item; at least what the
+  // warps; 4 with two lane groups, which walk most vertices one by one: 2^18
+  // vertices, K = 16: 5.0 -> 4.5 ms), in the loop as many as give every warp one item; at least what the
   // lane groups of a narrow form take at a time, at most 32.
   uint32_t items_per_warp(bool loop, uint32_t K) const {
     const uint32_t warps = (uint32_t)nsm * 32, neg = 32u / (uint32_t)lanes_per_edge(std::min(K, 32u));
-    uint32_t per = loop ? (nv + warps - 1) / warps : 8u;
+    uint32_t per = loop ? (nv + warps - 1) / warps : neg == 2 ? 4u : 8u;
     return std::min(32u, std::max(per, neg));
   }
 

@@ -201,3 +201,30 @@ def test_ppr_long_steps_and_more_steps_than_the_history(nv0):
     P = _p(nv, row, col, w)
     d = (1 - alpha) * T + alpha * (P.T @ X) - X
     assert np.abs(d).sum() <= tol + 64 * 1e-15 * np.abs(X).sum()
+
+
+@pytest.mark.parametrize("K", [1, 2, 3, 8, 16])
+@pytest.mark.parametrize("degree", [32, 33, 60, 64])
+def test_ppr_items_of_heavier_vertices(degree, K):
+    """Whole items of vertices at and above the 32 edges that a lane group takes
+    by itself, and the odd one among lighter ones, up to the piece size of small
+    graphs (64)."""
+    n = 300
+    rng = np.random.default_rng(degree)
+    src = [np.argsort(rng.random((n, n)), axis=1)[:, :degree]]  # in-neighbours of [0, n)
+    dst = [np.repeat(np.arange(n), degree).reshape(n, degree)]
+    light = n + np.arange(700)  # lighter ones, every 50th as heavy
+    deg = np.where(light % 50 == 0, degree, 3)
+    src.append(rng.integers(0, n + 700, deg.sum()))
+    dst.append(np.repeat(light, deg))
+    nv = n + 700
+    row, col = O.csr_from_edges(nv, np.concatenate([a.ravel() for a in src]).astype(np.uint32),
+                                np.concatenate([a.ravel() for a in dst]).astype(np.uint32))
+    w, T, G = _inputs(nv, len(col), K, degree)
+    tol = 1e-13 * nv * K
+    with sgs.Ppr(nv, row, col) as g:
+        X = g.forward(w, T, tol=tol)
+        gw, gT = g.backward(w, X, G, tol=tol)
+    assert np.abs(X - D.ppr_dense(nv, row, col, w, T)).sum() <= ALPHA / (1 - ALPHA) * tol
+    Y = np.linalg.solve(np.eye(nv) - ALPHA * _p(nv, row, col, w).toarray(), G)
+    assert np.abs(gT / (1 - ALPHA) - Y).max() <= ALPHA / (1 - ALPHA) * tol + 1e-13 * np.abs(Y).max()
