@@ -1529,7 +1529,12 @@ struct sgs_engine {
       // -> 8.92 ms with reads every other round near the end; half a million,
       // 9.5 M slots: 26 rounds instead of 28, 3.42 -> 3.29 ms).  At 2.4 M slots
       // the read is the longer of the two (1.97 -> 2.10 ms).
+      // A run without long rounds goes on for a hundred or more, each a little
+      // below the one before: as many are queued as that takes to the end (163,840
+      // vertices, 160 rounds: 7.9 -> 7.4 ms).
       rb = r >= 16 && (pr_in & EDGE_MASK) > 1u << 23 ? 2 : 4;
+      if (!end.longs && r >= 32 && nb > 1)
+        rb = StepRule::steps_left(hl[nb - 1], hl[nb - 2], cfg.pr_tol, rb, 32);
     }
     return r;
   }

@@ -1007,6 +1007,8 @@ struct sgs_ppr {
     double norm = 0.0;   // the last step's, whatever its length
     const double entries = (double)nv * K;
     std::vector<double> hd;
+    const uint32_t few = bytes > 256e6 ? 2 : 4;
+    uint32_t ahead = few;
     while (it < max_iter) {
       if (k == HIST) {
         // the rule looks back four entries: move them to the front.  (An even
@@ -1022,9 +1024,10 @@ struct sgs_ppr {
       }
       // A launch per step: 8 steps before the first host read (never fewer are
       // needed), then 2 to 4 -- a read costs about 10 us, steps past the end
-      // their own time.
+      // their own time -- or, when no long step was taken by step 32, as many as
+      // the end is away.
       uint32_t nb = std::min<uint32_t>(HIST - k, max_iter - it);
-      if (!loop) nb = std::min<uint32_t>(nb, it == 0 ? 8 : bytes > 256e6 ? 2 : 4);
+      if (!loop) nb = std::min<uint32_t>(nb, it == 0 ? 8 : ahead);
       if (timing) PCK(cudaEventRecord(ev[0], s));
       steps(a, loop, b0, b1, k, k + nb, under, it == 0);
       if (timing) PCK(cudaEventRecord(ev[1], s));
@@ -1057,6 +1060,10 @@ struct sgs_ppr {
       k += n;
       st.iters += (int32_t)n;
       cur = k % 2 ? b1 : b0;
+      if (!longs && it >= 32 && n > 1)
+        ahead = sgs::StepRule::steps_left(h.l1()[n - 1], h.l1()[n - 2], tol * sgs::LONG_TOL, few, 32);
+      else
+        ahead = few;
       if (lost) return -1;
       if (end) return (int)it;
     }

@@ -27,6 +27,7 @@
 // L1 norm instead of 7e-7 in those runs, is then no larger than that of the slow
 // approach and the steps that were queued past its end.
 #pragma once
+#include <cmath>
 #include <cstdint>
 #include <cstring>
 #include <cuda_runtime.h>
@@ -74,6 +75,13 @@ __host__ __device__ __forceinline__ double exact_slack(double unit, double n) {
 }
 
 struct StepRule {
+  // The plain steps that norms falling as the last two did take to tol, in
+  // [least, most] (host: how many to queue before the next look).
+  static uint32_t steps_left(double l1, double before, double tol, uint32_t least, uint32_t most) {
+    if (!(l1 > tol && l1 < before && tol > 0.0)) return least;
+    const double n = std::ceil(std::log(l1 / tol) / std::log(before / l1));
+    return n > least ? (n < most ? (uint32_t)n : most) : least;
+  }
   double w;   // step length
   double mu;  // > 0: take the fit with it
   int state;
