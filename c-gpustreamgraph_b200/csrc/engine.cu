@@ -740,6 +740,7 @@ struct sgs_engine {
     in_release();
     in_failed = false;
     pr_warm.release();
+    drop_gather();
     if (sc) CK(cudaStreamSynchronize(sc));
     stg_head = stg_count = 0;  // staged batches belonged to the old graph
     est = sgs_engine_stats{};
@@ -1846,7 +1847,7 @@ struct sgs_engine {
               break;
             } catch (const SgsError &f) {
               // out of memory: drop pooled empty groups (not pending here) once
-              bool freed = false;
+              bool freed = f.code == SGS_ERR_OOM && attempt == 0 && drop_gather();
               if (f.code == SGS_ERR_OOM && attempt == 0)
                 for (size_t j = groups.size(); j-- > 0;) {
                   bool pend = false;
@@ -2814,9 +2815,12 @@ struct sgs_engine {
     // keeps, then one copy to the caller.  (A buffer allocated and freed per
     // call cost 0.6 ms in the two calls, each of which waits for the device; a
     // snapshot with 64 results on 262,144 vertices went from 52 to 3.8 ms, one
-    // with 3 on a million from 4.0 to 1.2 ms.)  The lock is for callers that
-    // read several queries from several threads.
+    // with 3 on a million from 4.0 to 1.2 ms.)  Up to 64 MB; the copy of a larger
+    // result takes many times as long, and its buffer goes when it is done.  The
+    // lock is for callers that read several queries from several threads.
     std::lock_guard<std::mutex> lock(gather_mu);
+    DBuf<uint32_t> large;
+    DBuf<uint32_t> &b_gather = nv <= KEPT_GATHER ? kept_gather : large;
     b_gather.ensure(nv);
     const bool parent = field == SGS_FIELD_PARENT;
     const uint32_t *val = parent ? nullptr : q.grp->val.p;
@@ -2828,8 +2832,15 @@ struct sgs_engine {
     CK(cudaMemcpyAsync(out, b_gather.p, sizeof(uint32_t) * nv, kind, s));
     sync();
   }
-  DBuf<uint32_t> b_gather;
+  static constexpr uint32_t KEPT_GATHER = 1u << 24;
+  DBuf<uint32_t> kept_gather;
   std::mutex gather_mu;
+  bool drop_gather() {
+    std::lock_guard<std::mutex> lock(gather_mu);
+    const bool any = kept_gather.p != nullptr;
+    kept_gather.release();
+    return any;
+  }
 
   void summary(Query &q, uint64_t out[4]) {
     CK(cudaMemsetAsync(b_stat.p, 0, sizeof(unsigned long long) * 4, s));

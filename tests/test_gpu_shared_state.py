@@ -1,5 +1,6 @@
 """What engines and calls share: launch attributes of a kernel between engines
-of different sizes, and a PageRank job between two updates."""
+of different sizes, the buffer that results are gathered through, and a
+PageRank job between two updates."""
 import threading
 
 import numpy as np
@@ -43,6 +44,26 @@ def test_engines_of_two_sizes_in_two_threads():
     for t in ts:
         t.join()
     assert not errors, errors
+
+
+def test_gather_gives_memory_back():
+    """A large graph's gather keeps no buffer of its size."""
+    import torch
+
+    def free():
+        torch.cuda.synchronize()
+        return torch.cuda.mem_get_info()[0]
+
+    nv = 1 << 25  # 128 MB of results
+    row = np.zeros(nv + 1, np.uint64)
+    row[1:] = 1
+    with sgs.Engine() as e:
+        e.load_csr(nv, row, np.array([1], np.uint32), np.array([3], np.uint32))
+        q = e.add_query(sgs.SSSP, 0)
+        before = free()
+        d = q.value()
+        assert d[0] == 0 and d[1] == 3 and np.all(d[2:] == sgs.INF)
+        assert before - free() < 64 << 20
 
 
 def test_pagerank_job_amended_between_long_steps():
