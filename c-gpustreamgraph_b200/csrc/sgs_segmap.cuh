@@ -54,12 +54,13 @@ __device__ __forceinline__ uint32_t visit_quad(const Op &op, uint32_t u,
 // positions) per step, lane i on quad i.  Owners need no search per quad: lane
 // j holds the start of entry s0 + j (s0 = owner of the window's first quad),
 // every start inside the window sets bit (start - window) / 4 of a warp-wide
-// OR, and a lane's owner is s0 plus the set bits at or below its quad.  Every
-// frontier entry has at least one slot (each append site checks it), so a
-// window meets at most 32 entries and no two starts share a bit.  The same
-// bits give the next window's first owner.  (With a binary search per
-// quad, eight dependent shared-memory reads, tombstoning 500,000 deletes at
-// scale 24 took 420 us instead of 402.)
+// OR, and a lane's owner is s0 plus the set bits at or below its quad.  The
+// entries of the chunk must all have slots: a window then meets at most 32 of
+// them and no two starts share a bit.  The same bits give the next window's
+// first owner.  (With a binary search per quad, eight dependent shared-memory
+// reads, tombstoning 500,000 deletes at scale 24 took 420 us instead of 402.)
+// A chunk with an empty entry, which none of the engine's frontiers has, is
+// walked by that search.
 template <int GC>
 struct WindowWalk {
   const uint64_t *eb;   // [GC + 1] starts of the chunk's entries
@@ -100,6 +101,22 @@ struct WindowWalk {
     q += 32;
     return in && j0 < len[own];
   }
+  // The same where entries may be empty: the last that starts at or before the
+  // quad, which is the one with slots.
+  __device__ __forceinline__ bool search(int &own, uint32_t &j0) {
+    const uint64_t p = (q + (threadIdx.x & 31)) << 2;
+    const bool in = q + (threadIdx.x & 31) < end;
+    int a = 0, b = GC - 1;
+    while (in && a < b) {
+      const int m = (a + b + 1) >> 1;
+      if (eb[m] <= p) a = m;
+      else b = m - 1;
+    }
+    own = a;
+    j0 = in ? (uint32_t)(p - eb[a]) : 0u;
+    q += 32;
+    return in && j0 < len[a];
+  }
 };
 
 // Each CTA walks one contiguous run of units [u_begin, u_end), staging up to
@@ -126,6 +143,7 @@ __global__ void __launch_bounds__(RELAX_THREADS)
     uint32_t s = __ldcg(&in.ustart[ub]);
     for (;;) {
       __syncthreads();  // previous chunk fully consumed
+      bool empty = false;
       {
         const uint32_t t = threadIdx.x;
         const uint32_t idx = s + t;
@@ -138,13 +156,15 @@ __global__ void __launch_bounds__(RELAX_THREADS)
         if (idx < n && eb < E1) {
           const uint32_t v = __ldcg(&in.vtx[idx]);
           s_vtx[t] = v;
-          s_len[t] = __ldcg(&in.len[idx]);
+          const uint32_t len = __ldcg(&in.len[idx]);
+          s_len[t] = len;
+          empty = len == 0;
           s_pay[t] = op.load(idx, v);
           if constexpr (op_touches<Op>::value)
             if (eb >= E0) op.touch(v, s_pay[t]);
         }
       }
-      __syncthreads();
+      const bool any_empty = __syncthreads_or(empty);
       const uint64_t lo = max(E0, s_eb[0]);
       const uint64_t hi = min(E1, s_eb[CHUNK]);
       WindowWalk<CHUNK> walk(s_eb, s_len, lo, hi, threadIdx.x >> 5, RELAX_THREADS / 32);
@@ -153,7 +173,7 @@ __global__ void __launch_bounds__(RELAX_THREADS)
         uint32_t av[4] = {0, 0, 0, 0}, ad[4] = {0, 0, 0, 0};
         int l;
         uint32_t j0;
-        if (walk.next(l, j0)) counted += visit_quad(op, s_vtx[l], s_pay[l], j0, s_len[l], app, av, ad);
+        if (any_empty ? walk.search(l, j0) : walk.next(l, j0)) counted += visit_quad(op, s_vtx[l], s_pay[l], j0, s_len[l], app, av, ad);
         if (Op::kAppends) {
           __syncwarp();
 #pragma unroll
