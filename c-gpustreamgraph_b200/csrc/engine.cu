@@ -740,6 +740,8 @@ struct sgs_engine {
     in_release();
     in_failed = false;
     pr_warm.release();
+    drop_job_vectors();
+    job_qid = 0;
     drop_gather();
     if (sc) CK(cudaStreamSynchronize(sc));
     stg_head = stg_count = 0;  // staged batches belonged to the old graph
@@ -1556,11 +1558,25 @@ struct sgs_engine {
     DBuf<double> prh;
     unsigned long long pr_in = 0;
     float ms = 0;
+    // The vectors of the last job, for the next of the same served trace: freeing
+    // them took from under 1 to 213 ms (67 million vertices), and the update behind
+    // waited for it.  drop_job_vectors() gives them back when the trace is served.
+    DBuf<double> rv, pvv;
     // a snapshot was applied while the job ran: its residual was amended
     // like any PageRank query's, and its dense frontier (block sizes of the
     // old graph) is rebuilt before the next sweep
     bool stale = false;
   } job;
+  int job_qid = 0;  // the query whose vectors the job takes back
+  template <class T>
+  static void swap_bufs(DBuf<T> &a, DBuf<T> &b) {
+    std::swap(a.p, b.p);
+    std::swap(a.n, b.n);
+  }
+  void drop_job_vectors() {
+    job.rv.release();
+    job.pvv.release();
+  }
   FrontierView job_view(uint32_t k) {
     FrontierView f;
     f.vtx = job.f.vtx.p;
@@ -1571,12 +1587,17 @@ struct sgs_engine {
     f.ucap = job.ucap;
     return f;
   }
-  // The job's dense frontier over the store its sweeps read, for the current
-  // graph (buffers sized for a dense frontier of either store).
-  void job_frontier() {
-    const uint64_t max_pos = std::max<uint64_t>(slots_total, in_capslots) + 3ull * nv;
+  // Units of a dense frontier of either store, by the stores' room, so that the
+  // buffer does not grow with every update that a job is amended for.
+  void job_units() {
+    const uint64_t max_pos = std::max<uint64_t>(arena_cap[0] + arena_cap[1], in_capslots) + 3ull * nv;
     job.ucap = (uint32_t)std::min<uint64_t>(max_pos / UNIT + 2, 0xFFFFFFF0ull);
     job.f.ustart.ensure(job.ucap);
+  }
+  // The job's dense frontier over the store its sweeps read, for the current
+  // graph.
+  void job_frontier() {
+    job_units();
     CK(cudaMemsetAsync(job.c.p, 0, sizeof(unsigned long long) * 2, s));
     const GraphView gi = job.pull ? in_view() : view();
     { ++n_launch; k_dense_frontier<<<grid_elem(nv), 256, 0, s>>>(gi, job_view(0)); }
@@ -1585,13 +1606,10 @@ struct sgs_engine {
   }
   int pr_job_start() {
     if (job.q) fail(SGS_ERR_STATE, "a PageRank job is already running");
-    // frontier buffers of the job, sized for a dense frontier of either store
-    const uint64_t max_pos = slots_total + 3ull * nv;
-    job.ucap = (uint32_t)std::min<uint64_t>(max_pos / UNIT + 2, 0xFFFFFFF0ull);
     job.f.vtx.ensure((size_t)nv + 1);
     job.f.len.ensure((size_t)nv + 1);
     job.f.ebase.ensure((size_t)nv + 1);
-    job.f.ustart.ensure(job.ucap);
+    job_units();
     job.c.ensure(3);
     job.prh.ensure(StepHist::FIELDS * (size_t)(cfg.max_rounds + 2));
     job.stale = false;
@@ -1599,9 +1617,12 @@ struct sgs_engine {
     auto q = std::make_unique<Query>();
     q->id = next_qid++;
     q->algo = SGS_PR;
-    q->x.ensure(nv);
+    swap_bufs(q->r, job.rv);
+    swap_bufs(q->pv, job.pvv);
+    if (!(pr_warm.p && pr_warm.n >= nv)) q->x.ensure(nv);  // (else pr_init hands it over)
     q->r.ensure(nv);
     q->pv.ensure(nv);
+    job_qid = q->id;
     CK(cudaEventRecord(ev_q.a, s));
     pr_init(*q, job_view(0), job_view(1));
     CK(cudaMemsetAsync(job.c.p, 0, sizeof(unsigned long long) * 3, s));
@@ -2168,6 +2189,11 @@ struct sgs_engine {
           if (!q.grp->used) q.grp->unrepaired = false;  // the next lanes start from scratch
         }
         if (job.q == &q) job.q = nullptr;
+        if (q.id == job_qid) {
+          swap_bufs(q.r, job.rv);
+          swap_bufs(q.pv, job.pvv);
+          job_qid = 0;
+        }
         if (q.algo == SGS_PR && cfg.pr_warm) {  // keep its vector for the next start
           std::swap(pr_warm.p, q.x.p);
           std::swap(pr_warm.n, q.x.n);
@@ -3229,6 +3255,12 @@ int pr_job_start(sgs_engine *e, int *qid) {
     if (!e->loaded) fail(SGS_ERR_STATE, "no graph loaded");
     CK(cudaSetDevice(e->dev));
     *qid = e->pr_job_start();
+  });
+}
+int serve_end(sgs_engine *e) {
+  return guarded([&] {
+    CK(cudaSetDevice(e->dev));
+    e->drop_job_vectors();
   });
 }
 int pr_job_advance(sgs_engine *e, uint32_t rounds, int *done) {

@@ -67,6 +67,7 @@ uint32_t serve_restarts(sgs_engine *e);
 int reserve_batch(sgs_engine *e, uint64_t ni, uint64_t nd);
 int pr_job_start(sgs_engine *e, int *qid);
 int pr_job_advance(sgs_engine *e, uint32_t rounds, int *done);
+int serve_end(sgs_engine *e);
 }  // namespace sgs
 
 namespace {
@@ -365,6 +366,7 @@ SGS_API int sgs_serve(sgs_engine *e, const sgs_request *req, uint32_t n, uint32_
     }
   }
   (void)running;
+  (void)sgs::serve_end(e);
   return SGS_OK;
 }
 

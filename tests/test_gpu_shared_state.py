@@ -91,3 +91,42 @@ def test_pagerank_job_amended_between_long_steps():
         assert np.max(np.abs(reqs[0]["value_out"] - ref)) <= 1e-6
         q = e.add_query(sgs.SSSP, 0)
         check_query(q, m, sgs.W_EXPLICIT)
+
+
+def test_served_pagerank_jobs_one_after_the_other():
+    """The second job of a trace takes over the first one's vectors; the call
+    gives them back."""
+    import torch
+
+    def free():
+        torch.cuda.synchronize()
+        return torch.cuda.mem_get_info()[0]
+
+    nv = 1 << 22  # 32 MB a vector
+    n0, row0, col0 = O.rmat_csr(13, 16, 8)
+    row = np.concatenate([row0, np.full(nv - n0, row0[-1], np.uint64)])
+    w = O.weights(n0, row0, col0, 1, 0)
+    src = np.repeat(np.arange(n0), np.diff(row0).astype(np.int64)).astype(np.uint32)
+    m = Mirror(nv, row, col0, w)
+
+    def update(k):  # two of the same size
+        d = np.arange(k, len(col0), 97)
+        i_s, i_d = np.arange(500 * k, 500 * k + 500, dtype=np.uint32), np.arange(2000, 2500, dtype=np.uint32)
+        b = (i_s, i_d, O.weights_pairs(1, i_s, i_d), src[d], col0[d])
+        m.apply(*b)
+        return dict(zip(("ins_src", "ins_dst", "ins_w", "del_src", "del_dst"), b), kind="update", arrival_s=0.5)
+
+    with sgs.Engine() as e:
+        e.load_csr(nv, row, col0, w)
+        out = [np.empty(nv) for _ in range(3)]
+        pr = [{"kind": "query", "algo": sgs.PR, "arrival_s": 0.4 * k, "value_out": out[k]} for k in range(3)]
+        e.serve([pr[0], update(0), pr[2]])  # what an update and a job allocate once
+        before = free()
+        ref = O.pagerank(nv, m.row, m.col)
+        assert np.max(np.abs(out[2] - ref)) <= 1e-6
+        done = e.serve([pr[0], pr[1], update(1), pr[2]])
+        assert all(c["status"] == 0 for c in done)
+        assert before - free() < 16 << 20
+        assert done[1]["version"] == 0 and np.max(np.abs(out[1] - ref)) <= 1e-6
+        assert done[3]["version"] == 1
+        assert np.max(np.abs(out[2] - O.pagerank(nv, m.row, m.col))) <= 1e-6
