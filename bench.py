@@ -451,7 +451,10 @@ def engine_arm(a, R):
     traffic = None
     if tr and dom in tr.get("per_kind", {}) and kd["launches"]:
         traffic = round(tr["per_kind"][dom]["dram_bytes_per_slot"] * kd["slots"] / kd["launches"])
-    roof = {"bound": "hbm", "kernel": f"group_map<{dom}>", "achieved": round(achieved, 1),
+    # (the restricted sweep reads 4 bytes a slot and is a kernel of its own)
+    restricted = dom == "group_sweep" and kd["bytes_alg"] < 8 * kd["slots"]
+    roof = {"bound": "hbm", "kernel": "k_group_sweep" if restricted else f"group_map<{dom}>",
+            "achieved": round(achieved, 1),
             "peak": peak, "unit": "GB/s", "frac": round(achieved / peak, 4),
             "peak_source": peak_src, "traffic": traffic,
             "launches": kd["launches"], "avg_launch_ms": kd["ms"] / max(kd["launches"], 1),
@@ -1018,11 +1021,17 @@ def ppr_arm(a, R):
     value = R.sum(relax) / (T_ms * 1e6)
     peak, peak_src = measured_peak_hbm()
     achieved = nbytes / (steps_ms * 1e-3) / 1e9
-    roof = {"bound": "hbm", "kernel": "k_ppr_step",
-            "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
-            "frac": round(achieved / peak, 4), "peak_source": peak_src, "traffic": None,
-            "launches": nsteps, "avg_launch_ms": round(steps_ms / nsteps, 4),
-            "alg_bytes_per_launch": sf["bytes_alg_step"]}
+    # most rows of a gather come from L2 (profiles/ppr_step_s20.md: 2.95 GB of
+    # DRAM traffic for 10.06 GB of these bytes), so the HBM peak is not a bound
+    # and there is no fraction of it; steps of less than 64 MB run in one
+    # looping launch per solve
+    loops = sf["bytes_alg_step"] < 64e6
+    n_launch = 2 * a.steps if loops else nsteps
+    roof = {"bound": "l2", "kernel": "k_ppr_steps" if loops else "k_ppr_step",
+            "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s (algorithmic)",
+            "frac": None, "peak_source": peak_src, "traffic": None,
+            "launches": n_launch, "avg_launch_ms": round(steps_ms / n_launch, 4),
+            "alg_bytes_per_step": sf["bytes_alg_step"]}
     # ---------------- e2e through the torch op from pinned host memory
     e2e = None
     if not a.no_e2e:
