@@ -375,6 +375,7 @@ __device__ __forceinline__ void ppr_step_body(const StepArgs &a, const sgs::Step
   constexpr bool Dyn = !Coh;
   constexpr unsigned full = 0xFFFFFFFFu;
   constexpr int NEG = 32 / LPE;
+  constexpr int DEEP = Coh || LPE >= 8 ? 8 : 4, GROUP_DEEP = Coh ? 8 : 4;  // loads in flight per lane group
   const int lane = threadIdx.x & 31;
   const int sub = lane % LPE, eg = lane / LPE;
   const uint32_t K = a.K;
@@ -389,7 +390,7 @@ __device__ __forceinline__ void ppr_step_body(const StepArgs &a, const sgs::Step
     if constexpr (LPE == 32) {
       gather_wide<CPL, Coh>(a.nbr, a.p, b, e, h, lane, k0 + lane, K, x, acc);
     } else {
-      acc[0] = gather_narrow<LPE, Coh ? 8 : 4, Coh>(a.nbr, a.p, b + eg, e, NEG, k0 + sub, K, x);
+      acc[0] = gather_narrow<LPE, DEEP, Coh>(a.nbr, a.p, b + eg, e, NEG, k0 + sub, K, x);
 #pragma unroll
       for (int o = 16; o >= LPE; o >>= 1) acc[0] += __shfl_xor_sync(full, acc[0], o);
     }
@@ -454,9 +455,9 @@ __device__ __forceinline__ void ppr_step_body(const StepArgs &a, const sgs::Step
         // so with heavier ones if that takes fewer loads in a row than the warp on
         // one after the other (20,000 vertices, a fifth of them with 64 in-edges,
         // K = 1: 36 -> 19 us a step)
-        constexpr uint32_t D = Coh ? 8 : 4;
         const uint32_t many = __popc(todo);
-        if ((many + NEG - 1) / NEG * ((a.piece + D - 1) / D) < many * ((a.piece + NEG * D - 1) / (NEG * D))) {
+        if ((many + NEG - 1) / NEG * ((a.piece + GROUP_DEEP - 1) / GROUP_DEEP) <
+            many * ((a.piece + NEG * DEEP - 1) / (NEG * DEEP))) {
           lo |= todo;
           todo = 0;
         }
@@ -464,7 +465,7 @@ __device__ __forceinline__ void ppr_step_body(const StepArgs &a, const sgs::Step
           const int my = eg < __popc(lo) ? (int)__fns(lo, 0, eg + 1) : -1;
           const uint64_t b = __shfl_sync(full, rb, my & 31), e = __shfl_sync(full, re, my & 31);
           if (my >= 0) {
-            const double s = gather_narrow<LPE, Coh ? 8 : 4, Coh>(a.nbr, a.p, b, e, 1, sub, K, x);
+            const double s = gather_narrow<LPE, GROUP_DEEP, Coh>(a.nbr, a.p, b, e, 1, sub, K, x);
             if ((uint32_t)sub < K) finish_entry<Coh>(a, rule, (uint64_t)(v0 + my) * K + sub, s, x, out, dsum, fsum);
           }
           __syncwarp();
@@ -536,8 +537,10 @@ __device__ __forceinline__ void ppr_step_body(const StepArgs &a, const sgs::Step
   }
 }
 
+// (From 5 columns on with 64 registers, and gathers 8 deep up to 16: 2^16 vertices,
+// K = 8, 1.00 ms, 1.11 with 48 and 4 deep.)
 template <int LPE, int CPL>
-__global__ void __launch_bounds__(THREADS, LPE == 32 ? 4 : 5)
+__global__ void __launch_bounds__(THREADS, LPE >= 8 ? 4 : 5)
     k_ppr_step(StepArgs a, const double *__restrict__ x, double *out, uint32_t k, bool first) {
   ppr_step_body<LPE, CPL, false>(a, sgs::step_rule<true>(a.h, k, a.alpha, a.tol * sgs::LONG_TOL), x, out, k, first);
 }
@@ -964,13 +967,16 @@ struct sgs_ppr {
     PCK(cudaGetLastError());
   }
 
-  // Light vertices per item: 8 from the counter (32 left the last items to few
-  // warps; 4 with two lane groups, which walk most vertices one by one: 2^18
-  // vertices, K = 16: 5.0 -> 4.5 ms), in the loop as many as give every warp one item; at least what the
-  // lane groups of a narrow form take at a time, at most 32.
+  // Light vertices per item.  From the counter: 8 with up to 8 columns, where the
+  // counter sets the pace of finer ones (2^20 vertices, K = 8: 9.9 ms, 11.5 with
+  // 4), and with 16 from 2^20 vertices on (12.5 ms, 13.1 with 4); 4 with more (K = 64: 24.0 ms, 24.4 with 8 and 26.0 with 2; 2^18 vertices, K =
+  // 16: 4.1 and 4.4 with 8), which keeps the last items short; 2 where a warp gets
+  // few items (20,480 vertices, a fifth with 64 edges, K = 64: 8.9 ms, 10.3 with 4 and
+  // 12.6 with 8).  In the loop as many as give every warp one item.  At least what
+  // the lane groups of a narrow form take at a time, at most 32.
   uint32_t items_per_warp(bool loop, uint32_t K) const {
     const uint32_t warps = (uint32_t)nsm * 32, neg = 32u / (uint32_t)lanes_per_edge(std::min(K, 32u));
-    uint32_t per = loop ? (nv + warps - 1) / warps : neg == 2 ? 4u : 8u;
+    uint32_t per = loop ? (nv + warps - 1) / warps : neg >= 4 || (neg == 2 && nv >= 1u << 20) ? 8u : nv < 8 * warps ? 2u : 4u;
     return std::min(32u, std::max(per, neg));
   }
 
